@@ -162,9 +162,26 @@ int occupancy_blocks(const void *fn, int threads, size_t smem)
     return blocks < 1 ? 1 : blocks;
 }
 
-/* Rows per tile: fixed so a candidate's reduction order depends only on n
-   and its own depth bucket. */
+/* Rows per tile of rc_score_noalloc (its scratch bound is stated for it). */
 const int TILE_ROWS = RC_TILE_ROWS;
+
+/* Rows per tile of the scoring calls: a function of n alone, so a
+   candidate's reduction order depends only on n and its own depth bucket.
+   About 32 tiles or more, so that a few candidates still spread over the
+   SMs and a candidate sent to the f64 lane is not one block's serial walk
+   over 32,768 rows; from 1,024 rows (one pass of the 256-thread shape) to
+   RC_TILE_ROWS (reached at a million rows, where the tiles are many already
+   and a longer tile amortises its reduction). Against 32,768-row tiles at
+   every n, a call takes 295 against 683 us for 800 programs x 8,000 rows,
+   143 against 996 us for 24 classification programs x 20,011 rows, and 1.60
+   against 3.37 ms for 701 programs x 131,101 rows under correlation (there
+   also with first-pass failures kept for the second pass). */
+int rc_score_tile_rows(int n)
+{
+    int rows = RC_TILE_ROWS_MIN;
+    while (rows < RC_TILE_ROWS && (long long)rows * 32 < n) rows *= 2;
+    return rows;
+}
 const int LANE_T = 128;
 
 const void *score_kernel_fn(int T, bool track)
@@ -262,8 +279,8 @@ float rc_score_run(RcCtx *c, const uint32_t *words, const uint32_t *off, int wid
     const int Tb[2] = {256, 64};
     /* the scoring kernel reads features from L2; nothing is staged */
     const int staged = 0;
-    const int ntiles = std::max(1, (c->n + TILE_ROWS - 1) / TILE_ROWS);
-    std::vector<int> cand_tiles(nprog, ntiles);
+    const int tile_rows = rc_score_tile_rows(c->n);
+    const int ntiles = std::max(1, (c->n + tile_rows - 1) / tile_rows);
     std::vector<int> order;
     order.reserve(nprog);
     for (int b = 0; b < 2; ++b) order.insert(order.end(), bk[b].cands.begin(), bk[b].cands.end());
@@ -271,13 +288,13 @@ float rc_score_run(RcCtx *c, const uint32_t *words, const uint32_t *off, int wid
     const bool corr = (mode == SM_CORRELATION || mode == SM_CORRELATION_SIGNED);
     const bool track = mode < SM_EVAL_SQUARED;
 
-    /* 3. layout: inputs [ins | ins_off | order | cand_tiles], outputs
-       [out | status | out_f32], work [part | bad | counters | pbar | lane]. */
+    /* 3. layout: inputs [ins | ins_off | order | opw], outputs
+       [out | status | out_f32 | rows], work zeroed with rows by one memset
+       [bad | bad64 | badrow | counters], work [part | pbar | lane]. */
     size_t cur = 0;
     const size_t o_ins = rc_take(&cur, sizeof(RcIns) * ins.size());
     const size_t o_insoff = rc_take(&cur, sizeof(int) * (nprog + 1));
     const size_t o_order = rc_take(&cur, sizeof(int) * nprog);
-    const size_t o_ctiles = rc_take(&cur, sizeof(int) * nprog);
     const size_t o_opw = rc_take(&cur, sizeof(int) * nprog);
     const size_t in_end = rc_take(&cur, 0);
     const size_t o_out = rc_take(&cur, sizeof(double) * nprog);
@@ -285,16 +302,16 @@ float rc_score_run(RcCtx *c, const uint32_t *words, const uint32_t *off, int wid
     const size_t o_f32 = rc_take(&cur, sizeof(float) * nprog);
     const size_t o_rows = rc_take(&cur, 4 * sizeof(unsigned long long));
     const size_t io_end = rc_take(&cur, 0);
-    const size_t o_part = rc_take(&cur, 4 * sizeof(double) * (size_t)nprog * ntiles);
     const size_t o_bad = rc_take(&cur, sizeof(int) * nprog);
     const size_t o_bad64 = rc_take(&cur, sizeof(int) * nprog);
+    const size_t o_badrow = rc_take(&cur, track ? sizeof(int) * nprog : 0);
     const size_t o_cnt = rc_take(&cur, sizeof(int) * 16);
     const size_t o_zero_end = rc_take(&cur, 0);
+    const size_t o_part = rc_take(&cur, 4 * sizeof(double) * (size_t)nprog * ntiles);
     const size_t o_pbar = rc_take(&cur, sizeof(double) * nprog);
     const size_t o_pbarerr = rc_take(&cur, sizeof(double) * nprog);
     const size_t o_pbar64 = rc_take(&cur, sizeof(double) * nprog);
     const size_t o_flagged = rc_take(&cur, sizeof(int) * nprog);
-    const size_t o_badrow = rc_take(&cur, track && !corr ? sizeof(int) * nprog : 0);
     const size_t o_part64 = rc_take(&cur, track ? 2 * sizeof(double) * (size_t)nprog * ntiles : 0);
     const size_t o_pred = rc_take(&cur, pred_out ? sizeof(float) * (size_t)nprog * c->n : 0);
     const size_t dev_end = rc_take(&cur, 0);
@@ -309,13 +326,10 @@ float rc_score_run(RcCtx *c, const uint32_t *words, const uint32_t *off, int wid
     memcpy(host + o_ins, ins.data(), sizeof(RcIns) * ins.size());
     memcpy(host + o_insoff, ins_off.data(), sizeof(int) * (nprog + 1));
     memcpy(host + o_order, order.data(), sizeof(int) * nprog);
-    memcpy(host + o_ctiles, cand_tiles.data(), sizeof(int) * nprog);
     memcpy(host + o_opw, opw.data(), sizeof(int) * nprog);
     cudaMemcpyAsync(dev, host, in_end, cudaMemcpyHostToDevice, c->s);
-    cudaMemsetAsync(dev + o_bad, 0, o_zero_end - o_bad, c->s);
-    cudaMemsetAsync(dev + o_rows, 0, 4 * sizeof(unsigned long long), c->s);
+    cudaMemsetAsync(dev + o_rows, 0, o_zero_end - o_rows, c->s);
     unsigned long long *d_rows = reinterpret_cast<unsigned long long *>(dev + o_rows);
-    if (track && !corr) cudaMemsetAsync(dev + o_badrow, 0x7f, sizeof(int) * nprog, c->s);
     st->h2d_ms += rc_now_ms() - t;
     st->h2d_bytes += in_end;
 
@@ -340,14 +354,13 @@ float rc_score_run(RcCtx *c, const uint32_t *words, const uint32_t *off, int wid
     a.ntiles = ntiles;
     a.part = reinterpret_cast<double *>(dev + o_part);
     a.bad = reinterpret_cast<int *>(dev + o_bad);
-    a.badrow = track && !corr ? reinterpret_cast<int *>(dev + o_badrow) : nullptr;
+    a.badrow = track ? reinterpret_cast<int *>(dev + o_badrow) : nullptr;
     a.rows = d_rows;
     a.opw = reinterpret_cast<const int *>(dev + o_opw);
     a.pred = pred_out ? reinterpret_cast<float *>(dev + o_pred) : nullptr;
     a.pbar = reinterpret_cast<const double *>(dev + o_pbar);
     a.pbar_err = reinterpret_cast<const double *>(dev + o_pbarerr);
     a.ybar = c->ybar;
-    const int *d_ctiles = reinterpret_cast<const int *>(dev + o_ctiles);
 
     t = rc_now_ms();
     cudaEventRecord(c->t0, c->s);
@@ -355,7 +368,8 @@ float rc_score_run(RcCtx *c, const uint32_t *words, const uint32_t *off, int wid
     const int passes = corr ? 2 : 1;
     for (int pass = 0; pass < passes; ++pass) {
         const int kmode = corr ? (pass == 0 ? SM_CORR_PASS1 : SM_CORR_PASS2) : mode;
-        if (pass == 1) cudaMemsetAsync(dev + o_bad, 0, sizeof(int) * nprog, c->s);
+        /* (a candidate that failed in the first pass fails in the second, on
+           the same predictions: `bad` stays, and its rows are skipped) */
         int obase = 0;
         for (int b = 0; b < 2; ++b) {
             const int nb = (int)bk[b].cands.size();
@@ -365,10 +379,16 @@ float rc_score_run(RcCtx *c, const uint32_t *words, const uint32_t *off, int wid
             auto it = c->tune.find(b);
             if (it != c->tune.end()) group = it->second.first;
             group = std::max(1, std::min(group, std::min(nb, 32)));
+            /* few (candidate, tile) pairs: smaller groups until the grid has
+               four items a block to balance (a candidate's bits do not
+               depend on its group) */
+            while (group > 1 &&
+                   (long long)((nb + group - 1) / group) * ntiles < (long long)c->sm_count * 16)
+                group /= 2;
             a.order = reinterpret_cast<const int *>(dev + o_order) + obase;
             a.ncand = nb;
             a.group = group;
-            a.subtiles = TILE_ROWS / (T * 4);
+            a.subtiles = tile_rows / (T * 4);
             const int ngroups = (nb + group - 1) / group;
             a.nitems = ngroups * ntiles;
             a.maxins = bk[b].maxins;
@@ -392,8 +412,8 @@ float rc_score_run(RcCtx *c, const uint32_t *words, const uint32_t *off, int wid
         }
         if (pass == passes - 1) cudaEventRecord(c->sp[1], c->s);
         c->launches += 1;
-        rc_score_finalize<<<(nprog + 127) / 128, 128, 0, c->s>>>(
-            nprog, d_ctiles, a.part, ntiles, a.bad, c->n, (corr && pass == 1) ? mode : kmode,
+        rc_score_finalize<<<(4 * nprog + 127) / 128, 128, 0, c->s>>>(
+            nprog, ntiles, a.part, ntiles, a.bad, c->n, (corr && pass == 1) ? mode : kmode,
             c->syy, d_out, d_status,
             reinterpret_cast<float *>(dev + o_f32), reinterpret_cast<double *>(dev + o_pbar),
             reinterpret_cast<double *>(dev + o_pbarerr), d_nflag,
@@ -415,6 +435,7 @@ float rc_score_run(RcCtx *c, const uint32_t *words, const uint32_t *off, int wid
         l.flagged = reinterpret_cast<const int *>(dev + o_flagged);
         l.nflag = d_nflag;
         l.ntiles = ntiles;
+        l.tile_rows = tile_rows;
         l.nslots = max_slots;
         l.part = reinterpret_cast<double *>(dev + o_part64);
         l.nprog = nprog;
@@ -446,7 +467,6 @@ float rc_score_run(RcCtx *c, const uint32_t *words, const uint32_t *off, int wid
         }
         for (int pass = 0; pass < passes; ++pass) {
             const int kmode = corr ? (pass == 0 ? SM_CORR_PASS1 : SM_CORR_PASS2) : mode;
-            if (pass == 1) cudaMemsetAsync(dev + o_bad64, 0, sizeof(int) * nprog, c->s);
             l.counter = d_cnt + 4 + pass;
             l.mode = kmode;
             c->launches += 2;
@@ -727,15 +747,14 @@ static __device__ __align__(256) unsigned char rc_noalloc_scratch[RC_NOALLOC_SCR
 __global__ void rc_noalloc_decode(const unsigned int *__restrict__ prog,
                                   const unsigned int *__restrict__ off, int nprog, int v,
                                   RcIns *__restrict__ ins, int *__restrict__ ins_off,
-                                  int *__restrict__ order, int *__restrict__ cand_tiles,
-                                  int *__restrict__ deep, int *__restrict__ ins_len, int ntiles)
+                                  int *__restrict__ order,
+                                  int *__restrict__ deep, int *__restrict__ ins_len)
 {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p > nprog) return;
     ins_off[p] = p * RC_MAX_INS;
     if (p == nprog) return;
     order[p] = p;
-    cand_tiles[p] = ntiles;
     deep[p] = 0;
     RcIns *out = ins + (size_t)p * RC_MAX_INS;
     const unsigned int b = off[p], e = off[p + 1];
@@ -870,7 +889,7 @@ extern "C" int rc_score_batch_noalloc(const float *cols, const float *y, int n, 
     const size_t o_ins = rc_take(&cur, sizeof(RcIns) * (size_t)nprog * RC_MAX_INS);
     const size_t o_insoff = rc_take(&cur, sizeof(int) * ((size_t)nprog + 1));
     const size_t o_order = rc_take(&cur, sizeof(int) * (size_t)nprog);
-    const size_t o_ctiles = rc_take(&cur, sizeof(int) * (size_t)nprog);
+    rc_take(&cur, sizeof(int) * (size_t)nprog); /* spare: the refusal bound counts it */
     const size_t o_deep = rc_take(&cur, sizeof(int) * (size_t)nprog);
     const size_t o_len = rc_take(&cur, sizeof(int) * (size_t)nprog);
     const size_t o_part = rc_take(&cur, 4 * sizeof(double) * (size_t)nprog * ntiles);
@@ -933,8 +952,7 @@ extern "C" int rc_score_batch_noalloc(const float *cols, const float *y, int n, 
     rc_noalloc_decode<<<(nprog + 1 + 127) / 128, 128, 0, s>>>(
         prog, off, nprog, v, reinterpret_cast<RcIns *>(sc + o_ins),
         reinterpret_cast<int *>(sc + o_insoff), reinterpret_cast<int *>(sc + o_order),
-        reinterpret_cast<int *>(sc + o_ctiles), reinterpret_cast<int *>(sc + o_deep),
-        reinterpret_cast<int *>(sc + o_len), ntiles);
+        reinterpret_cast<int *>(sc + o_deep), reinterpret_cast<int *>(sc + o_len));
     int *cnt = reinterpret_cast<int *>(sc + o_cnt);
     ScoreArgs a;
     memset(&a, 0, sizeof(a));
@@ -974,8 +992,8 @@ extern "C" int rc_score_batch_noalloc(const float *cols, const float *y, int n, 
             return -1;
         }
     }
-    rc_score_finalize<<<(nprog + 127) / 128, 128, 0, s>>>(
-        nprog, reinterpret_cast<const int *>(sc + o_ctiles), a.part, ntiles, a.bad, n, kind, 0.0,
+    rc_score_finalize<<<(4 * nprog + 127) / 128, 128, 0, s>>>(
+        nprog, ntiles, a.part, ntiles, a.bad, n, kind, 0.0,
         out, status, nullptr, nullptr, nullptr, cnt + 8, reinterpret_cast<int *>(sc + o_flagged));
     Score64Args l;
     memset(&l, 0, sizeof(l));
@@ -988,6 +1006,7 @@ extern "C" int rc_score_batch_noalloc(const float *cols, const float *y, int n, 
     l.flagged = reinterpret_cast<const int *>(sc + o_flagged);
     l.nflag = cnt + 8;
     l.ntiles = ntiles;
+    l.tile_rows = TILE_ROWS;
     l.nslots = RC_SHALLOW_SLOTS;
     l.counter = cnt + 4;
     l.part = reinterpret_cast<double *>(sc + o_part64);

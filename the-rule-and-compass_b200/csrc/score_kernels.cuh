@@ -37,9 +37,11 @@ enum {
    loss is rescored in f64 (ten times below the 1e-4 parity bar). */
 #define RC_FLAG_TOL 1e-5
 
-/* Rows per work-item tile, fixed so that a candidate's reduction order
-   depends only on n and the kernel shape. */
+/* Rows per work-item tile: at most RC_TILE_ROWS, less for a small table
+   (rc_score_tile_rows), a function of n alone so that a candidate's
+   reduction order depends only on n and the kernel shape. */
 #define RC_TILE_ROWS 32768
+#define RC_TILE_ROWS_MIN 1024
 
 __device__ __forceinline__ bool rc_mode_tracks(int mode)
 {
@@ -445,6 +447,10 @@ __device__ __forceinline__ double rc_class_row_loss_d(double p, double tsign, in
     return CUDART_NAN;
 }
 
+/* badrow holds this minus the lowest failing 4-row group, so that a zeroed
+   array means none and an atomic max keeps the lowest. */
+#define RC_BADROW_BASE 0x7fffffff
+
 struct ScoreArgs {
     const float *cols;
     const float *y;
@@ -468,7 +474,8 @@ struct ScoreArgs {
     int nprog;
     int ptiles;
     int *bad;             /* [P] */
-    int *badrow;          /* [P] or null: first 4-row group of a hard failure */
+    int *badrow;          /* [P] or null, zeroed: RC_BADROW_BASE - (first 4-row group of a
+                             hard failure) */
     unsigned long long *rows; /* or null: [0] += rows the interpreter evaluated,
                                  [2] += those rows x (ops + 2) of their candidate */
     const int *opw;           /* [P] postfix ops + 2 per candidate (with rows) */
@@ -666,7 +673,7 @@ __global__ void __launch_bounds__(T) rc_score_kernel(ScoreArgs a)
                 if (skip_bad && __any_sync(0xffffffffu, bad)) {
                     const int grp = __reduce_min_sync(0xffffffffu,
                                                       bad ? (unsigned)myrow : 0x7fffffffu);
-                    if (a.badrow && lane == 0) atomicMin(a.badrow + cand, grp);
+                    if (a.badrow && lane == 0) atomicMax(a.badrow + cand, RC_BADROW_BASE - grp);
                     break;
                 }
             }
@@ -722,7 +729,7 @@ __global__ void __launch_bounds__(T) rc_score_kernel(ScoreArgs a)
    the objective, the status, and the flag that sends the candidate to the
    f64 lane (a non-finite f32 row, or an error bound above RC_FLAG_TOL of the
    objective's sums). */
-__global__ void rc_score_finalize(int nprog, const int *__restrict__ cand_tiles,
+__global__ void rc_score_finalize(int nprog, int ntiles,
                                   const double *__restrict__ part, int ptiles,
                                   const int *__restrict__ bad, int n, int mode, double syy,
                                   double *__restrict__ out, int *__restrict__ status,
@@ -730,16 +737,23 @@ __global__ void rc_score_finalize(int nprog, const int *__restrict__ cand_tiles,
                                   double *__restrict__ pbar_err, int *__restrict__ nflag,
                                   int *__restrict__ flagged)
 {
-    const int cand = blockIdx.x * blockDim.x + threadIdx.x;
-    if (cand >= nprog) return;
-    const int nt = cand_tiles[cand];
-    double s[4] = {0.0, 0.0, 0.0, 0.0};
-    for (int q = 0; q < 4; ++q) {
-        for (int t = 0; t < nt; ++t) {
-            const double v = part[((size_t)q * nprog + cand) * ptiles + t];
-            s[q] = (mode == SM_MAXIMUM) ? fmax(s[q], v) : s[q] + v;
+    /* four lanes per candidate, one per partial sum (no lane leaves before
+       the shuffles) */
+    const int gt = blockIdx.x * blockDim.x + threadIdx.x;
+    const int cand = gt >> 2, q = gt & 3;
+    double sq = 0.0;
+    if (cand < nprog) {
+        const double *pp = part + ((size_t)q * nprog + cand) * ptiles;
+#pragma unroll 8
+        for (int t = 0; t < ntiles; ++t) {
+            const double v = pp[t];
+            sq = (mode == SM_MAXIMUM) ? fmax(sq, v) : sq + v;
         }
     }
+    double s[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) s[k] = __shfl_sync(0xffffffffu, sq, (threadIdx.x & 28) + k);
+    if (cand >= nprog || q != 0) return;
     if (mode >= SM_EVAL_SQUARED && mode <= SM_EVAL_ABSOLUTE) {
         out_f32[cand] = (float)s[0];
         return;
@@ -952,6 +966,7 @@ struct Score64Args {
     const int *flagged;
     const int *nflag;
     int ntiles;
+    int tile_rows;
     int nslots;
     int *counter;
     double *part;      /* [2][P][ptiles] */
@@ -976,7 +991,7 @@ __global__ void __launch_bounds__(T) rc_score64_kernel(Score64Args a)
     __shared__ int s_item, s_known;
     const int tid = threadIdx.x;
     const int SUB = 2 * T;
-    const int subtiles = RC_TILE_ROWS / SUB;
+    const int subtiles = a.tile_rows / SUB;
     const int mode = a.mode;
     for (;;) {
         const int total = *a.nflag * a.ntiles;
@@ -1098,7 +1113,8 @@ __global__ void __launch_bounds__(T) rc_badrow_check(Score64Args a, const int *b
     const int k = blockIdx.x, tid = threadIdx.x;
     if (k >= *a.nflag) return;
     const int cand = a.flagged[k];
-    const int r = badrow[cand];
+    if (badrow[cand] == 0) return;
+    const int r = RC_BADROW_BASE - badrow[cand];
     if (r < 0 || r >= a.n) return;
     const int b = a.ins_off[cand], e = a.ins_off[cand + 1];
     for (int q = tid; q < e - b; q += T) sprog[q] = a.ins[b + q];
