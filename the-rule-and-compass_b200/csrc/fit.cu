@@ -211,7 +211,7 @@ struct FitArgs {
     const double *c0;
     const int *gauge;      /* [2P] correlation gauge pair (scale, offset), -1 = none */
     const int *valid;
-    const FIns *fins;      /* stack-machine translation of the records */
+    const FOp *fins;       /* stack-machine translation of the records */
     const int *fins_off;   /* [P+1] start of [forward | reverse] */
     const int4 *finfo;     /* [P] forward count, reverse count, active threads | launch
                               class << 16,
@@ -225,12 +225,12 @@ struct FitArgs {
                               first cache column */
     float *cache;          /* [columns][npad] values of constant-free subtrees */
     double *cache64;       /* the same columns in f64 for the polish, or null */
-    const FIns *sub_fins;  /* forward lists of the cached subtrees */
+    const FOp *sub_fins;   /* forward lists of the cached subtrees */
     const int *sub_off;    /* [nsub + 1] */
     const int *sub_col;    /* [nsub] */
     int nsub;
     int sub_slots, sub_maxins;
-    const FIns *xfins;     /* implicit metric: input-mode lists [forward | reverse] */
+    const FOp *xfins;      /* implicit metric: input-mode lists [forward | reverse] */
     const int *xfins_off;  /* [P + 1] */
     const int4 *xinfo;     /* forward count, reverse count, spill slots, tape slots */
     int xmaxins, xslots, xtape;
@@ -380,7 +380,7 @@ __device__ void ft_tile_implicit(const FitArgs &a, const uint4 *rec, int ni, int
    gradient, or a zero gradient norm, marks the tile undefined
    (implicit.rs:156-174). */
 template <int T>
-__device__ void ft_tile_icost_x(const FitArgs &a, const FIns *fwd, int nf, int nr,
+__device__ void ft_tile_icost_x(const FitArgs &a, const FOp *fwd, const FOp *rev,
                                 const double *cd, FiV<double, 1>::V4 *stk,
                                 FiV<double, 1>::V4 *tape, FiV<double, 1>::V4 *ig, double *red,
                                 int r0, int r1, double *pt)
@@ -391,7 +391,7 @@ __device__ void ft_tile_icost_x(const FitArgs &a, const FIns *fwd, int nf, int n
     for (int base = r0; base < r1; base += T) {
         const int row = base + tid;
         double fv;
-        fi_forward<double, 1, true>(fwd, cd, a.cols64, a.npad, row, stk, tape, T, tid, &fv);
+        fi_forward<double, 1, true>(fwd, cd, a.cols64 + row, a.npad, stk + tid, tape + tid, T, &fv);
         if (row >= r1) continue;
         const double wr = a.w ? a.w[row] : 1.0;
         if (!(isfinite(wr) && wr >= 0.0)) {
@@ -405,7 +405,7 @@ __device__ void ft_tile_icost_x(const FitArgs &a, const FIns *fwd, int nf, int n
         }
         for (int k = 0; k < a.v; ++k) ig[k * T + tid].v[0] = 0.0;
         double seed = 1.0;
-        fi_reverse_x<double, 1>(fwd + nf, nr, stk, tape, T, tid, ig, &seed);
+        fi_reverse_x<double, 1>(rev, stk + tid, tape + tid, T, ig + tid, &seed);
         double nsq = 0.0;
         bool ok = true;
         for (int k = 0; k < a.v; ++k) {
@@ -445,7 +445,7 @@ __global__ void __launch_bounds__(T) ft_sweep(FitArgs a, int q)
     {
         /* [instructions | constants | spill slots | tape | input gradients | reduction] */
         using V4 = FiV<double, 1>::V4;
-        FIns *ins = reinterpret_cast<FIns *>(sm);
+        FOp *ins = reinterpret_cast<FOp *>(sm);
         double *cd = reinterpret_cast<double *>(sm + 8 * (size_t)((a.xmaxins + 1) & ~1));
         V4 *stk = reinterpret_cast<V4 *>(cd + FT_MAX_CONST);
         V4 *tape = stk + (size_t)a.xslots * T;
@@ -475,7 +475,7 @@ __global__ void __launch_bounds__(T) ft_sweep(FitArgs a, int q)
             const int r0 = tile * FT_TILE_ROWS;
             const int r1 = min(a.n, r0 + FT_TILE_ROWS);
             double *pt = a.part + ((size_t)cand * a.ntiles + tile) * FT_PART_STRIDE;
-            ft_tile_icost_x<T>(a, ins, info.x, info.y, cd, stk, tape, ig, red, r0, r1, pt);
+            ft_tile_icost_x<T>(a, ins, ins + info.x, cd, stk, tape, ig, red, r0, r1, pt);
             __syncthreads();
         }
     }
@@ -727,8 +727,8 @@ __device__ __forceinline__ void ft_fold(const V *g, int R, int A, int w, int gid
    independently over their own rows; the tile's sum is a fixed-order sum
    over warps, written in the packed 4x4-block layout the controller reads. */
 template <typename V, int NR, int T, bool CORR>
-__device__ void ft_tile_asm(const FitArgs &a, const FIns *fwd, const FIns *rev, int nr, int p,
-                            int A, int slots, int ntape, const V *cv, unsigned char *region,
+__device__ void ft_tile_asm(const FitArgs &a, const FOp *fwd, const FOp *rev, int p, int A,
+                            int slots, int ntape, const V *cv, unsigned char *region,
                             double *red, int r0, int r1, double *pt, const V *ccols)
 {
     using F = FiV<V, NR>;
@@ -755,7 +755,8 @@ __device__ void ft_tile_asm(const FitArgs &a, const FIns *fwd, const FIns *rev, 
         for (int base = r0; base < r1; base += NR * A) {
             const int row = base + NR * tid;
             V pr[NR];
-            fi_forward<V, NR, true>(fwd, cv, cols, a.npad, row, stk, tape, A, tid, pr, ccols);
+            fi_forward<V, NR, true>(fwd, cv, cols + row, a.npad, stk + tid, tape + tid, A, pr,
+                                    ccols + row);
             FtRow rw[NR];
             V seed[NR];
             bool special = false;
@@ -767,7 +768,7 @@ __device__ void ft_tile_asm(const FitArgs &a, const FIns *fwd, const FIns *rev, 
                 seed[i] = (V)rw[i].seed;
                 special = special || rw[i].s_zero != 0.0f;
             }
-            const bool fin = fi_reverse<V, NR>(rev, nr, stk, tape, A, tid, gt, R, A, seed);
+            const bool fin = fi_reverse<V, NR>(rev, stk + tid, tape + tid, A, gt, R, A, seed);
             if (!fin || special) {
                 /* rare rows: a non-finite Jacobian entry (the row is dropped
                    from the Jacobian; in f32 it counts as failed), or a zero
@@ -853,7 +854,7 @@ __device__ void ft_tile_asm(const FitArgs &a, const FIns *fwd, const FIns *rev, 
 /* Objective of one tile in f32 or f64 (eval.cu:1808-1855): the forward
    sweep only; a row that is not finite costs 1e30. */
 template <typename V, int NR, int T>
-__device__ void ft_tile_loss(const FitArgs &a, const FIns *ins, const V *cv,
+__device__ void ft_tile_loss(const FitArgs &a, const FOp *ins, const V *cv,
                              typename FiV<V, NR>::V4 *stk, double *red, int r0, int r1, double *pt,
                              const V *ccols)
 {
@@ -863,7 +864,7 @@ __device__ void ft_tile_loss(const FitArgs &a, const FIns *ins, const V *cv,
     double local = 0.0;
     for (int row = r0 + NR * tid; row < r1; row += NR * T) {
         V pr[NR];
-        fi_forward<V, NR, false>(ins, cv, cols, a.npad, row, stk, nullptr, T, tid, pr, ccols);
+        fi_forward<V, NR, false>(ins, cv, cols + row, a.npad, stk + tid, nullptr, T, pr, ccols + row);
 #pragma unroll
         for (int i = 0; i < NR; ++i) {
             const int rr = row + i;
@@ -905,7 +906,7 @@ __device__ void ft_tile_loss(const FitArgs &a, const FIns *ins, const V *cv,
    prediction or target is not finite marks the tile bad, which rejects the
    trial. */
 template <int NR, int T>
-__device__ void ft_tile_corr_score(const FitArgs &a, const FIns *ins, const float *cv,
+__device__ void ft_tile_corr_score(const FitArgs &a, const FOp *ins, const float *cv,
                                    typename FiV<float, NR>::V4 *stk, double *red, int r0, int r1,
                                    double *pt, const float *ccols)
 {
@@ -914,7 +915,8 @@ __device__ void ft_tile_corr_score(const FitArgs &a, const FIns *ins, const floa
     int bad = 0;
     for (int row = r0 + NR * tid; row < r1; row += NR * T) {
         float pr[NR];
-        fi_forward<float, NR, false>(ins, cv, a.cols, a.npad, row, stk, nullptr, T, tid, pr, ccols);
+        fi_forward<float, NR, false>(ins, cv, a.cols + row, a.npad, stk + tid, nullptr, T, pr,
+                                     ccols + row);
 #pragma unroll
         for (int i = 0; i < NR; ++i) {
             const int rr = row + i;
@@ -956,7 +958,7 @@ __global__ void __launch_bounds__(T) ft_sweep4(FitArgs a, int q)
                                                                 : FT_LOSS64_NR;
     using V4 = typename FiV<V, NR>::V4;
     extern __shared__ __align__(16) unsigned char sm[];
-    FIns *ins = reinterpret_cast<FIns *>(sm);
+    FOp *ins = reinterpret_cast<FOp *>(sm);
     V *cv = reinterpret_cast<V *>(sm + 8 * (size_t)((a.fmaxins + 1) & ~1));
     unsigned char *region = reinterpret_cast<unsigned char *>(sm + 8 * (size_t)((a.fmaxins + 1) & ~1) +
                                                               8 * FT_MAX_CONST);
@@ -989,7 +991,7 @@ __global__ void __launch_bounds__(T) ft_sweep4(FitArgs a, int q)
         const bool CACHED = sizeof(V) == 4 || a.cache64 != nullptr;
         const int2 fc = CACHED ? a.fcinfo[cand] : make_int2(info.x, 0);
         const int nf = fc.x;
-        const FIns *fsrc = a.fins + ib + (CACHED ? info.x + nr : 0);
+        const FOp *fsrc = a.fins + ib + (CACHED ? info.x + nr : 0);
         const V *ccols =
             !CACHED ? nullptr
                     : (sizeof(V) == 4 ? reinterpret_cast<const V *>(a.cache)
@@ -1006,7 +1008,7 @@ __global__ void __launch_bounds__(T) ft_sweep4(FitArgs a, int q)
         const int r1 = min(a.n, r0 + FT_TILE_ROWS);
         double *pt = a.part + ((size_t)cand * a.ntiles + tile) * FT_PART_STRIDE;
         if (ft_op_assembles(OPK))
-            ft_tile_asm<V, NR, T, BK == FOP_CASM>(a, ins, ins + nf, nr, p, info.z & 0xffff,
+            ft_tile_asm<V, NR, T, BK == FOP_CASM>(a, ins, ins + nf, p, info.z & 0xffff,
                                                   info.w & 0xffff,
                                                   info.w >> 16, cv, region, red, r0, r1, pt, ccols);
         else if (BK == FOP_CSCORE)
@@ -1029,7 +1031,7 @@ __global__ void __launch_bounds__(FT_FILL_T) ft_cache_fill(FitArgs a)
 {
     using V4 = FiV<float, 4>::V4;
     extern __shared__ __align__(16) unsigned char sm[];
-    FIns *ins = reinterpret_cast<FIns *>(sm);
+    FOp *ins = reinterpret_cast<FOp *>(sm);
     V4 *stk = reinterpret_cast<V4 *>(sm + 8 * (size_t)((a.sub_maxins + 1) & ~1));
     const int s = blockIdx.x / a.ntiles, tile = blockIdx.x % a.ntiles;
     const int tid = threadIdx.x;
@@ -1040,7 +1042,7 @@ __global__ void __launch_bounds__(FT_FILL_T) ft_cache_fill(FitArgs a)
     float *out = a.cache + (size_t)a.sub_col[s] * a.npad;
     for (int row = r0 + 4 * tid; row < r1; row += 4 * FT_FILL_T) {
         float pr[4];
-        fi_forward<float, 4, false>(ins, nullptr, a.cols, a.npad, row, stk, nullptr, FT_FILL_T, tid,
+        fi_forward<float, 4, false>(ins, nullptr, a.cols + row, a.npad, stk + tid, nullptr, FT_FILL_T,
                                     pr);
 #pragma unroll
         for (int i = 0; i < 4; ++i)
@@ -1055,7 +1057,7 @@ __global__ void __launch_bounds__(FT_FILL_T) ft_cache_fill64(FitArgs a)
 {
     using V4 = FiV<double, 2>::V4;
     extern __shared__ __align__(16) unsigned char sm[];
-    FIns *ins = reinterpret_cast<FIns *>(sm);
+    FOp *ins = reinterpret_cast<FOp *>(sm);
     V4 *stk = reinterpret_cast<V4 *>(sm + 8 * (size_t)((a.sub_maxins + 1) & ~1));
     const int s = blockIdx.x / a.ntiles, tile = blockIdx.x % a.ntiles;
     const int tid = threadIdx.x;
@@ -1066,8 +1068,8 @@ __global__ void __launch_bounds__(FT_FILL_T) ft_cache_fill64(FitArgs a)
     double *out = a.cache64 + (size_t)a.sub_col[s] * a.npad;
     for (int row = r0 + 2 * tid; row < r1; row += 2 * FT_FILL_T) {
         double pr[2];
-        fi_forward<double, 2, false>(ins, nullptr, a.cols64, a.npad, row, stk, nullptr, FT_FILL_T,
-                                     tid, pr);
+        fi_forward<double, 2, false>(ins, nullptr, a.cols64 + row, a.npad, stk + tid, nullptr, FT_FILL_T,
+                                     pr);
 #pragma unroll
         for (int i = 0; i < 2; ++i)
             if (row + i < r1) out[row + i] = pr[i];
@@ -1920,7 +1922,7 @@ __global__ void __launch_bounds__(32) ft_grad4_kernel(FitArgs a, int row0, int n
     const int4 info = a.finfo[cand];
     const int nf = info.x, nr = info.y, slots = info.w & 0xffff, ntape = info.w >> 16;
     const int p = a.pcount[cand];
-    FIns *ins = reinterpret_cast<FIns *>(smem);
+    FOp *ins = reinterpret_cast<FOp *>(smem);
     float *cf = reinterpret_cast<float *>(smem + 8 * (size_t)((a.fmaxins + 1) & ~1));
     V4 *stk = reinterpret_cast<V4 *>(cf + FT_MAX_CONST);
     V4 *tape = stk + (size_t)slots * 32;
@@ -1935,8 +1937,8 @@ __global__ void __launch_bounds__(32) ft_grad4_kernel(FitArgs a, int row0, int n
     if (row >= row0 + nrows || row >= a.n) return;
     float pr[NR], seed[NR];
     for (int i = 0; i < NR; ++i) seed[i] = 1.0f;
-    fi_forward<float, NR, true>(ins, cf, a.cols, a.npad, row, stk, tape, 32, tid, pr);
-    fi_reverse<float, NR>(ins + nf, nr, stk, tape, 32, tid, g + tid, R, 32, seed);
+    fi_forward<float, NR, true>(ins, cf, a.cols + row, a.npad, stk + tid, tape + tid, 32, pr);
+    fi_reverse<float, NR>(ins + nf, stk + tid, tape + tid, 32, g + tid, R, 32, seed);
     for (int i = 0; i < NR; ++i) {
         const int rr = row + i;
         if (rr < row0 || rr >= row0 + nrows) continue;
@@ -1955,7 +1957,7 @@ __global__ void __launch_bounds__(32) ft_grad4_kernel(FitArgs a, int row0, int n
    weight, value, gradient or distance marks the candidate bad. */
 template <int T, int NR>
 __global__ void __launch_bounds__(T) ft_implicit_score_x(
-    const FIns *__restrict__ fins, const int *__restrict__ fins_off, const int4 *__restrict__ info,
+    const FOp *__restrict__ fins, const int *__restrict__ fins_off, const int4 *__restrict__ info,
     const int *__restrict__ valid, const double *__restrict__ c, int kmax,
     const float *__restrict__ cols, int npad, int n, int v, const double *__restrict__ w,
     int ntiles, int rows_per_tile, int maxins, int slots, int ntape, double *partial, int *bad)
@@ -1966,7 +1968,7 @@ __global__ void __launch_bounds__(T) ft_implicit_score_x(
     const int cand = blockIdx.x / ntiles;
     const int tile = blockIdx.x % ntiles;
     const int tid = threadIdx.x;
-    FIns *ins = reinterpret_cast<FIns *>(smem);
+    FOp *ins = reinterpret_cast<FOp *>(smem);
     float *cf = reinterpret_cast<float *>(smem + 8 * (size_t)((maxins + 1) & ~1));
     V4 *stk = reinterpret_cast<V4 *>(cf + FT_MAX_CONST);
     V4 *tape = stk + (size_t)(slots > 0 ? slots : 1) * T;
@@ -1985,7 +1987,7 @@ __global__ void __launch_bounds__(T) ft_implicit_score_x(
         __syncthreads();
         for (int row = r0 + NR * tid; row < r1; row += NR * T) {
             float pr[NR];
-            fi_forward<float, NR, true>(ins, cf, cols, npad, row, stk, tape, T, tid, pr);
+            fi_forward<float, NR, true>(ins, cf, cols + row, npad, stk + tid, tape + tid, T, pr);
             for (int k = 0; k < v; ++k) {
                 float z[NR];
 #pragma unroll
@@ -1995,7 +1997,7 @@ __global__ void __launch_bounds__(T) ft_implicit_score_x(
             float a[NR];
 #pragma unroll
             for (int i = 0; i < NR; ++i) a[i] = 1.0f;
-            fi_reverse_x<float, NR>(ins + nf, nr, stk, tape, T, tid, ig, a);
+            fi_reverse_x<float, NR>(ins + nf, stk + tid, tape + tid, T, ig + tid, a);
             double nsq[NR];
             bool gfin[NR];
 #pragma unroll
@@ -2174,13 +2176,16 @@ void prep_batch(const unsigned int *off, const unsigned int *prog, const int *pc
             b.valid[i] = 0;
             continue;
         }
-        b.fins.insert(b.fins.end(), fwd.begin(), fwd.end());
-        b.fins.insert(b.fins.end(), rev.begin(), rev.end());
+        const size_t base_f = b.fins.size();
+        fi_emit_forward(fwd, b.fins);
+        const size_t base_r = b.fins.size();
+        fi_emit_reverse(rev, false, b.fins);
+        const size_t base_c = b.fins.size();
         if (caching) {
             /* the cached list (or the full one again past the cap) */
             const bool fits = (size_t)(b.ncache + (int)subs.size()) * cache_bytes_per_col <= cache_cap;
             bool ok = fits && !subs.empty();
-            std::vector<FIns> cand_sub;
+            std::vector<FOp> cand_sub;
             std::vector<int> cand_off;
             int smax = 0, imax = 0;
             for (size_t s = 0; ok && s < subs.size(); ++s) {
@@ -2190,12 +2195,12 @@ void prep_batch(const unsigned int *off, const unsigned int *prog, const int *pc
                     break;
                 }
                 cand_off.push_back((int)cand_sub.size());
-                cand_sub.insert(cand_sub.end(), sf.begin(), sf.end());
+                fi_emit_forward(sf, cand_sub);
                 smax = std::max(smax, a2);
                 imax = std::max(imax, (int)sf.size());
             }
             const std::vector<FIns> &use = ok ? fwdc : fwd;
-            b.fins.insert(b.fins.end(), use.begin(), use.end());
+            fi_emit_forward(use, b.fins);
             b.fcinfo[i] = make_int2((int)use.size(), ok ? b.ncache : 0);
             if (ok) {
                 const int base = (int)b.sub_fins.size();
@@ -2211,7 +2216,7 @@ void prep_batch(const unsigned int *off, const unsigned int *prog, const int *pc
             }
         } else {
             /* no cache: the f32 list is the full one again */
-            b.fins.insert(b.fins.end(), fwd.begin(), fwd.end());
+            fi_emit_forward(fwd, b.fins);
             b.fcinfo[i] = make_int2((int)fwd.size(), 0);
         }
         const int ncols = pcount[i] + 1 + extra_cols;
@@ -2223,14 +2228,14 @@ void prep_batch(const unsigned int *off, const unsigned int *prog, const int *pc
         const size_t reg = ft_asm_region(A, ns, nt, 8 * ((ncols + 7) / 8));
         const int cls = ft_cls_of(A, reg);
         /* z: active threads, launch class above bit 16 */
-        b.finfo[i] = make_int4((int)fwd.size(), (int)rev.size(), A | (cls << 16),
+        b.finfo[i] = make_int4((int)(base_r - base_f), (int)(base_c - base_r), A | (cls << 16),
                                ns | (nt << 16));
         b.asm_region = std::max(b.asm_region, reg);
         b.asm_reg[cls] = std::max(b.asm_reg[cls], reg);
         b.nclass[cls]++;
         b.fslots = std::max(b.fslots, ns);
         b.ftape = std::max(b.ftape, nt);
-        b.fmaxins = std::max(b.fmaxins, (int)(fwd.size() + rev.size()));
+        b.fmaxins = std::max(b.fmaxins, (int)(base_c - base_f));
     }
     b.fins_off[nprog] = (int)b.fins.size();
     b.sub_cand_off[nprog] = (int)b.sub_col.size();
@@ -2280,7 +2285,7 @@ struct SweepLaunch {
    [forward | reverse] per candidate, counts and slot sizes in info. A
    candidate it cannot translate becomes invalid. */
 struct XPrep {
-    std::vector<FIns> fins;
+    std::vector<FOp> fins;
     std::vector<int> off;
     std::vector<int4> info;
     int slots = 1, tape = 1, maxins = 2;
@@ -2303,12 +2308,14 @@ void prep_inputs(const unsigned int *off, const unsigned int *prog, int nprog,
             valid[i] = 0;
             continue;
         }
-        x.fins.insert(x.fins.end(), fwd.begin(), fwd.end());
-        x.fins.insert(x.fins.end(), rev.begin(), rev.end());
-        x.info[i] = make_int4((int)fwd.size(), (int)rev.size(), ns, nt);
+        fi_emit_forward(fwd, x.fins);
+        const int nf = (int)x.fins.size() - x.off[i];
+        fi_emit_reverse(rev, true, x.fins);
+        const int nr = (int)x.fins.size() - x.off[i] - nf;
+        x.info[i] = make_int4(nf, nr, ns, nt);
         x.slots = std::max(x.slots, ns);
         x.tape = std::max(x.tape, nt);
-        x.maxins = std::max(x.maxins, (int)(fwd.size() + rev.size()));
+        x.maxins = std::max(x.maxins, nf + nr);
     }
     x.off[nprog] = (int)x.fins.size();
     if (x.fins.empty()) x.fins.resize(1);
@@ -2495,14 +2502,14 @@ float fit_run(RcCtx *c, const unsigned int *prog, const unsigned int *off, const
     const size_t o_c0 = rc_take(&cur, sizeof(double) * (size_t)nprog * kmax);
     const size_t o_valid = rc_take(&cur, sizeof(int) * nprog);
     const size_t o_gauge = rc_take(&cur, sizeof(int) * 2 * (size_t)nprog);
-    const size_t o_fins = rc_take(&cur, sizeof(FIns) * b.fins.size());
+    const size_t o_fins = rc_take(&cur, sizeof(FOp) * b.fins.size());
     const size_t o_finsoff = rc_take(&cur, sizeof(int) * (nprog + 1));
     const size_t o_finfo = rc_take(&cur, sizeof(int4) * nprog);
     const size_t o_fcinfo = rc_take(&cur, sizeof(int2) * nprog);
-    const size_t o_subf = rc_take(&cur, sizeof(FIns) * b.sub_fins.size());
+    const size_t o_subf = rc_take(&cur, sizeof(FOp) * b.sub_fins.size());
     const size_t o_suboff = rc_take(&cur, sizeof(int) * b.sub_off.size());
     const size_t o_subcol = rc_take(&cur, sizeof(int) * b.sub_col.size());
-    const size_t o_xfins = rc_take(&cur, sizeof(FIns) * xp.fins.size());
+    const size_t o_xfins = rc_take(&cur, sizeof(FOp) * xp.fins.size());
     const size_t o_xoff = rc_take(&cur, sizeof(int) * xp.off.size());
     const size_t o_xinfo = rc_take(&cur, sizeof(int4) * xp.info.size());
     const size_t in_end = rc_take(&cur, 0);
@@ -2533,14 +2540,14 @@ float fit_run(RcCtx *c, const unsigned int *prog, const unsigned int *off, const
     memcpy(host + o_valid, b.valid.data(), sizeof(int) * nprog);
     if (gauge) memcpy(host + o_gauge, gauge, sizeof(int) * 2 * (size_t)nprog);
     else memset(host + o_gauge, 0xff, sizeof(int) * 2 * (size_t)nprog);
-    memcpy(host + o_fins, b.fins.data(), sizeof(FIns) * b.fins.size());
+    memcpy(host + o_fins, b.fins.data(), sizeof(FOp) * b.fins.size());
     memcpy(host + o_finsoff, b.fins_off.data(), sizeof(int) * (nprog + 1));
     memcpy(host + o_finfo, b.finfo.data(), sizeof(int4) * nprog);
     memcpy(host + o_fcinfo, b.fcinfo.data(), sizeof(int2) * nprog);
-    memcpy(host + o_subf, b.sub_fins.data(), sizeof(FIns) * b.sub_fins.size());
+    memcpy(host + o_subf, b.sub_fins.data(), sizeof(FOp) * b.sub_fins.size());
     memcpy(host + o_suboff, b.sub_off.data(), sizeof(int) * b.sub_off.size());
     memcpy(host + o_subcol, b.sub_col.data(), sizeof(int) * b.sub_col.size());
-    memcpy(host + o_xfins, xp.fins.data(), sizeof(FIns) * xp.fins.size());
+    memcpy(host + o_xfins, xp.fins.data(), sizeof(FOp) * xp.fins.size());
     if (!xp.off.empty()) memcpy(host + o_xoff, xp.off.data(), sizeof(int) * xp.off.size());
     if (!xp.info.empty()) memcpy(host + o_xinfo, xp.info.data(), sizeof(int4) * xp.info.size());
     memcpy(host + o_c, c0, sizeof(double) * (size_t)nprog * kmax);
@@ -2566,19 +2573,19 @@ float fit_run(RcCtx *c, const unsigned int *prog, const unsigned int *off, const
     a.c0 = reinterpret_cast<const double *>(dev + o_c0);
     a.valid = reinterpret_cast<const int *>(dev + o_valid);
     a.gauge = reinterpret_cast<const int *>(dev + o_gauge);
-    a.fins = reinterpret_cast<const FIns *>(dev + o_fins);
+    a.fins = reinterpret_cast<const FOp *>(dev + o_fins);
     a.fins_off = reinterpret_cast<const int *>(dev + o_finsoff);
     a.finfo = reinterpret_cast<const int4 *>(dev + o_finfo);
     a.fcinfo = reinterpret_cast<const int2 *>(dev + o_fcinfo);
     a.cache = reinterpret_cast<float *>(dev + o_cache);
     a.cache64 = use64 ? reinterpret_cast<double *>(dev + o_cache64) : nullptr;
-    a.sub_fins = reinterpret_cast<const FIns *>(dev + o_subf);
+    a.sub_fins = reinterpret_cast<const FOp *>(dev + o_subf);
     a.sub_off = reinterpret_cast<const int *>(dev + o_suboff);
     a.sub_col = reinterpret_cast<const int *>(dev + o_subcol);
     a.nsub = (int)b.sub_off.size() - 1;
     a.sub_slots = b.sub_slots;
     a.sub_maxins = b.sub_maxins;
-    a.xfins = reinterpret_cast<const FIns *>(dev + o_xfins);
+    a.xfins = reinterpret_cast<const FOp *>(dev + o_xfins);
     a.xfins_off = reinterpret_cast<const int *>(dev + o_xoff);
     a.xinfo = reinterpret_cast<const int4 *>(dev + o_xinfo);
     a.xmaxins = xp.maxins;
@@ -3002,7 +3009,7 @@ int rc_grad_batch(void *ctx, const unsigned int *prog, const unsigned int *off, 
     const size_t o_val = rc_take(&cur, sizeof(float) * (size_t)nprog * nrows);
     const size_t o_out = rc_take(&cur, sizeof(float) * (size_t)nprog * nrows * width);
     const size_t io_end = rc_take(&cur, 0);
-    const size_t o_fins = rc_take(&cur, sizeof(FIns) * b.fins.size());
+    const size_t o_fins = rc_take(&cur, sizeof(FOp) * b.fins.size());
     const size_t o_finsoff = rc_take(&cur, sizeof(int) * (nprog + 1));
     const size_t o_finfo = rc_take(&cur, sizeof(int4) * nprog);
     const size_t dev_end = rc_take(&cur, 0);
@@ -3031,10 +3038,10 @@ int rc_grad_batch(void *ctx, const unsigned int *prog, const unsigned int *off, 
     if (want == 1) {
         /* the four-row sweeps of the f32 assembly */
         std::vector<unsigned char> stage(dev_end - io_end);
-        memcpy(stage.data() + (o_fins - io_end), b.fins.data(), sizeof(FIns) * b.fins.size());
+        memcpy(stage.data() + (o_fins - io_end), b.fins.data(), sizeof(FOp) * b.fins.size());
         memcpy(stage.data() + (o_finsoff - io_end), b.fins_off.data(), sizeof(int) * (nprog + 1));
         memcpy(stage.data() + (o_finfo - io_end), b.finfo.data(), sizeof(int4) * nprog);
-        a.fins = reinterpret_cast<const FIns *>(dev + o_fins);
+        a.fins = reinterpret_cast<const FOp *>(dev + o_fins);
         a.fins_off = reinterpret_cast<const int *>(dev + o_finsoff);
         a.finfo = reinterpret_cast<const int4 *>(dev + o_finfo);
         a.fmaxins = b.fmaxins;
@@ -3082,7 +3089,7 @@ float rc_implicit_score_batch(void *ctx, const unsigned int *prog, const unsigne
     /* the input-mode translation: partials and pruning along input paths */
     XPrep xp;
     prep_inputs(off, prog, nprog, b.node_off, b.valid, xp);
-    std::vector<FIns> &xfins = xp.fins;
+    std::vector<FOp> &xfins = xp.fins;
     std::vector<int> &xoff = xp.off;
     std::vector<int4> &xinfo = xp.info;
     const int slots = xp.slots, ntape = xp.tape, maxins = xp.maxins;
@@ -3091,7 +3098,7 @@ float rc_implicit_score_batch(void *ctx, const unsigned int *prog, const unsigne
     const int rows_per_tile = 16384;
     const int ntiles = (rc->n + rows_per_tile - 1) / rows_per_tile;
     size_t cur = 0;
-    const size_t o_fins = rc_take(&cur, sizeof(FIns) * xfins.size());
+    const size_t o_fins = rc_take(&cur, sizeof(FOp) * xfins.size());
     const size_t o_xoff = rc_take(&cur, sizeof(int) * (nprog + 1));
     const size_t o_info = rc_take(&cur, sizeof(int4) * nprog);
     const size_t o_c = rc_take(&cur, sizeof(double) * (size_t)nprog * kmax);
@@ -3106,7 +3113,7 @@ float rc_implicit_score_batch(void *ctx, const unsigned int *prog, const unsigne
     if (rc_reserve(rc, dev_end, io_end) != 0) return -1.0f;
     unsigned char *dev = rc->dev, *host = rc->host;
     double t = rc_now_ms();
-    memcpy(host + o_fins, xfins.data(), sizeof(FIns) * xfins.size());
+    memcpy(host + o_fins, xfins.data(), sizeof(FOp) * xfins.size());
     memcpy(host + o_xoff, xoff.data(), sizeof(int) * (nprog + 1));
     memcpy(host + o_info, xinfo.data(), sizeof(int4) * nprog);
     memcpy(host + o_c, c, sizeof(double) * (size_t)nprog * kmax);
@@ -3121,7 +3128,7 @@ float rc_implicit_score_batch(void *ctx, const unsigned int *prog, const unsigne
     cudaEventRecord(rc->t0, rc->s);
     rc->launches += 2;
     ft_implicit_score_x<128, NR><<<nprog * ntiles, T, smem, rc->s>>>(
-        reinterpret_cast<const FIns *>(dev + o_fins), reinterpret_cast<const int *>(dev + o_xoff),
+        reinterpret_cast<const FOp *>(dev + o_fins), reinterpret_cast<const int *>(dev + o_xoff),
         reinterpret_cast<const int4 *>(dev + o_info), reinterpret_cast<const int *>(dev + o_valid),
         reinterpret_cast<const double *>(dev + o_c), kmax, rc->d_cols, rc->npad, rc->n, rc->v,
         rc->d_w64, ntiles, rows_per_tile, maxins, slots, ntape,

@@ -277,6 +277,143 @@ inline bool fi_decode(const uint32_t *rec, int m, std::vector<FIns> &fwd, std::v
     return true;
 }
 
+/* ---- device instruction words --------------------------------------------
+ *
+ * What bounds the sweeps is the interpreter itself: ncu shows the ALU pipe at
+ * 40-52 % and the FMA and f64 pipes at 3-15 %, with most stalls fixed-latency
+ * waits, so decoding costs more than the arithmetic. The device runs an
+ * 8-byte form of the lists above in which the code names operator and operand
+ * kind together (one dispatch reaches straight-line code), the next word is
+ * loaded while the current one executes, and reverse steps that change
+ * nothing (a sum's one live operand) are dropped on the host. Lists end with
+ * FC_END / RC_END; a sweep may load (not run) the word after the end.
+ *
+ *   x: code | FO_* flags | z << 16    z: push: spill slot or FO_NONE; operator:
+ *                                        tape slot of the right partial;
+ *                                        FC_RARE: the operator
+ *   y: operand | w << 16              operand: spill slot, input column, cache
+ *                                        column or constant slot
+ *                                     w: tape slot of the left / only partial */
+struct FOp {
+    uint32_t x, y;
+};
+
+inline FOp fi_op(unsigned code, unsigned y, unsigned z, unsigned w)
+{
+    return FOp{code | (z << 16), y | (w << 16)};
+}
+
+#define FO_NONE 0xffffu
+#define FO_HP_L 256u  /* keep (or use) the left / only partial */
+#define FO_HP_R 512u  /* keep (or use) the right partial */
+#define FO_ACC 1024u  /* reverse: the constant's adjoint adds to an earlier one */
+#define FO_COL 2048u  /* DIV / POW: right operand an input column */
+#define FO_CON 4096u  /* DIV / POW: right operand a constant */
+
+enum FiCode {
+    FC_END = 0, FC_PUSH_V, FC_PUSH_C, FC_PUSH_P, FC_ADD_S, FC_ADD_V, FC_ADD_P, FC_SUB_S, FC_SUB_V,
+    FC_SUB_P, FC_MUL_S, FC_MUL_V, FC_MUL_P, FC_DIV, FC_POW, FC_NEG, FC_SQUARE, FC_SIN, FC_COS,
+    FC_EXP, FC_TANH, FC_SIG, FC_GAUSS, FC_RARE
+};
+
+enum RiCode {
+    RC_END = 0,
+    RC_RESTORE, /* a = slot y */
+    RC_PUSH_P,  /* constant y receives a; a = slot z */
+    RC_NEG,     /* a = -a */
+    RC_MUL,     /* a = child(a, tape w) */
+    RC_ADD2,    /* slot y = a (both operands live) */
+    RC_SUB2,    /* slot y = a; a = -a */
+    RC_MUL2,    /* slot y = child(a, tape w); a = child(a, tape z) */
+    RC_ADD_P,   /* constant y receives a */
+    RC_SUB_P,   /* constant y receives -a */
+    RC_MUL_P,   /* constant y receives child(a, tape z); a = child(a, tape w), or 0 */
+    RC_PUSH_X,  /* input y receives a; a = slot z */
+    RC_ADD_X,   /* input y receives a */
+    RC_SUB_X,   /* input y receives -a */
+    RC_MUL_X    /* input y receives child(a, tape z); a = child(a, tape w), or 0 */
+};
+
+/* Append the device words of a forward list (its FI_HALT becomes FC_END). */
+inline void fi_emit_forward(const std::vector<FIns> &fwd, std::vector<FOp> &out)
+{
+    for (const FIns &in : fwd) {
+        const unsigned k = in.kind & FI_KIND_MASK;
+        const unsigned fl = ((in.kind & FI_HP_L) ? FO_HP_L : 0u) | ((in.kind & FI_HP_R) ? FO_HP_R : 0u);
+        if (k <= FI_PUSH_CACHE) {
+            out.push_back(fi_op(k == FI_PUSH_VAR ? FC_PUSH_V : (k == FI_PUSH_PARAM ? FC_PUSH_P : FC_PUSH_C),
+                                in.imm, in.spill == 0xff ? FO_NONE : in.spill, 0));
+        } else if (k == FI_UNARY) {
+            unsigned code = FC_RARE;
+            switch (in.op) {
+                case OP_NEG: code = FC_NEG; break;
+                case OP_SQUARE: code = FC_SQUARE; break;
+                case OP_SIN: code = FC_SIN; break;
+                case OP_COS: code = FC_COS; break;
+                case OP_EXP: code = FC_EXP; break;
+                case OP_TANH: code = FC_TANH; break;
+                case OP_SIG: code = FC_SIG; break;
+                case OP_GAUSS: code = FC_GAUSS; break;
+                default: break;
+            }
+            out.push_back(fi_op(code | fl, 0, in.op, in.tape));
+        } else if (k != FI_HALT) {
+            const unsigned mode = k == FI_BIN_S ? 0 : (k == FI_BIN_V ? 1 : 2);
+            unsigned code;
+            if (in.op == OP_DIV || in.op == OP_POW)
+                code = (in.op == OP_DIV ? FC_DIV : FC_POW) |
+                       (mode == 1 ? FO_COL : (mode == 2 ? FO_CON : 0u));
+            else
+                code = (in.op == OP_ADD ? FC_ADD_S : (in.op == OP_SUB ? FC_SUB_S : FC_MUL_S)) + mode;
+            out.push_back(fi_op(code | fl, mode == 0 ? in.arg : in.imm,
+                                in.tape + ((in.kind & FI_HP_L) ? 1u : 0u), in.tape));
+        } else {
+            out.push_back(fi_op(FC_END, 0, 0, 0));
+        }
+    }
+}
+
+/* Append the device words of a reverse list, in the order the device walks
+   it (last to first), closed by RC_END. */
+inline void fi_emit_reverse(const std::vector<FIns> &rev, bool inputs, std::vector<FOp> &out)
+{
+    for (int j = (int)rev.size() - 1; j >= 0; --j) {
+        const FIns &in = rev[j];
+        const unsigned k = in.kind & FI_KIND_MASK;
+        const bool hl = in.kind & FI_HP_L, hr = in.kind & FI_HP_R;
+        const unsigned acc = (in.kind & FI_ACC) ? FO_ACC : 0u;
+        const unsigned spill = in.spill == 0xff ? FO_NONE : in.spill;
+        const unsigned tl = in.tape, tr = in.tape + (hl ? 1u : 0u);
+        if (k <= FI_PUSH_CACHE) {
+            if (inputs ? k == FI_PUSH_VAR : k == FI_PUSH_PARAM)
+                out.push_back(fi_op((inputs ? RC_PUSH_X : RC_PUSH_P) | acc, in.imm, spill, 0));
+            else if (spill != FO_NONE)
+                out.push_back(fi_op(RC_RESTORE, spill, 0, 0));
+            continue;
+        }
+        const bool add = in.op == OP_ADD, sub = in.op == OP_SUB;
+        if (k == FI_UNARY) {
+            out.push_back(fi_op(in.op == OP_NEG ? RC_NEG : RC_MUL, 0, 0, tl));
+        } else if (k == FI_BIN_S) {
+            if (hl && hr)
+                out.push_back(fi_op(add ? RC_ADD2 : (sub ? RC_SUB2 : RC_MUL2), in.arg, tr, tl));
+            else if (!add && !sub)
+                out.push_back(fi_op(RC_MUL, 0, 0, hr ? tr : tl));
+            else if (sub && hr)
+                out.push_back(fi_op(RC_NEG, 0, 0, 0));
+        } else if (inputs ? k == FI_BIN_V : k == FI_BIN_P) {
+            /* the right operand is a constant, or an input */
+            const unsigned code = inputs ? (add ? RC_ADD_X : (sub ? RC_SUB_X : RC_MUL_X))
+                                         : (add ? RC_ADD_P : (sub ? RC_SUB_P : RC_MUL_P)) | acc;
+            out.push_back(fi_op(code | (hl ? FO_HP_L : 0u), in.imm, tr, tl));
+        } else if (!add && !sub) {
+            /* (in an adjoint list its operator has a live left operand) */
+            out.push_back(fi_op(RC_MUL, 0, 0, tl));
+        }
+    }
+    out.push_back(fi_op(RC_END, 0, 0, 0));
+}
+
 /* Local partials of one operator (ft_partials_f / ft_partials_d semantics,
    with the operator's value `r` reused where it is the same expression). A
    `pow` with a non-positive base passes nothing. */
@@ -359,329 +496,350 @@ struct FiV {
     }
 };
 
+#define FI_COPY(d, s) _Pragma("unroll") for (int i_ = 0; i_ < NR; ++i_) d[i_] = s[i_]
+#define FI_CONST(d, c_)                                                            \
+    do {                                                                            \
+        const V fc_ = (c_);                                                         \
+        _Pragma("unroll") for (int i_ = 0; i_ < NR; ++i_) d[i_] = fc_;              \
+    } while (0)
+
 template <typename V>
 __device__ __forceinline__ V fi_child(V a, V d)
 {
     return a == V(0) ? V(0) : a * d;
 }
 
-/* One operator on the thread's rows: values, and with PARTIALS the
-   partials the instruction keeps. The operator is a compile-time constant in
-   each case, so the value and partial switches fold away. */
-#define FI_OPN(OPC)                                                                   \
-    case OPC: {                                                                       \
-        _Pragma("unroll") for (int i = 0; i < NR; ++i) r[i] = F::value(OPC, a[i], b[i]); \
-        if (PARTIALS && fi_nonlinear(OPC) && (kind & (FI_HP_L | FI_HP_R))) {          \
-            V pl[NR], pr[NR];                                                         \
-            _Pragma("unroll") for (int i = 0; i < NR; ++i)                            \
-                fi_partials<V>(OPC, a[i], b[i], r[i], pl[i], pr[i]);                  \
-            int ts = in.tape;                                                         \
-            if (kind & FI_HP_L) {                                                     \
-                tape[ts * S + tid] = F::pack(pl);                             \
-                ++ts;                                                                 \
-            }                                                                         \
-            if (kind & FI_HP_R) tape[ts * S + tid] = F::pack(pr);             \
-        }                                                                             \
-    } break;
+/* Keep the thread's partials of one operator: `d` by tape slot. */
+template <typename V, int NR>
+__device__ __forceinline__ void fi_keep(typename FiV<V, NR>::V4 *tape, unsigned slot, int S,
+                                        const V *d)
+{
+    tape[slot * S] = FiV<V, NR>::pack(d);
+}
 
-/* Forward sweep of the thread's NR rows. Constants from `cf`, inputs from
-   the columns at `row` (aligned to the row vector), cached subtree values
-   from `ccols` (same stride). Spill slots and the tape are [slot][S] row
-   vectors with this thread at `tid`. The prediction of row i is left in
-   out[i]. */
+/* A unary operator on the thread's rows: value, and with PARTIALS the
+   partial when the word keeps it. */
+#define FI_UN(OPC)                                                                     \
+    {                                                                                  \
+        V r[NR];                                                                       \
+        _Pragma("unroll") for (int i = 0; i < NR; ++i) r[i] = F::value(OPC, t[i], V(0)); \
+        if (PARTIALS && (in.x & FO_HP_L)) {                                            \
+            V pl[NR], pr[NR];                                                          \
+            _Pragma("unroll") for (int i = 0; i < NR; ++i)                             \
+                fi_partials<V>(OPC, t[i], V(0), r[i], pl[i], pr[i]);                   \
+            fi_keep<V, NR>(tape, (in.y >> 16), S, pl);                                         \
+        }                                                                              \
+        _Pragma("unroll") for (int i = 0; i < NR; ++i) t[i] = r[i];                    \
+    }
+
+/* t = a op b for an exact binary operator, its partials (of a product) kept. */
+#define FI_BI(EXPR, PRODUCT)                                                           \
+    {                                                                                  \
+        if (PARTIALS && (PRODUCT)) {                                                   \
+            if (in.x & FO_HP_L) fi_keep<V, NR>(tape, (in.y >> 16), S, b);                      \
+            if (in.x & FO_HP_R) fi_keep<V, NR>(tape, (in.x >> 16), S, a);                      \
+        }                                                                              \
+        _Pragma("unroll") for (int i = 0; i < NR; ++i) t[i] = (EXPR);                  \
+    }
+
+/* Forward sweep of the thread's NR rows over a forward list. Constants from
+   `cf`, inputs from `cols` (already at the thread's first row) with columns
+   `npad` values apart, cached subtree values from `ccols` likewise. `stk`
+   and `tape` are this thread's spill and tape row vectors, slots S apart.
+   The prediction of row i is left in out[i]. */
 template <typename V, int NR, bool PARTIALS>
-__device__ __forceinline__ void fi_forward(const FIns *__restrict__ prog, const V *cf,
-                                           const V *__restrict__ cols, int npad, int row,
+__device__ __forceinline__ void fi_forward(const FOp *__restrict__ prog, const V *cf,
+                                           const V *__restrict__ cols, unsigned npad,
                                            typename FiV<V, NR>::V4 *stk,
-                                           typename FiV<V, NR>::V4 *tape, int S, int tid, V *out,
+                                           typename FiV<V, NR>::V4 *tape, int S, V *out,
                                            const V *__restrict__ ccols = nullptr)
 {
     using F = FiV<V, NR>;
+    auto column = [&](const V *base, unsigned k, V *v) {
+        F::ldg(base + (unsigned long long)k * npad, v);
+    };
     V t[NR];
 #pragma unroll
     for (int i = 0; i < NR; ++i) t[i] = V(0);
-    for (int pc = 0; pc < 512; ++pc) {
-        const FIns in = prog[pc];
-        const unsigned kind = in.kind;
-        const unsigned k = kind & FI_KIND_MASK;
-        if (k <= FI_PUSH_CACHE) {
-            if (in.spill != 0xff) stk[in.spill * S + tid] = F::pack(t);
-            if (k == FI_PUSH_VAR) {
-                F::ldg(cols + (size_t)in.imm * (size_t)npad + row, t);
-            } else if (k == FI_PUSH_CACHE) {
-                F::ldg(ccols + (size_t)in.imm * (size_t)npad + row, t);
-            } else {
-                const V c = cf[in.imm];
+    FOp in = *prog;
+    for (;;) {
+        const FOp nx = *++prog;
+        const unsigned code = in.x & 0xffu;
+        switch (code) {
+            case FC_PUSH_V:
+                if ((in.x >> 16) != FO_NONE) stk[(in.x >> 16) * S] = F::pack(t);
+                column(cols, (in.y & 0xffffu), t);
+                break;
+            case FC_PUSH_C:
+                if ((in.x >> 16) != FO_NONE) stk[(in.x >> 16) * S] = F::pack(t);
+                column(ccols, (in.y & 0xffffu), t);
+                break;
+            case FC_PUSH_P:
+                if ((in.x >> 16) != FO_NONE) stk[(in.x >> 16) * S] = F::pack(t);
+                FI_CONST(t, cf[(in.y & 0xffffu)]);
+                break;
+            case FC_ADD_S: { V a[NR], b[NR]; F::unpack(stk[(in.y & 0xffffu) * S], a); FI_COPY(b, t); FI_BI(a[i] + b[i], false) } break;
+            case FC_SUB_S: { V a[NR], b[NR]; F::unpack(stk[(in.y & 0xffffu) * S], a); FI_COPY(b, t); FI_BI(a[i] - b[i], false) } break;
+            case FC_MUL_S: { V a[NR], b[NR]; F::unpack(stk[(in.y & 0xffffu) * S], a); FI_COPY(b, t); FI_BI(a[i] * b[i], true) } break;
+            case FC_ADD_V: { V a[NR], b[NR]; column(cols, (in.y & 0xffffu), b); FI_COPY(a, t); FI_BI(a[i] + b[i], false) } break;
+            case FC_SUB_V: { V a[NR], b[NR]; column(cols, (in.y & 0xffffu), b); FI_COPY(a, t); FI_BI(a[i] - b[i], false) } break;
+            case FC_MUL_V: { V a[NR], b[NR]; column(cols, (in.y & 0xffffu), b); FI_COPY(a, t); FI_BI(a[i] * b[i], true) } break;
+            case FC_ADD_P: { V a[NR], b[NR]; FI_CONST(b, cf[(in.y & 0xffffu)]); FI_COPY(a, t); FI_BI(a[i] + b[i], false) } break;
+            case FC_SUB_P: { V a[NR], b[NR]; FI_CONST(b, cf[(in.y & 0xffffu)]); FI_COPY(a, t); FI_BI(a[i] - b[i], false) } break;
+            case FC_MUL_P: { V a[NR], b[NR]; FI_CONST(b, cf[(in.y & 0xffffu)]); FI_COPY(a, t); FI_BI(a[i] * b[i], true) } break;
+            case FC_DIV:
+            case FC_POW: {
+                V a[NR], b[NR], r[NR];
+                if (in.x & (FO_COL | FO_CON)) {
+                    FI_COPY(a, t);
+                    if (in.x & FO_COL) column(cols, (in.y & 0xffffu), b);
+                    else FI_CONST(b, cf[(in.y & 0xffffu)]);
+                } else {
+                    F::unpack(stk[(in.y & 0xffffu) * S], a);
+                    FI_COPY(b, t);
+                }
+                if (code == FC_DIV) {
 #pragma unroll
-                for (int i = 0; i < NR; ++i) t[i] = c;
-            }
-            continue;
-        }
-        if (k == FI_HALT) break;
-        V a[NR], b[NR];
-        if (k == FI_BIN_S) {
-            F::unpack(stk[in.arg * S + tid], a);
+                    for (int i = 0; i < NR; ++i) r[i] = F::value(OP_DIV, a[i], b[i]);
+                    if (PARTIALS && (in.x & FO_HP_L)) {
+                        V d[NR], e[NR];
 #pragma unroll
-            for (int i = 0; i < NR; ++i) b[i] = t[i];
-        } else {
-#pragma unroll
-            for (int i = 0; i < NR; ++i) {
-                a[i] = t[i];
-                b[i] = V(0);
-            }
-            if (k == FI_BIN_V) {
-                F::ldg(cols + (size_t)in.imm * (size_t)npad + row, b);
-            } else if (k == FI_BIN_P) {
-                const V c = cf[in.imm];
-#pragma unroll
-                for (int i = 0; i < NR; ++i) b[i] = c;
-            }
-        }
-        V r[NR];
-        switch (in.op) {
-            FI_OPN(OP_ADD) FI_OPN(OP_SUB) FI_OPN(OP_MUL) FI_OPN(OP_DIV) FI_OPN(OP_POW)
-            case OP_SIN:
-            case OP_COS:
-                if (sizeof(V) == 4 && PARTIALS && (kind & FI_HP_L)) {
-                    /* one f32 sincosf gives the value and the partial (its
-                       results equal sinf / cosf bit for bit on B200) */
-                    V pl[NR];
-                    const bool is_sin = in.op == OP_SIN;
-#pragma unroll
-                    for (int i = 0; i < NR; ++i) {
-                        float s, c;
-                        sincosf((float)a[i], &s, &c);
-                        r[i] = is_sin ? s : c;
-                        pl[i] = is_sin ? c : -s;
+                        for (int i = 0; i < NR; ++i) fi_partials<V>(OP_DIV, a[i], b[i], r[i], d[i], e[i]);
+                        fi_keep<V, NR>(tape, (in.y >> 16), S, d);
                     }
-                    tape[in.tape * S + tid] = F::pack(pl);
-                } else if (in.op == OP_SIN) {
+                    if (PARTIALS && (in.x & FO_HP_R)) {
+                        V d[NR], e[NR];
 #pragma unroll
-                    for (int i = 0; i < NR; ++i) r[i] = F::value(OP_SIN, a[i], b[i]);
-                    if (PARTIALS && (kind & FI_HP_L)) {
-                        V pl[NR];
-#pragma unroll
-                        for (int i = 0; i < NR; ++i) pl[i] = cos(a[i]);
-                        tape[in.tape * S + tid] = F::pack(pl);
+                        for (int i = 0; i < NR; ++i) fi_partials<V>(OP_DIV, a[i], b[i], r[i], d[i], e[i]);
+                        fi_keep<V, NR>(tape, (in.x >> 16), S, e);
                     }
                 } else {
 #pragma unroll
-                    for (int i = 0; i < NR; ++i) r[i] = F::value(OP_COS, a[i], b[i]);
-                    if (PARTIALS && (kind & FI_HP_L)) {
-                        V pl[NR];
+                    for (int i = 0; i < NR; ++i) r[i] = F::value(OP_POW, a[i], b[i]);
+                    if (PARTIALS && (in.x & (FO_HP_L | FO_HP_R))) {
+                        V d[NR], e[NR];
 #pragma unroll
-                        for (int i = 0; i < NR; ++i) pl[i] = -sin(a[i]);
-                        tape[in.tape * S + tid] = F::pack(pl);
+                        for (int i = 0; i < NR; ++i) fi_partials<V>(OP_POW, a[i], b[i], r[i], d[i], e[i]);
+                        if (in.x & FO_HP_L) fi_keep<V, NR>(tape, (in.y >> 16), S, d);
+                        if (in.x & FO_HP_R) fi_keep<V, NR>(tape, (in.x >> 16), S, e);
                     }
                 }
-                break;
-            FI_OPN(OP_TAN) FI_OPN(OP_EXP) FI_OPN(OP_LOG)
-            FI_OPN(OP_SQRT) FI_OPN(OP_ABS) FI_OPN(OP_TANH) FI_OPN(OP_SIG) FI_OPN(OP_SQUARE)
-            FI_OPN(OP_CUBE) FI_OPN(OP_NEG) FI_OPN(OP_GAUSS) FI_OPN(OP_SINH) FI_OPN(OP_COSH)
-            FI_OPN(OP_ERF) FI_OPN(OP_ERFC)
-            default:
+                FI_COPY(t, r);
+            } break;
+            case FC_NEG:
 #pragma unroll
-                for (int i = 0; i < NR; ++i) r[i] = V(NAN);
+                for (int i = 0; i < NR; ++i) t[i] = -t[i];
                 break;
+            case FC_SQUARE: FI_UN(OP_SQUARE) break;
+            case FC_SIN:
+            case FC_COS: {
+                const bool is_sin = code == FC_SIN;
+                V r[NR];
+                if (PARTIALS && (in.x & FO_HP_L)) {
+                    V pl[NR];
+#pragma unroll
+                    for (int i = 0; i < NR; ++i) {
+                        if (sizeof(V) == 4) {
+                            /* one f32 sincosf gives the value and the partial
+                               (its results equal sinf / cosf bit for bit on
+                               B200) */
+                            float s, c;
+                            sincosf((float)t[i], &s, &c);
+                            r[i] = is_sin ? s : c;
+                            pl[i] = is_sin ? c : -s;
+                        } else if (is_sin) {
+                            r[i] = F::value(OP_SIN, t[i], V(0));
+                            pl[i] = cos(t[i]);
+                        } else {
+                            r[i] = F::value(OP_COS, t[i], V(0));
+                            pl[i] = -sin(t[i]);
+                        }
+                    }
+                    fi_keep<V, NR>(tape, (in.y >> 16), S, pl);
+                } else if (is_sin) {
+#pragma unroll
+                    for (int i = 0; i < NR; ++i) r[i] = F::value(OP_SIN, t[i], V(0));
+                } else {
+#pragma unroll
+                    for (int i = 0; i < NR; ++i) r[i] = F::value(OP_COS, t[i], V(0));
+                }
+                FI_COPY(t, r);
+            } break;
+            case FC_EXP: FI_UN(OP_EXP) break;
+            case FC_TANH: FI_UN(OP_TANH) break;
+            case FC_SIG: FI_UN(OP_SIG) break;
+            case FC_GAUSS: FI_UN(OP_GAUSS) break;
+            case FC_RARE:
+                switch (in.x >> 16) {
+                    case OP_TAN: FI_UN(OP_TAN) break;
+                    case OP_LOG: FI_UN(OP_LOG) break;
+                    case OP_SQRT: FI_UN(OP_SQRT) break;
+                    case OP_ABS: FI_UN(OP_ABS) break;
+                    case OP_CUBE: FI_UN(OP_CUBE) break;
+                    case OP_SINH: FI_UN(OP_SINH) break;
+                    case OP_COSH: FI_UN(OP_COSH) break;
+                    case OP_ERF: FI_UN(OP_ERF) break;
+                    case OP_ERFC: FI_UN(OP_ERFC) break;
+                    default: FI_CONST(t, V(NAN)); break;
+                }
+                break;
+            default: /* FC_END */
+#pragma unroll
+                for (int i = 0; i < NR; ++i) out[i] = t[i];
+                return;
         }
-#pragma unroll
-        for (int i = 0; i < NR; ++i) t[i] = r[i];
+        in = nx;
     }
-#pragma unroll
-    for (int i = 0; i < NR; ++i) out[i] = t[i];
 }
-#undef FI_OPN
+#undef FI_UN
+#undef FI_BI
 
-/* Reverse sweep of the thread's rows over the reverse list (`nr` entries,
-   walked from the last). The adjoints start at the rows' seeds `a`.
-   Constant adjoints are stored to g[slot * R + i * A] for row i (`g` is
-   this thread's first row). Returns whether every stored value is
-   finite. */
+/* Reverse sweep of the thread's rows over a reverse list. The adjoints start
+   at the rows' seeds `a`. Constant adjoints are stored to g[slot * R + i * A]
+   for row i (`g` is this thread's first row). Returns whether every stored
+   value is finite. */
 template <typename V, int NR>
-__device__ __forceinline__ bool fi_reverse(const FIns *__restrict__ rev, int nr,
+__device__ __forceinline__ bool fi_reverse(const FOp *__restrict__ rev,
                                            typename FiV<V, NR>::V4 *stk,
-                                           const typename FiV<V, NR>::V4 *tape, int S, int tid,
-                                           V *g, int R, int A, V *a)
+                                           const typename FiV<V, NR>::V4 *tape, int S, V *g, int R,
+                                           int A, V *a)
 {
     using F = FiV<V, NR>;
     bool fin = true;
-    for (int pc = nr - 1; pc >= 0; --pc) {
-        const FIns in = rev[pc];
-        const unsigned kind = in.kind;
-        const unsigned k = kind & FI_KIND_MASK;
-        if (k <= FI_PUSH_CACHE) {
-            if (k == FI_PUSH_PARAM) {
-                V *gs = g + in.imm * R;
+    auto give = [&](unsigned x, unsigned slot, const V *r) {
+        V *gs = g + slot * R;
 #pragma unroll
-                for (int i = 0; i < NR; ++i) {
-                    const V v = (kind & FI_ACC) ? a[i] + gs[i * A] : a[i];
-                    gs[i * A] = v;
-                    fin = fin && isfinite(v);
-                }
-            }
-            if (in.spill != 0xff) F::unpack(stk[in.spill * S + tid], a);
-            continue;
+        for (int i = 0; i < NR; ++i) {
+            const V v = (x & FO_ACC) ? r[i] + gs[i * A] : r[i];
+            gs[i * A] = v;
+            fin = fin && isfinite(v);
         }
-        if (k == FI_UNARY) {
-            if (in.op == OP_NEG) {
+    };
+    auto child = [&](unsigned slot, V *o) {
+        V d[NR];
+        F::unpack(tape[slot * S], d);
+#pragma unroll
+        for (int i = 0; i < NR; ++i) o[i] = fi_child(a[i], d[i]);
+    };
+    FOp in = *rev;
+    for (;;) {
+        const FOp nx = *++rev;
+        switch (in.x & 0xffu) {
+            case RC_RESTORE: F::unpack(stk[(in.y & 0xffffu) * S], a); break;
+            case RC_PUSH_P:
+                give(in.x, (in.y & 0xffffu), a);
+                if ((in.x >> 16) != FO_NONE) F::unpack(stk[(in.x >> 16) * S], a);
+                break;
+            case RC_NEG:
 #pragma unroll
                 for (int i = 0; i < NR; ++i) a[i] = -a[i];
-            } else {
-                V d[NR];
-                F::unpack(tape[in.tape * S + tid], d);
+                break;
+            case RC_MUL: child((in.y >> 16), a); break;
+            case RC_ADD2: stk[(in.y & 0xffffu) * S] = F::pack(a); break;
+            case RC_SUB2:
+                stk[(in.y & 0xffffu) * S] = F::pack(a);
 #pragma unroll
-                for (int i = 0; i < NR; ++i) a[i] = fi_child(a[i], d[i]);
-            }
-            continue;
-        }
-        /* binary: left adjoint l, right adjoint r, for the sides with a
-           constant */
-        V l[NR], r[NR];
-        if (in.op == OP_ADD || in.op == OP_SUB) {
-            const bool sub = in.op == OP_SUB;
-#pragma unroll
-            for (int i = 0; i < NR; ++i) {
-                l[i] = a[i];
-                r[i] = sub ? -a[i] : a[i];
-            }
-        } else {
-            int ts = in.tape;
-#pragma unroll
-            for (int i = 0; i < NR; ++i) l[i] = r[i] = V(0);
-            if (kind & FI_HP_L) {
-                V d[NR];
-                F::unpack(tape[ts * S + tid], d);
-#pragma unroll
-                for (int i = 0; i < NR; ++i) l[i] = fi_child(a[i], d[i]);
-                ++ts;
-            }
-            if (kind & FI_HP_R) {
-                V d[NR];
-                F::unpack(tape[ts * S + tid], d);
-#pragma unroll
-                for (int i = 0; i < NR; ++i) r[i] = fi_child(a[i], d[i]);
-            }
-        }
-        if (k == FI_BIN_S) {
-            if ((kind & FI_HP_L) && (kind & FI_HP_R)) {
+                for (int i = 0; i < NR; ++i) a[i] = -a[i];
+                break;
+            case RC_MUL2: {
                 /* the left adjoint waits in its spill slot while the right
                    subtree is walked; that subtree's first push restores it */
-                stk[in.arg * S + tid] = F::pack(l);
+                V l[NR];
+                child((in.y >> 16), l);
+                child((in.x >> 16), a);
+                stk[(in.y & 0xffffu) * S] = F::pack(l);
+            } break;
+            case RC_ADD_P: give(in.x, (in.y & 0xffffu), a); break;
+            case RC_SUB_P: {
+                V r[NR];
 #pragma unroll
-                for (int i = 0; i < NR; ++i) a[i] = r[i];
-            } else if (kind & FI_HP_R) {
-#pragma unroll
-                for (int i = 0; i < NR; ++i) a[i] = r[i];
-            } else {
-#pragma unroll
-                for (int i = 0; i < NR; ++i) a[i] = l[i];
-            }
-        } else {
-            if (k == FI_BIN_P) {
-                V *gs = g + in.imm * R;
-#pragma unroll
-                for (int i = 0; i < NR; ++i) {
-                    const V v = (kind & FI_ACC) ? r[i] + gs[i * A] : r[i];
-                    gs[i * A] = v;
-                    fin = fin && isfinite(v);
-                }
-            }
-#pragma unroll
-            for (int i = 0; i < NR; ++i) a[i] = l[i];
+                for (int i = 0; i < NR; ++i) r[i] = -a[i];
+                give(in.x, (in.y & 0xffffu), r);
+            } break;
+            case RC_MUL_P: {
+                V r[NR];
+                child((in.x >> 16), r);
+                give(in.x, (in.y & 0xffffu), r);
+                if (in.x & FO_HP_L) child((in.y >> 16), a);
+                else FI_CONST(a, V(0));
+            } break;
+            default: return fin; /* RC_END */
         }
+        in = nx;
     }
-    return fin;
 }
 
 /* Reverse sweep of the thread's rows over an input-mode reverse list (see
    fi_decode): the same stack machine as fi_reverse, seeded with a[], whose
-   input leaves add their adjoints to the thread's gradient rows
-   ig[col * S + tid] (zeroed by the caller). Constants receive nothing. */
+   input leaves add their adjoints to the thread's gradient row vectors
+   ig[col * S] (zeroed by the caller). Constants receive nothing. */
 template <typename V, int NR>
-__device__ __forceinline__ void fi_reverse_x(const FIns *__restrict__ rev, int nr,
+__device__ __forceinline__ void fi_reverse_x(const FOp *__restrict__ rev,
                                              typename FiV<V, NR>::V4 *stk,
-                                             const typename FiV<V, NR>::V4 *tape, int S, int tid,
+                                             const typename FiV<V, NR>::V4 *tape, int S,
                                              typename FiV<V, NR>::V4 *ig, V *a)
 {
     using F = FiV<V, NR>;
-    for (int pc = nr - 1; pc >= 0; --pc) {
-        const FIns in = rev[pc];
-        const unsigned kind = in.kind;
-        const unsigned k = kind & FI_KIND_MASK;
-        if (k <= FI_PUSH_CACHE) {
-            if (k == FI_PUSH_VAR) {
-                V gv[NR];
-                F::unpack(ig[in.imm * S + tid], gv);
+    auto give = [&](unsigned col, const V *r) {
+        V gv[NR];
+        F::unpack(ig[col * S], gv);
 #pragma unroll
-                for (int i = 0; i < NR; ++i) gv[i] += a[i];
-                ig[in.imm * S + tid] = F::pack(gv);
-            }
-            if (in.spill != 0xff) F::unpack(stk[in.spill * S + tid], a);
-            continue;
-        }
-        if (k == FI_UNARY) {
-            if (in.op == OP_NEG) {
+        for (int i = 0; i < NR; ++i) gv[i] += r[i];
+        ig[col * S] = F::pack(gv);
+    };
+    auto child = [&](unsigned slot, V *o) {
+        V d[NR];
+        F::unpack(tape[slot * S], d);
+#pragma unroll
+        for (int i = 0; i < NR; ++i) o[i] = fi_child(a[i], d[i]);
+    };
+    FOp in = *rev;
+    for (;;) {
+        const FOp nx = *++rev;
+        switch (in.x & 0xffu) {
+            case RC_RESTORE: F::unpack(stk[(in.y & 0xffffu) * S], a); break;
+            case RC_PUSH_X:
+                give((in.y & 0xffffu), a);
+                if ((in.x >> 16) != FO_NONE) F::unpack(stk[(in.x >> 16) * S], a);
+                break;
+            case RC_NEG:
 #pragma unroll
                 for (int i = 0; i < NR; ++i) a[i] = -a[i];
-            } else {
-                V d[NR];
-                F::unpack(tape[in.tape * S + tid], d);
+                break;
+            case RC_MUL: child((in.y >> 16), a); break;
+            case RC_ADD2: stk[(in.y & 0xffffu) * S] = F::pack(a); break;
+            case RC_SUB2:
+                stk[(in.y & 0xffffu) * S] = F::pack(a);
 #pragma unroll
-                for (int i = 0; i < NR; ++i) a[i] = fi_child(a[i], d[i]);
-            }
-            continue;
+                for (int i = 0; i < NR; ++i) a[i] = -a[i];
+                break;
+            case RC_MUL2: {
+                V l[NR];
+                child((in.y >> 16), l);
+                child((in.x >> 16), a);
+                stk[(in.y & 0xffffu) * S] = F::pack(l);
+            } break;
+            case RC_ADD_X: give((in.y & 0xffffu), a); break;
+            case RC_SUB_X: {
+                V r[NR];
+#pragma unroll
+                for (int i = 0; i < NR; ++i) r[i] = -a[i];
+                give((in.y & 0xffffu), r);
+            } break;
+            case RC_MUL_X: {
+                V r[NR];
+                child((in.x >> 16), r);
+                give((in.y & 0xffffu), r);
+                if (in.x & FO_HP_L) child((in.y >> 16), a);
+                else FI_CONST(a, V(0));
+            } break;
+            default: return; /* RC_END */
         }
-        V l[NR], r[NR];
-        if (in.op == OP_ADD || in.op == OP_SUB) {
-            const bool sub = in.op == OP_SUB;
-#pragma unroll
-            for (int i = 0; i < NR; ++i) {
-                l[i] = a[i];
-                r[i] = sub ? -a[i] : a[i];
-            }
-        } else {
-            int ts = in.tape;
-#pragma unroll
-            for (int i = 0; i < NR; ++i) l[i] = r[i] = V(0);
-            if (kind & FI_HP_L) {
-                V d[NR];
-                F::unpack(tape[ts * S + tid], d);
-#pragma unroll
-                for (int i = 0; i < NR; ++i) l[i] = fi_child(a[i], d[i]);
-                ++ts;
-            }
-            if (kind & FI_HP_R) {
-                V d[NR];
-                F::unpack(tape[ts * S + tid], d);
-#pragma unroll
-                for (int i = 0; i < NR; ++i) r[i] = fi_child(a[i], d[i]);
-            }
-        }
-        if (k == FI_BIN_S) {
-            if ((kind & FI_HP_L) && (kind & FI_HP_R)) {
-                stk[in.arg * S + tid] = F::pack(l);
-#pragma unroll
-                for (int i = 0; i < NR; ++i) a[i] = r[i];
-            } else if (kind & FI_HP_R) {
-#pragma unroll
-                for (int i = 0; i < NR; ++i) a[i] = r[i];
-            } else {
-#pragma unroll
-                for (int i = 0; i < NR; ++i) a[i] = l[i];
-            }
-        } else {
-            if (k == FI_BIN_V) {
-                V gv[NR];
-                F::unpack(ig[in.imm * S + tid], gv);
-#pragma unroll
-                for (int i = 0; i < NR; ++i) gv[i] += r[i];
-                ig[in.imm * S + tid] = F::pack(gv);
-            }
-#pragma unroll
-            for (int i = 0; i < NR; ++i) a[i] = l[i];
-        }
+        in = nx;
     }
 }
+#undef FI_COPY
+#undef FI_CONST
 
 /* D = A * B + D for one 8x8x4 f64 tile (mma.sync; A row-major, B
    column-major). Lane (g = lane / 4, t = lane % 4) holds A[g][t], B[t][g]

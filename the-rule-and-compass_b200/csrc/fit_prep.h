@@ -13,7 +13,7 @@
 struct FitPrep {
     std::vector<int> node_off, valid; /* record offsets [P+1]; 1 = accepted */
     std::vector<int> ninternal;       /* per candidate: records that are not leaves */
-    std::vector<FIns> fins;           /* per candidate: forward list | reverse list */
+    std::vector<FOp> fins;            /* per candidate: forward list | reverse list */
     std::vector<int> fins_off;        /* [P+1] */
     std::vector<int4> finfo;          /* forward count, reverse count, assembly threads |
                                          launch class << 16, spill slots | tape slots << 16 */
@@ -29,7 +29,7 @@ struct FitPrep {
     /* constant-free subtree cache (requested by prep_batch's cache_npad) */
     std::vector<int2> fcinfo;         /* per candidate: cached forward count (the list
                                          follows the reverse list), first cache column */
-    std::vector<FIns> sub_fins;       /* forward lists of the cached subtrees */
+    std::vector<FOp> sub_fins;        /* forward lists of the cached subtrees */
     std::vector<int> sub_off;         /* [nsub + 1] */
     std::vector<int> sub_col;         /* [nsub] cache column of each subtree */
     std::vector<int> sub_cand_off;    /* [P + 1] first subtree of each candidate */

@@ -119,7 +119,7 @@ __device__ __forceinline__ void rs_count_keys(const u64 *src, long long r0, long
    count NULL it counts nothing). */
 static_assert(RK_T == RS_T, "the digit count runs on the key kernel's blocks");
 template <int MODE>
-__global__ void __launch_bounds__(RK_T) rk_keys(const FIns *fins, const int *fins_off,
+__global__ void __launch_bounds__(RK_T) rk_keys(const FOp *fins, const int *fins_off,
                                                 const int4 *finfo, const int *valid,
                                                 const double *c0, int kmax, const double *cols,
                                                 const double *y, int npad, int n, int ntrials,
@@ -130,7 +130,7 @@ __global__ void __launch_bounds__(RK_T) rk_keys(const FIns *fins, const int *fin
     __shared__ unsigned int cnt[RS_PASSES][256];
     using V4 = FiV<double, 2>::V4;
     extern __shared__ __align__(16) unsigned char sm[];
-    FIns *ins = reinterpret_cast<FIns *>(sm);
+    FOp *ins = reinterpret_cast<FOp *>(sm);
     double *cv = reinterpret_cast<double *>(sm + 8 * (size_t)((maxins + 1) & ~1));
     V4 *stk = reinterpret_cast<V4 *>(cv + FT_MAX_CONST);
     const int ls = blockIdx.x / tiles;
@@ -153,7 +153,8 @@ __global__ void __launch_bounds__(RK_T) rk_keys(const FIns *fins, const int *fin
     bool bad = !ok;
     for (int row = r0 + 2 * tid; row < r1; row += 2 * RK_T) {
         double pr[2] = {CUDART_NAN, CUDART_NAN};
-        if (ok) fi_forward<double, 2, false>(ins, cv, cols, npad, row, stk, nullptr, RK_T, tid, pr);
+        if (ok)
+            fi_forward<double, 2, false>(ins, cv, cols + row, npad, stk + tid, nullptr, RK_T, pr);
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
             const int rr = row + i;
@@ -728,7 +729,7 @@ __device__ __forceinline__ unsigned rb_hash(unsigned a, unsigned b)
 /* Keys of S sample rows per segment: S / 2 row pairs, pair p at rows 2q and
    2q + 1 with q drawn by a fixed hash from the p-th of S / 2 equal strata of
    the n / 2 pairs; the f64 sweep and the keys of rk_keys. */
-__global__ void __launch_bounds__(RK_T) rb_sample(const FIns *fins, const int *fins_off,
+__global__ void __launch_bounds__(RK_T) rb_sample(const FOp *fins, const int *fins_off,
                                                   const int4 *finfo, const int *valid,
                                                   const double *c0, int kmax, const double *cols,
                                                   int npad, int n, int ntrials, int seg0,
@@ -736,7 +737,7 @@ __global__ void __launch_bounds__(RK_T) rb_sample(const FIns *fins, const int *f
 {
     using V4 = FiV<double, 2>::V4;
     extern __shared__ __align__(16) unsigned char sm[];
-    FIns *ins = reinterpret_cast<FIns *>(sm);
+    FOp *ins = reinterpret_cast<FOp *>(sm);
     double *cv = reinterpret_cast<double *>(sm + 8 * (size_t)((maxins + 1) & ~1));
     V4 *stk = reinterpret_cast<V4 *>(cv + FT_MAX_CONST);
     const int ls = blockIdx.x / sblocks, blk = blockIdx.x % sblocks;
@@ -755,7 +756,8 @@ __global__ void __launch_bounds__(RK_T) rb_sample(const FIns *fins, const int *f
     const int stride = (n / 2) / hp;
     const int q = p * stride + (int)(rb_hash((unsigned)seg, (unsigned)p) % (unsigned)stride);
     double pr[2] = {CUDART_NAN, CUDART_NAN};
-    if (ok) fi_forward<double, 2, false>(ins, cv, cols, npad, 2 * q, stk, nullptr, RK_T, tid, pr);
+    if (ok)
+        fi_forward<double, 2, false>(ins, cv, cols + 2 * q, npad, stk + tid, nullptr, RK_T, pr);
 #pragma unroll
     for (int i = 0; i < 2; ++i)
         samp[(size_t)ls * RB_MAXS + 2 * p + i] = isfinite(pr[i]) ? rk_key(pr[i]) : ~0ULL;
@@ -1235,7 +1237,7 @@ __global__ void __launch_bounds__(OS_T) os_pick(const u64 *ka, const u64 *kb,
    intervals {delta : |r + b delta| <= t}, b = dr/dc from the reverse sweep,
    where a row with b = 0 only vetoes (|r| > t). A row that is not finite
    stops the thread and marks the segment. */
-__global__ void __launch_bounds__(MX_T) mx_scan(const FIns *fins, const int *fins_off,
+__global__ void __launch_bounds__(MX_T) mx_scan(const FOp *fins, const int *fins_off,
                                                 const int4 *finfo, const int *valid,
                                                 const int *pcount, const double *c0, int kmax,
                                                 const int *coords, const double *levels,
@@ -1254,7 +1256,7 @@ __global__ void __launch_bounds__(MX_T) mx_scan(const FIns *fins, const int *fin
     const int4 info = finfo[cand];
     const int nf = info.x, nr = info.y, slots = info.w & 0xffff, ntape = info.w >> 16;
     const int p = pcount[cand];
-    FIns *ins = reinterpret_cast<FIns *>(sm);
+    FOp *ins = reinterpret_cast<FOp *>(sm);
     double *cv = reinterpret_cast<double *>(sm + 8 * (size_t)((maxins + 1) & ~1));
     V4 *stk = reinterpret_cast<V4 *>(cv + FT_MAX_CONST);
     V4 *tape = stk + (size_t)slots * MX_T;
@@ -1274,8 +1276,10 @@ __global__ void __launch_bounds__(MX_T) mx_scan(const FIns *fins, const int *fin
     int mybad = ok ? 0 : 1;
     for (int row = tid; ok && row < n; row += MX_T) {
         double pr;
-        if (want) fi_forward<double, 1, true>(ins, cv, cols, npad, row, stk, tape, MX_T, tid, &pr);
-        else fi_forward<double, 1, false>(ins, cv, cols, npad, row, stk, nullptr, MX_T, tid, &pr);
+        if (want)
+            fi_forward<double, 1, true>(ins, cv, cols + row, npad, stk + tid, tape + tid, MX_T, &pr);
+        else
+            fi_forward<double, 1, false>(ins, cv, cols + row, npad, stk + tid, nullptr, MX_T, &pr);
         const double r = pr - y[row];
         if (!isfinite(pr) || fabs(pr) > 1e30 || !isfinite(r)) {
             mybad |= 1;
@@ -1289,7 +1293,7 @@ __global__ void __launch_bounds__(MX_T) mx_scan(const FIns *fins, const int *fin
         if (want && (mybad & 2) == 0) {
             for (int j = 0; j < p; ++j) g[(size_t)j * MX_T + tid] = 0.0;
             double seed = 1.0;
-            fi_reverse<double, 1>(ins + nf, nr, stk, tape, MX_T, tid, g + tid, MX_T, MX_T, &seed);
+            fi_reverse<double, 1>(ins + nf, stk + tid, tape + tid, MX_T, g + tid, MX_T, MX_T, &seed);
             const double b = g[(size_t)coord * MX_T + tid];
             if (!isfinite(b)) {
                 mybad |= 1;
@@ -1423,7 +1427,7 @@ void stat_inputs(RcCtx *c, const unsigned int *prog, const unsigned int *off, co
                  int nsets, int nsegs, int kmax, const double *c0, size_t *cur, StatPrep &sp)
 {
     prep_batch(off, prog, pcount, nsets, c->v, sp.b);
-    sp.o_fins = rc_take(cur, sizeof(FIns) * sp.b.fins.size());
+    sp.o_fins = rc_take(cur, sizeof(FOp) * sp.b.fins.size());
     sp.o_finsoff = rc_take(cur, sizeof(int) * (nsets + 1));
     sp.o_finfo = rc_take(cur, sizeof(int4) * nsets);
     sp.o_valid = rc_take(cur, sizeof(int) * nsets);
@@ -1436,7 +1440,7 @@ void stat_copy(RcCtx *c, const int *pcount, int nsets, int nsegs, int kmax, cons
                const StatPrep &sp)
 {
     unsigned char *h = c->host;
-    memcpy(h + sp.o_fins, sp.b.fins.data(), sizeof(FIns) * sp.b.fins.size());
+    memcpy(h + sp.o_fins, sp.b.fins.data(), sizeof(FOp) * sp.b.fins.size());
     memcpy(h + sp.o_finsoff, sp.b.fins_off.data(), sizeof(int) * (nsets + 1));
     memcpy(h + sp.o_finfo, sp.b.finfo.data(), sizeof(int4) * nsets);
     memcpy(h + sp.o_valid, sp.b.valid.data(), sizeof(int) * nsets);
@@ -1577,7 +1581,7 @@ float rc_rank_score_batch(void *ctx, const unsigned int *prog, const unsigned in
         return -1.0f;
     const int ktiles = (n + RK_TILE - 1) / RK_TILE;
     const int ntiles = (n + RS_TILE - 1) / RS_TILE;
-    const FIns *d_fins = reinterpret_cast<const FIns *>(dev + sp.o_fins);
+    const FOp *d_fins = reinterpret_cast<const FOp *>(dev + sp.o_fins);
     const int *d_finsoff = reinterpret_cast<const int *>(dev + sp.o_finsoff);
     const int4 *d_finfo = reinterpret_cast<const int4 *>(dev + sp.o_finfo);
     const int *d_valid = reinterpret_cast<const int *>(dev + sp.o_valid);
@@ -1736,7 +1740,7 @@ float rc_order_stat_score_batch(void *ctx, const unsigned int *prog, const unsig
         const RsBuffers b = rs_carve(dev, &wc, ns, n, false, &part);
         cudaMemsetAsync(b.count, 0, sizeof(unsigned int) * RS_PASSES * 256 * (size_t)ns, c->s);
         rk_keys<RK_ABS><<<(unsigned)ns * ktiles, RK_T, smem, c->s>>>(
-            reinterpret_cast<const FIns *>(dev + sp.o_fins),
+            reinterpret_cast<const FOp *>(dev + sp.o_fins),
             reinterpret_cast<const int *>(dev + sp.o_finsoff),
             reinterpret_cast<const int4 *>(dev + sp.o_finfo),
             reinterpret_cast<const int *>(dev + sp.o_valid),
@@ -1798,7 +1802,7 @@ float rc_max_scan_batch(void *ctx, const unsigned int *prog, const unsigned int 
     cudaEventRecord(c->t0, c->s);
     c->launches += 1;
     mx_scan<<<nsegs, MX_T, smem, c->s>>>(
-        reinterpret_cast<const FIns *>(dev + sp.o_fins),
+        reinterpret_cast<const FOp *>(dev + sp.o_fins),
         reinterpret_cast<const int *>(dev + sp.o_finsoff),
         reinterpret_cast<const int4 *>(dev + sp.o_finfo),
         reinterpret_cast<const int *>(dev + sp.o_valid), reinterpret_cast<const int *>(dev + sp.o_p),
