@@ -1985,7 +1985,11 @@ __global__ void __launch_bounds__(T) ft_implicit_score_x(
         for (int i = tid; i < nf + nr; i += T) ins[i] = fins[ib + i];
         if (tid < kmax) cf[tid] = (float)c[(size_t)cand * kmax + tid];
         __syncthreads();
-        for (int row = r0 + NR * tid; row < r1; row += NR * T) {
+        /* every lane takes every step (the vote below needs the whole warp); a
+           step's rows stay below n rounded up to NR * T, which the columns
+           hold, and rows past r1 count for nothing */
+        for (int base = r0; base < r1; base += NR * T) {
+            const int row = base + NR * tid;
             float pr[NR];
             fi_forward<float, NR, true>(ins, cf, cols + row, npad, stk + tid, tape + tid, T, pr);
             for (int k = 0; k < v; ++k) {
@@ -2035,7 +2039,7 @@ __global__ void __launch_bounds__(T) ft_implicit_score_x(
                 wsum += wr;
             }
             /* an infeasible candidate's sums are not read: stop its rows */
-            if (__any_sync(0xffffffffu, isbad) || *((volatile int *)(bad + cand))) {
+            if (__any_sync(0xffffffffu, isbad || *((volatile int *)(bad + cand)))) {
                 isbad = 1;
                 break;
             }

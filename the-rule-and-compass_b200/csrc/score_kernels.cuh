@@ -632,6 +632,8 @@ __global__ void __launch_bounds__(T) rc_score_kernel(ScoreArgs a)
             for (int q = tid; q < e - b; q += T) sprog[c * a.maxins + q] = a.ins[b + q];
             if (skip_bad && *((volatile int *)(a.bad + cand))) skipmask |= 1u << c;
         }
+        /* one answer per warp: the votes below need all of its lanes */
+        skipmask = __reduce_or_sync(0xffffffffu, skipmask);
         for (int q = tid; q < gcount * NW * 4; q += T) swarp[q] = 0.0;
         if (tid == 0) {
             s_bad = 0;
