@@ -57,6 +57,16 @@ int rc_raise_smem(const void *fn, size_t bytes)
     return 0;
 }
 
+void rc_fit_free_streams(RcCtx *c)
+{
+    for (int i = 0; i < 6; ++i) {
+        if (c->fit_ev[i]) cudaEventDestroy(c->fit_ev[i]);
+        if (c->fit_side[i]) cudaStreamDestroy(c->fit_side[i]);
+        c->fit_ev[i] = nullptr;
+        c->fit_side[i] = nullptr;
+    }
+}
+
 size_t rc_take(size_t *cur, size_t bytes)
 {
     size_t o = (*cur + 255) & ~(size_t)255;
@@ -276,6 +286,7 @@ void rc_destroy(void *ctx)
     free_ptr(c->dev);
     if (c->host) cudaFreeHost(c->host);
     if (c->fit_graph) cudaGraphExecDestroy(c->fit_graph);
+    rc_fit_free_streams(c);
     if (c->t0) cudaEventDestroy(c->t0);
     if (c->t1) cudaEventDestroy(c->t1);
     if (c->ev_done) cudaEventDestroy(c->ev_done);

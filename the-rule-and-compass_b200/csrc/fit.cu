@@ -14,18 +14,21 @@
  * GPU waits for the slowest candidate. Here every sweep is spread over
  * (candidate x 2,048-row tile) work items for all active candidates at once:
  *
- *   step s:  sweep kernels, one per kind (f32 assembly, f64 assembly, f32
- *            objective, f64 objective; implicit Jacobian / cost), each a
- *            persistent grid over the (candidate, tile) items whose candidate
- *            requested that kind -> per-tile partials (packed J^T J / J^T r
- *            blocks, objective, flags);
+ *   step s:  sweep kernels (f64 and f32 assembly; f64 and f32 objective;
+ *            implicit Jacobian / cost), each a persistent grid over the
+ *            (candidate, tile) items whose candidate requested one of its
+ *            kinds -> per-tile partials (packed J^T J / J^T r blocks,
+ *            objective, flags);
  *            control kernel: per candidate that had a sweep, reduce its tile
  *            partials in ascending tile order, run the reference's LM state
  *            machine (damped Jacobi-equilibrated Cholesky in f64, trial
  *            clamp, accept / reject, lambda, IRLS rounds, polish) until it
  *            needs the next sweep, and queue it for step s+1.
  *
- * The number of steps any candidate can need is bounded (two sweeps per LM
+ * The candidates of a large batch are split into chains by the shape of their
+ * assemblies; each chain runs its own steps on its own stream (chains below),
+ * so one chain's sweeps fill the GPU while another's last tiles and its
+ * controller run. The number of steps any candidate can need is bounded (two sweeps per LM
  * iteration, four with L1 halvings, plus the polish), so the whole fit is a
  * fixed graph of kernels replayed per batch; candidates that finish early
  * simply stop queueing work. Every statistic is a fixed-order sum (per row
@@ -56,24 +59,19 @@
 
 enum {
     FOP_NONE = 0, FOP_ASM32 = 1, FOP_ASM64 = 2, FOP_LOSS32 = 3, FOP_LOSS64 = 4,
-    FOP_IJAC = 5, FOP_ICOST = 6, FOP_CASM = 7, FOP_CSCORE = 8, FOP_IJACS = 9,
-    /* the assembly queues of the other launch classes (ft_cls_*): their
-       sweeps run in blocks of the class's threads, sized for the class */
-    FOP_ASM32_64 = 10, FOP_ASM32_32 = 11, FOP_ASM64_64 = 12, FOP_ASM64_32 = 13,
-    FOP_ASM32_64A = 14, FOP_ASM32_64B = 15, FOP_ASM64_64A = 16, FOP_ASM64_64B = 17,
-    FOP_ASM32_128L = 18, FOP_ASM64_128L = 19,
-    FOP_COUNT = 20
+    FOP_IJAC = 5, FOP_ICOST = 6, FOP_CASM = 7, FOP_CSCORE = 8,
+    FOP_COUNT = 9
 };
 
-/* Launch classes of the assemblies. A candidate's active threads A and its
-   shared region decide it: 0: A = 128 with a region of at most 41 KB; 5:
-   A = 128 with a larger one (a length bucket the autotuner gave a bigger
-   budget); 1, 2, 3: A = 64 with a region of at most 21 KB, at most 30 KB, or
-   more; 4: A = 32. A class's launch uses blocks of A threads and the largest
-   region of its candidates, so the small-region classes fit more blocks on
-   an SM (10, 7 and 5 of 64 threads at 21, 30 and 40 KB), and a large region
-   never shrinks the launch of the others. Which launch runs a candidate does
-   not change its arithmetic (that depends on A alone). */
+/* Assembly classes. A candidate's active threads A and its shared region
+   decide it: 0: A = 128 with a region of at most 41 KB; 5: A = 128 with a
+   larger one (a length bucket the autotuner gave a bigger budget); 1, 2, 3:
+   A = 64 with a region of at most 21 KB, at most 30 KB, or more; 4: A = 32.
+   A class's launch uses blocks of A threads and the largest region of its
+   candidates, so the small-region classes fit more blocks on an SM (9, 7 and
+   5 of 64 threads at 21, 30 and 40 KB), and a large region never shrinks the
+   launch of the others. Which launch runs a candidate does not change its
+   arithmetic (that depends on A alone). */
 #define FT_NCLS 6
 __host__ __device__ constexpr int ft_cls_threads(int cls)
 {
@@ -87,41 +85,8 @@ inline int ft_cls_of(int A, size_t region)
     return region <= 21 * 1024 ? 1 : (region <= 30 * 1024 ? 2 : 3);
 }
 
-/* The kind a queue's sweep performs (a class queue performs its base kind). */
-__host__ __device__ constexpr int ft_base_kind(int k)
-{
-    return (k == FOP_ASM32_64 || k == FOP_ASM32_32 || k == FOP_ASM32_64A || k == FOP_ASM32_64B ||
-            k == FOP_ASM32_128L)
-               ? FOP_ASM32
-           : (k == FOP_ASM64_64 || k == FOP_ASM64_32 || k == FOP_ASM64_64A ||
-              k == FOP_ASM64_64B || k == FOP_ASM64_128L)
-               ? FOP_ASM64
-               : k;
-}
-
-/* The launch class of an assembly queue kind (0 for the base kinds). */
-__host__ __device__ constexpr int ft_kind_cls(int k)
-{
-    return (k == FOP_ASM32_64A || k == FOP_ASM64_64A)   ? 1
-           : (k == FOP_ASM32_64B || k == FOP_ASM64_64B) ? 2
-           : (k == FOP_ASM32_64 || k == FOP_ASM64_64)   ? 3
-           : (k == FOP_ASM32_32 || k == FOP_ASM64_32)   ? 4
-           : (k == FOP_ASM32_128L || k == FOP_ASM64_128L) ? 5
-                                                        : 0;
-}
-
-/* The queue of a sweep request: f32 / f64 assemblies go to the queue of the
-   candidate's launch class. */
-__host__ __device__ inline int ft_queue_kind(int op, int cls)
-{
-    static constexpr int k32[FT_NCLS] = {FOP_ASM32, FOP_ASM32_64A, FOP_ASM32_64B, FOP_ASM32_64,
-                                         FOP_ASM32_32, FOP_ASM32_128L};
-    static constexpr int k64[FT_NCLS] = {FOP_ASM64, FOP_ASM64_64A, FOP_ASM64_64B, FOP_ASM64_64,
-                                         FOP_ASM64_32, FOP_ASM64_128L};
-    if (op == FOP_ASM32) return k32[cls];
-    if (op == FOP_ASM64) return k64[cls];
-    return op;
-}
+/* Chains a fit is split into at most (one per class). */
+#define FT_MAX_CHAINS FT_NCLS
 
 enum {
     PC_INIT = 0, PC_AFTER_FIRST_ASM, PC_ROUND, PC_ITER, PC_AFTER_ASM, PC_SOLVE,
@@ -213,14 +178,13 @@ struct FitArgs {
     const int *valid;
     const FOp *fins;       /* stack-machine translation of the records */
     const int *fins_off;   /* [P+1] start of [forward | reverse] */
-    const int4 *finfo;     /* [P] forward count, reverse count, active threads | launch
-                              class << 16,
+    const int4 *finfo;     /* [P] forward count, reverse count, active threads | assembly
+                              class << 16 | chain << 24,
                               spill slots | tape slots << 16 */
-    int fslots;            /* spill slots needed by the batch */
+    int fslots;            /* spill slots needed by the chain */
     int ftape;             /* partial-tape slots needed by the batch */
     int fmaxins;           /* longest forward + reverse list */
-    size_t asm_region;     /* assembly region of a 128-thread launch over every class */
-    size_t asm_reg[6];     /* assembly region of each launch class (ft_cls_of) */
+    size_t asm_region;     /* assembly region of the chain */
     const int2 *fcinfo;    /* [P] cached forward count (after the reverse list),
                               first cache column */
     float *cache;          /* [columns][npad] values of constant-free subtrees */
@@ -237,17 +201,14 @@ struct FitArgs {
     int iters, metric, flags;
     int ntiles;
     int mmax;
-    int ijac_small;        /* implicit: programs of at most this many records take the
-                              short Jacobian launch (FOP_IJACS); 0: one launch */
     int ijac_tape;         /* internal-node tape slots of the Jacobian launch */
-    int ijac_tape_small;   /* ... and of the short one */
     int Wmax;
     int nprog;
     FitState *state;
     double *part;      /* [P][ntiles][FT_PART_STRIDE] */
-    int *lists;        /* [2][FOP_COUNT][P] */
-    int *counts;       /* [2][FOP_COUNT] candidates queued per kind */
-    int *work;         /* [2][FOP_COUNT] persistent-grid work counters */
+    int *lists;        /* the chain's [2][FOP_COUNT][P] */
+    int *counts;       /* the chain's [2][FOP_COUNT] candidates queued per kind */
+    int *work;         /* the chain's [2][FOP_COUNT] persistent-grid work counters */
     double *outc;
     double *outsse;
     int *outstatus;
@@ -255,14 +216,21 @@ struct FitArgs {
 
 /* ---- sweep kernels ------------------------------------------------------ */
 
-__host__ __device__ inline bool ft_op_assembles(int opk)
+__host__ __device__ constexpr bool ft_op_assembles(int opk)
 {
-    opk = ft_base_kind(opk);
-    return opk == FOP_ASM32 || opk == FOP_ASM64 || opk == FOP_IJAC || opk == FOP_CASM ||
-           opk == FOP_IJACS;
+    return opk == FOP_ASM32 || opk == FOP_ASM64 || opk == FOP_IJAC || opk == FOP_CASM;
 }
 
-__host__ __device__ inline bool ft_op_ijac(int opk) { return opk == FOP_IJAC || opk == FOP_IJACS; }
+/* Ready the queue and work counters of the other parity for the controller
+   that follows this sweep (its sweep and controller are done); every sweep
+   kernel's first block does it. */
+__device__ __forceinline__ void ft_clear_other(const FitArgs &a, int q)
+{
+    if (blockIdx.x == 0 && threadIdx.x < FOP_COUNT) {
+        a.counts[(q ^ 1) * FOP_COUNT + threadIdx.x] = 0;
+        a.work[(q ^ 1) * FOP_COUNT + threadIdx.x] = 0;
+    }
+}
 
 /* Columns of a sweep's augmented Gram: the Jacobian and the residual, or for
    the correlation assembly the Jacobian and the weighted 1, f and y
@@ -453,6 +421,7 @@ __global__ void __launch_bounds__(T) ft_sweep(FitArgs a, int q)
         double *red = reinterpret_cast<double *>(ig + (size_t)a.v * T);
         __shared__ int s_item;
         const int tid = threadIdx.x;
+        ft_clear_other(a, q);
         const int *list = a.lists + ((size_t)q * FOP_COUNT + OPK) * a.nprog;
         const int total = a.counts[q * FOP_COUNT + OPK] * a.ntiles;
         int *work = a.work + q * FOP_COUNT + OPK;
@@ -481,16 +450,17 @@ __global__ void __launch_bounds__(T) ft_sweep(FitArgs a, int q)
     }
 }
 
-/* The exact-Jacobian sweep (FOP_IJAC, or FOP_IJACS for the short programs)
-   over every queued (candidate, tile) item of step parity q: eight 64-thread
-   blocks per SM fit beside the compact tapes, so registers are held to
-   that. The short launch is laid out for its own record and tape bounds. */
-template <int OPK, int T>
+/* The exact-Jacobian sweep over every queued (candidate, tile) item of step
+   parity q: eight 64-thread blocks per SM fit beside the compact tapes, so
+   registers are held to that. A chain's launch is laid out for its own record
+   and tape bounds. */
+template <int T>
 __global__ void __launch_bounds__(T, 8) ft_jac_sweep(FitArgs a, int q)
 {
     extern __shared__ __align__(16) unsigned char sm[];
-    const int mcap = OPK == FOP_IJACS ? a.ijac_small : a.mmax;
-    const int tcap = OPK == FOP_IJACS ? a.ijac_tape_small : a.ijac_tape;
+    constexpr int OPK = FOP_IJAC;
+    const int mcap = a.mmax;
+    const int tcap = a.ijac_tape;
     uint4 *rec = reinterpret_cast<uint4 *>(sm);
     unsigned *refs = reinterpret_cast<unsigned *>(sm + 16 * (size_t)mcap);
     double *cd = reinterpret_cast<double *>(sm + 16 * (size_t)mcap + 16 * (size_t)((mcap + 3) / 4));
@@ -500,6 +470,7 @@ __global__ void __launch_bounds__(T, 8) ft_jac_sweep(FitArgs a, int q)
     double *red = rows + ft_rows_bytes(a.Wmax, T) / 8;
     __shared__ int s_item, s_ni;
     const int tid = threadIdx.x;
+    ft_clear_other(a, q);
     const int *list = a.lists + ((size_t)q * FOP_COUNT + OPK) * a.nprog;
     const int total = a.counts[q * FOP_COUNT + OPK] * a.ntiles;
     int *work = a.work + q * FOP_COUNT + OPK;
@@ -571,11 +542,6 @@ inline int ft_asm_threads(int slots, int tape, int ncols, size_t budget)
 
 /* Length bucket of a fit program of m records (the autotuner's key). */
 inline int ft_length_bucket(int m) { return m <= 16 ? 0 : (m <= 32 ? 1 : (m <= 64 ? 2 : 3)); }
-
-__host__ __device__ inline bool ft_op_f64(int opk)
-{
-    return ft_base_kind(opk) == FOP_ASM64 || opk == FOP_LOSS64;
-}
 
 /* Shared memory of a four-row sweep: forward and reverse instructions,
    constants, the assembly region (or the spill slots of an objective sweep),
@@ -945,79 +911,112 @@ __device__ void ft_tile_corr_score(const FitArgs &a, const FOp *ins, const float
     if (tid == 0) pt[FT_PART_BAD] = bad ? 1.0 : 0.0;
 }
 
-/* The assembly / objective sweeps (f32 and f64) over the four-row
-   interpreter: a persistent grid over the queued (candidate, tile) items. */
+/* One (candidate, tile) item of a sweep of kind OPK in a block of T threads. */
 template <int OPK, int T>
-__global__ void __launch_bounds__(T) ft_sweep4(FitArgs a, int q)
+__device__ void ft_sweep_item(const FitArgs &a, unsigned char *sm, int cand, int tile)
 {
-    constexpr int BK = ft_base_kind(OPK);
-    using V = typename std::conditional<BK == FOP_ASM64 || BK == FOP_LOSS64, double, float>::type;
-    constexpr int NR = (BK == FOP_ASM32 || BK == FOP_CASM) ? FT_ASM32_NR
-                       : BK == FOP_ASM64                     ? FT_ASM64_NR
-                       : (BK == FOP_LOSS32 || BK == FOP_CSCORE) ? FT_LOSS32_NR
-                                                                : FT_LOSS64_NR;
+    using V = typename std::conditional<OPK == FOP_ASM64 || OPK == FOP_LOSS64, double, float>::type;
+    constexpr int NR = (OPK == FOP_ASM32 || OPK == FOP_CASM) ? FT_ASM32_NR
+                       : OPK == FOP_ASM64                     ? FT_ASM64_NR
+                       : (OPK == FOP_LOSS32 || OPK == FOP_CSCORE) ? FT_LOSS32_NR
+                                                                  : FT_LOSS64_NR;
     using V4 = typename FiV<V, NR>::V4;
-    extern __shared__ __align__(16) unsigned char sm[];
     FOp *ins = reinterpret_cast<FOp *>(sm);
     V *cv = reinterpret_cast<V *>(sm + 8 * (size_t)((a.fmaxins + 1) & ~1));
-    unsigned char *region = reinterpret_cast<unsigned char *>(sm + 8 * (size_t)((a.fmaxins + 1) & ~1) +
-                                                              8 * FT_MAX_CONST);
-    /* a class queue's region is sized for its class; the 128-thread launch
-       of a base assembly kind for every candidate it may hold */
-    const size_t asm_reg = OPK != BK ? a.asm_reg[ft_kind_cls(OPK)]
-                           : (BK == FOP_CASM ? a.asm_region : a.asm_reg[0]);
+    unsigned char *region = sm + 8 * (size_t)((a.fmaxins + 1) & ~1) + 8 * FT_MAX_CONST;
     double *red = reinterpret_cast<double *>(
-        region + (ft_op_assembles(OPK) ? asm_reg
+        region + (ft_op_assembles(OPK) ? a.asm_region
                                        : 16 * (size_t)(a.fslots > 0 ? a.fslots : 1) * T));
+    const int tid = threadIdx.x;
+    const FitState *st = a.state + cand;
+    const int ib = a.fins_off[cand];
+    const int4 info = a.finfo[cand];
+    const int nr = info.y;
+    /* f32 sweeps run the cached forward list (constant-free subtrees read
+       from the cache), the f64 polish the full one */
+    const bool CACHED = sizeof(V) == 4 || a.cache64 != nullptr;
+    const int2 fc = CACHED ? a.fcinfo[cand] : make_int2(info.x, 0);
+    const int nf = fc.x;
+    const FOp *fsrc = a.fins + ib + (CACHED ? info.x + nr : 0);
+    const V *ccols = !CACHED ? nullptr
+                             : (sizeof(V) == 4 ? reinterpret_cast<const V *>(a.cache)
+                                               : reinterpret_cast<const V *>(a.cache64)) +
+                                   (size_t)fc.y * a.npad;
+    const int p = a.pcount[cand];
+    const int sel = st->sel;
+    for (int i = tid; i < nf; i += T) ins[i] = fsrc[i];
+    if (ft_op_assembles(OPK))
+        for (int i = tid; i < nr; i += T) ins[nf + i] = a.fins[ib + info.x + i];
+    if (tid < p) cv[tid] = (V)(sel ? st->trial[tid] : st->c[tid]);
+    __syncthreads();
+    const int r0 = tile * FT_TILE_ROWS;
+    const int r1 = min(a.n, r0 + FT_TILE_ROWS);
+    double *pt = a.part + ((size_t)cand * a.ntiles + tile) * FT_PART_STRIDE;
+    if constexpr (ft_op_assembles(OPK))
+        ft_tile_asm<V, NR, T, OPK == FOP_CASM>(a, ins, ins + nf, p, info.z & 0xffff, info.w & 0xffff,
+                                               info.w >> 16, cv, region, red, r0, r1, pt, ccols);
+    else if constexpr (OPK == FOP_CSCORE)
+        ft_tile_corr_score<NR, T>(a, ins, cv, reinterpret_cast<V4 *>(region), red, r0, r1, pt, ccols);
+    else
+        ft_tile_loss<V, NR, T>(a, ins, cv, reinterpret_cast<V4 *>(region), red, r0, r1, pt, ccols);
+}
+
+/* The sweeps of kinds K0, K1, ... of step parity q in one launch: a
+   persistent grid over their queued (candidate, tile) items, the kinds in
+   the order named (the longest items first), so that one kind's last tiles
+   run beside the next kind's. Registers are held to 640 threads an SM for the
+   assemblies, what their shared memory allows (5 blocks of 128 threads at
+   40 KB), and to 1,024 for the objective sweeps. */
+template <int T, int K0, int... KS>
+__global__ void __launch_bounds__(T, ft_op_assembles(K0) ? 640 / T : 1024 / T)
+    ft_sweep4(FitArgs a, int q)
+{
+    extern __shared__ __align__(16) unsigned char sm[];
+    constexpr int kinds[] = {K0, KS...};
+    constexpr int NK = 1 + sizeof...(KS);
     __shared__ int s_item;
     const int tid = threadIdx.x;
-    const int *list = a.lists + ((size_t)q * FOP_COUNT + OPK) * a.nprog;
-    const int total = a.counts[q * FOP_COUNT + OPK] * a.ntiles;
-    int *work = a.work + q * FOP_COUNT + OPK;
+    ft_clear_other(a, q);
+    int counts[NK], total = 0;
+#pragma unroll
+    for (int k = 0; k < NK; ++k) {
+        counts[k] = a.counts[q * FOP_COUNT + kinds[k]];
+        total += counts[k];
+    }
+    total *= a.ntiles;
+    int *work = a.work + q * FOP_COUNT + K0;
     for (;;) {
         if (tid == 0) s_item = atomicAdd(work, 1);
         __syncthreads();
         const int item = s_item;
         __syncthreads();
         if (item >= total) break;
-        const int cand = list[item / a.ntiles];
-        const int tile = item % a.ntiles;
-        const FitState *st = a.state + cand;
-        const int ib = a.fins_off[cand];
-        const int4 info = a.finfo[cand];
-        const int nr = info.y;
-        /* f32 sweeps run the cached forward list (constant-free subtrees read
-           from the cache), the f64 polish the full one */
-        const bool CACHED = sizeof(V) == 4 || a.cache64 != nullptr;
-        const int2 fc = CACHED ? a.fcinfo[cand] : make_int2(info.x, 0);
-        const int nf = fc.x;
-        const FOp *fsrc = a.fins + ib + (CACHED ? info.x + nr : 0);
-        const V *ccols =
-            !CACHED ? nullptr
-                    : (sizeof(V) == 4 ? reinterpret_cast<const V *>(a.cache)
-                                      : reinterpret_cast<const V *>(a.cache64)) +
-                          (size_t)fc.y * a.npad;
-        const int p = a.pcount[cand];
-        const int sel = st->sel;
-        for (int i = tid; i < nf; i += T) ins[i] = fsrc[i];
-        if (ft_op_assembles(OPK))
-            for (int i = tid; i < nr; i += T) ins[nf + i] = a.fins[ib + info.x + i];
-        if (tid < p) cv[tid] = (V)(sel ? st->trial[tid] : st->c[tid]);
-        __syncthreads();
-        const int r0 = tile * FT_TILE_ROWS;
-        const int r1 = min(a.n, r0 + FT_TILE_ROWS);
-        double *pt = a.part + ((size_t)cand * a.ntiles + tile) * FT_PART_STRIDE;
-        if (ft_op_assembles(OPK))
-            ft_tile_asm<V, NR, T, BK == FOP_CASM>(a, ins, ins + nf, p, info.z & 0xffff,
-                                                  info.w & 0xffff,
-                                                  info.w >> 16, cv, region, red, r0, r1, pt, ccols);
-        else if (BK == FOP_CSCORE)
-            ft_tile_corr_score<NR, T>(a, ins, reinterpret_cast<const float *>(cv),
-                                      reinterpret_cast<typename FiV<float, NR>::V4 *>(region), red,
-                                      r0, r1, pt, reinterpret_cast<const float *>(ccols));
-        else
-            ft_tile_loss<V, NR, T>(a, ins, cv, reinterpret_cast<V4 *>(region), red, r0, r1, pt,
-                                   ccols);
+        int c = item / a.ntiles;
+        const int tile = item - c * a.ntiles;
+        int kind = K0;
+        const int *lists = a.lists + (size_t)q * FOP_COUNT * a.nprog;
+        bool found = false;
+        int cand = 0;
+#pragma unroll
+        for (int k = 0; k < NK; ++k) {
+            if (found) continue;
+            if (c < counts[k]) {
+                kind = kinds[k];
+                cand = lists[(size_t)kind * a.nprog + c];
+                found = true;
+            } else {
+                c -= counts[k];
+            }
+        }
+        if constexpr (NK == 1) {
+            ft_sweep_item<K0, T>(a, sm, cand, tile);
+        } else {
+            auto run = [&](auto K) {
+                if (kind == decltype(K)::value) ft_sweep_item<decltype(K)::value, T>(a, sm, cand, tile);
+            };
+            run(std::integral_constant<int, K0>{});
+            (run(std::integral_constant<int, KS>{}), ...);
+        }
         __syncthreads();
     }
 }
@@ -1601,10 +1600,7 @@ __device__ void ft_advance(const FitArgs &a, FitState &st, int cand, int p, doub
                    unchanged point after a rejected or singular step; the
                    system kept from the last assembly is the same one */
                 if (!st.assembled) {
-                    st.op = (a.ijac_small > 0 &&
-                             a.node_off[cand + 1] - a.node_off[cand] <= a.ijac_small)
-                                ? FOP_IJACS
-                                : FOP_IJAC;
+                    st.op = FOP_IJAC;
                     st.sel = 0;
                     st.pc = PC_I_AFTER_JAC;
                     return;
@@ -1699,7 +1695,7 @@ __global__ void __launch_bounds__(FT_CTRL_T) ft_control(FitArgs a, int q, int in
                         base += a.counts[q * FOP_COUNT + k];
                         ++k;
                     }
-                    op = ft_base_kind(k);
+                    op = k;
                     cand = a.lists[((size_t)q * FOP_COUNT + k) * a.nprog + (t - base)];
                 }
                 s_cand = cand;
@@ -1819,7 +1815,7 @@ __global__ void __launch_bounds__(FT_CTRL_T) ft_control(FitArgs a, int q, int in
             const int op = sst.op;
             const int k = (op == FOP_ASM32 || op == FOP_CASM)      ? 0
                           : (op == FOP_LOSS32 || op == FOP_CSCORE) ? 1
-                          : (op == FOP_ASM64 || ft_op_ijac(op))     ? 2
+                          : (op == FOP_ASM64 || op == FOP_IJAC)    ? 2
                                                                     : 3;
             sst.nsw[k]++;
         }
@@ -1830,21 +1826,15 @@ __global__ void __launch_bounds__(FT_CTRL_T) ft_control(FitArgs a, int q, int in
             for (int i = tid; i < (int)(sizeof(FitState) / 8); i += FT_CTRL_T) dst[i] = src[i];
         }
         if (tid == 0 && sst.op != FOP_NONE) {
-            const int kq = ft_queue_kind(sst.op, a.finfo[cand].z >> 16);
-            const int k = atomicAdd(&a.counts[nq * FOP_COUNT + kq], 1);
-            a.lists[((size_t)nq * FOP_COUNT + kq) * a.nprog + k] = cand;
+            /* the start of a fit serves every chain: its arguments are the
+               first chain's */
+            const size_t ch = init ? (size_t)((unsigned)a.finfo[cand].z >> 24) : 0;
+            int *counts = a.counts + ch * 2 * FOP_COUNT;
+            int *lists = a.lists + ch * 2 * FOP_COUNT * (size_t)a.nprog;
+            const int k = atomicAdd(&counts[nq * FOP_COUNT + sst.op], 1);
+            lists[((size_t)nq * FOP_COUNT + sst.op) * a.nprog + k] = cand;
         }
         __syncthreads();
-    }
-}
-
-/* Clear the queue that step s fills and the work counters it consumes. */
-__global__ void ft_step_reset(FitArgs a, int q)
-{
-    const int t = threadIdx.x;
-    if (t < FOP_COUNT) {
-        a.counts[(q ^ 1) * FOP_COUNT + t] = 0;
-        a.work[q * FOP_COUNT + t] = 0;
     }
 }
 
@@ -2154,11 +2144,7 @@ void prep_batch(const unsigned int *off, const unsigned int *prog, const int *pc
     b.fins.clear();
     b.fins_off.assign(nprog + 1, 0);
     b.finfo.assign(nprog, make_int4(0, 0, 32, 0));
-    b.asm_region = 256;
-    for (int k = 0; k < FT_NCLS; ++k) {
-        b.asm_reg[k] = 256;
-        b.nclass[k] = 0;
-    }
+    b.pcount.assign(pcount, pcount + nprog);
     const bool caching = cache_bytes_per_col > 0;
     b.fcinfo.assign(nprog, make_int2(0, 0));
     b.sub_fins.clear();
@@ -2234,9 +2220,6 @@ void prep_batch(const unsigned int *off, const unsigned int *prog, const int *pc
         /* z: active threads, launch class above bit 16 */
         b.finfo[i] = make_int4((int)(base_r - base_f), (int)(base_c - base_r), A | (cls << 16),
                                ns | (nt << 16));
-        b.asm_region = std::max(b.asm_region, reg);
-        b.asm_reg[cls] = std::max(b.asm_reg[cls], reg);
-        b.nclass[cls]++;
         b.fslots = std::max(b.fslots, ns);
         b.ftape = std::max(b.ftape, nt);
         b.fmaxins = std::max(b.fmaxins, (int)(base_c - base_f));
@@ -2282,8 +2265,31 @@ struct SweepLaunch {
     size_t smem;
     int grid;
     int threads;
-    int opk; /* the queue kind it serves */
 };
+
+/* One chain of a fit: its arguments (own queues and launch shapes) and the
+   sweeps of one of its steps. */
+struct FitChain {
+    FitArgs a;
+    SweepLaunch sw[2];
+    int nk = 0;
+    int ncand = 0;
+};
+
+SweepLaunch sweep_shape(RcCtx *c, const void *fn, int threads, size_t smem, long long items)
+{
+    /* persistent grids take their items from work counters, so a grid no
+       larger than the items that can exist answers the same and launches no
+       idle blocks */
+    SweepLaunch s;
+    s.fn = fn;
+    s.smem = smem;
+    rc_raise_smem(fn, smem);
+    s.grid = (int)std::max<long long>(
+        1, std::min<long long>((long long)c->sm_count * occupancy(fn, threads, smem), items));
+    s.threads = threads;
+    return s;
+}
 
 /* Input-mode translation (fi_decode with `inputs`) of every valid candidate:
    [forward | reverse] per candidate, counts and slot sizes in info. A
@@ -2325,60 +2331,28 @@ void prep_inputs(const unsigned int *off, const unsigned int *prog, int nprog,
     if (x.fins.empty()) x.fins.resize(1);
 }
 
-/* The implicit cost sweep on the stack machine. */
-SweepLaunch icost_launch(RcCtx *c, const XPrep &x)
-{
-    SweepLaunch s;
-    s.fn = (const void *)ft_sweep<FOP_ICOST, FT_ITHREADS>;
-    s.opk = FOP_ICOST;
-    s.smem = 8 * (size_t)((x.maxins + 1) & ~1) + 8 * FT_MAX_CONST +
-             8 * (size_t)FT_ITHREADS * (x.slots + x.tape + c->v) + 8 * (size_t)FT_ITHREADS;
-    rc_raise_smem(s.fn, s.smem);
-    s.grid = c->sm_count * occupancy(s.fn, FT_ITHREADS, s.smem);
-    s.threads = FT_ITHREADS;
-    return s;
-}
-
-template <int OPK>
-SweepLaunch sweep_launch(RcCtx *c, int mrec, int tcap, int Wmax)
-{
-    SweepLaunch s;
-    s.fn = (const void *)ft_jac_sweep<OPK, FT_ITHREADS>;
-    s.opk = OPK;
-    s.smem = ft_ijac_smem(mrec, tcap, Wmax, FT_ITHREADS);
-    rc_raise_smem(s.fn, s.smem);
-    s.grid = c->sm_count * occupancy(s.fn, FT_ITHREADS, s.smem);
-    s.threads = FT_ITHREADS;
-    return s;
-}
-
-/* The tape bound of the Jacobian launch (the most internal nodes of the
-   batch) and the record and tape bounds of the short launch. The sweep
-   keeps two f64 tapes per row in shared memory, one slot per internal
-   node, sized for the largest program of the launch, so one launch sized
-   for the batch runs the short programs at the largest one's occupancy.
-   Each split (programs of at most t records to the short launch) is
+/* The record bound that splits an implicit batch into two chains. The
+   Jacobian sweep keeps two f64 tapes per row in shared memory, one slot per
+   internal node, sized for the largest program of the launch, so one launch
+   sized for the batch runs the short programs at the largest one's occupancy.
+   Each split (programs of at most t records to the short chain) is
    estimated as the internal nodes swept over the resident blocks each
-   launch allows; the best is kept if it saves at least 5 %, else `small`
-   is 0 and one launch serves all. The split depends on the batch, but a
-   candidate's arithmetic does not depend on which launch runs it. */
-struct IjacSplit {
-    int tape = 1, small = 0, tape_small = 1;
-};
-
-IjacSplit ijac_split(RcCtx *c, const FitPrep &b, int Wmax)
+   launch allows; the best is kept if it saves at least 5 %, else 0: one
+   chain. The split depends on the batch, but a candidate's arithmetic does
+   not depend on which launch runs it. */
+int ijac_split(RcCtx *c, const FitPrep &b, int Wmax)
 {
-    IjacSplit out;
+    int out = 0, tape = 1;
     std::vector<std::pair<int, int>> ms; /* (records, internal nodes) */
     for (size_t i = 0; i + 1 < b.node_off.size(); ++i)
         if (b.valid[i]) {
             ms.emplace_back(b.node_off[i + 1] - b.node_off[i], b.ninternal[i]);
-            out.tape = std::max(out.tape, b.ninternal[i]);
+            tape = std::max(tape, b.ninternal[i]);
         }
     if (ms.size() < 2) return out;
-    const void *fn = (const void *)ft_jac_sweep<FOP_IJACS, FT_ITHREADS>;
+    const void *fn = (const void *)ft_jac_sweep<FT_ITHREADS>;
     /* occupancy queries up to the largest layout the split can choose */
-    const size_t smax = ft_ijac_smem(b.mmax, out.tape, Wmax, FT_ITHREADS);
+    const size_t smax = ft_ijac_smem(b.mmax, tape, Wmax, FT_ITHREADS);
     if (rc_raise_smem(fn, smax) != 0) return out;
     std::sort(ms.begin(), ms.end());
     auto occ = [&](int mrec, int tcap) {
@@ -2386,7 +2360,7 @@ IjacSplit ijac_split(RcCtx *c, const FitPrep &b, int Wmax)
     };
     double total = 0.0;
     for (const auto &e : ms) total += e.second + 1;
-    const double big = occ(b.mmax, out.tape);
+    const double big = occ(b.mmax, tape);
     const double one = total / big;
     double best = one, below = 0.0;
     int tmax = 1;
@@ -2398,44 +2372,125 @@ IjacSplit ijac_split(RcCtx *c, const FitPrep &b, int Wmax)
         const double cost = below / occ(ms[i].first, tmax) + (total - below) / big;
         if (cost < best) {
             best = cost;
-            out.small = ms[i].first;
-            out.tape_small = tmax;
+            out = ms[i].first;
         }
     }
-    if (!(best <= 0.95 * one)) {
-        out.small = 0;
-        out.tape_small = 1;
+    return best <= 0.95 * one ? out : 0;
+}
+
+/* The assembly and objective launches of a class, one per block width. */
+template <int K64, int K32>
+const void *asm_kernel(int threads)
+{
+    return threads == 128  ? (const void *)ft_sweep4<128, K64, K32>
+           : threads == 64 ? (const void *)ft_sweep4<64, K64, K32>
+                           : (const void *)ft_sweep4<32, K64, K32>;
+}
+
+const void *casm_kernel(int threads)
+{
+    return threads == 128  ? (const void *)ft_sweep4<128, FOP_CASM>
+           : threads == 64 ? (const void *)ft_sweep4<64, FOP_CASM>
+                           : (const void *)ft_sweep4<32, FOP_CASM>;
+}
+
+/* The chain of the candidates `ids` (indexes into the batch; `cls` their
+   assembly class): the batch's arguments `a` with the chain's launch shapes.
+   `small`: every kind of a step in one launch of 128-thread blocks. */
+FitChain make_chain(RcCtx *c, const FitArgs &a, const FitPrep &b, const XPrep &xp,
+                    const std::vector<int> &ids, int cls, bool small)
+{
+    FitChain ch;
+    ch.a = a;
+    ch.ncand = (int)ids.size();
+    int slots = 1, mmax = 1, pmax = 0, ninternal = 1, xslots = 1, xtape = 1;
+    int maxins = 2, xmaxins = 2;
+    size_t region = 256;
+    const int extra = a.metric == FM_CORRELATION || a.metric == FM_CORRELATION_SIGNED ? 2 : 0;
+    for (int i : ids) {
+        if (!b.valid[i]) continue;
+        const int4 f = b.finfo[i];
+        const int p = b.pcount[i];
+        slots = std::max(slots, f.w & 0xffff);
+        maxins = std::max(maxins, f.x + f.y);
+        region = std::max(region, ft_asm_region(f.z & 0xffff, f.w & 0xffff, f.w >> 16,
+                                                8 * ((p + 1 + extra + 7) / 8)));
+        mmax = std::max(mmax, b.node_off[i + 1] - b.node_off[i]);
+        pmax = std::max(pmax, p);
+        ninternal = std::max(ninternal, b.ninternal[i]);
+        if (a.metric == FM_IMPLICIT) {
+            const int4 x = xp.info[i];
+            xmaxins = std::max(xmaxins, x.x + x.y);
+            xslots = std::max(xslots, x.z);
+            xtape = std::max(xtape, x.w);
+        }
     }
-    return out;
+    ch.a.fslots = slots;
+    ch.a.fmaxins = maxins;
+    ch.a.asm_region = region;
+    ch.a.mmax = mmax;
+    ch.a.ijac_tape = ninternal;
+    ch.a.Wmax = 4 * ((pmax + 1 + 3) / 4);
+    ch.a.xslots = xslots;
+    ch.a.xtape = xtape;
+    ch.a.xmaxins = xmaxins;
+    const long long items = (long long)ch.ncand * a.ntiles;
+    if (a.metric == FM_IMPLICIT) {
+        ch.sw[ch.nk++] = sweep_shape(c, (const void *)ft_jac_sweep<FT_ITHREADS>, FT_ITHREADS,
+                                     ft_ijac_smem(mmax, ninternal, ch.a.Wmax, FT_ITHREADS), items);
+        const size_t xs = 8 * (size_t)((xmaxins + 1) & ~1) + 8 * FT_MAX_CONST +
+                          8 * (size_t)FT_ITHREADS * (xslots + xtape + a.v) + 8 * (size_t)FT_ITHREADS;
+        ch.sw[ch.nk++] = sweep_shape(c, (const void *)ft_sweep<FOP_ICOST, FT_ITHREADS>, FT_ITHREADS,
+                                     xs, items);
+        return ch;
+    }
+    const int T = small ? 128 : ft_cls_threads(cls);
+    const size_t sa = ft_sweep4_smem(FOP_ASM32, maxins, slots, region, T);
+    const size_t sl = ft_sweep4_smem(FOP_LOSS32, maxins, slots, region, 128);
+    if (extra) {
+        if (small) {
+            ch.sw[ch.nk++] = sweep_shape(c, (const void *)ft_sweep4<128, FOP_CASM, FOP_CSCORE>, 128,
+                                         std::max(sa, sl), items);
+        } else {
+            ch.sw[ch.nk++] = sweep_shape(c, casm_kernel(T), T, sa, items);
+            ch.sw[ch.nk++] = sweep_shape(c, (const void *)ft_sweep4<128, FOP_CSCORE>, 128, sl, items);
+        }
+    } else if (small) {
+        ch.sw[ch.nk++] = sweep_shape(
+            c, (const void *)ft_sweep4<128, FOP_ASM64, FOP_ASM32, FOP_LOSS64, FOP_LOSS32>, 128,
+            std::max(sa, sl), items);
+    } else {
+        ch.sw[ch.nk++] = sweep_shape(c, asm_kernel<FOP_ASM64, FOP_ASM32>(T), T, sa, items);
+        ch.sw[ch.nk++] = sweep_shape(c, (const void *)ft_sweep4<128, FOP_LOSS64, FOP_LOSS32>, 128, sl,
+                                     items);
+    }
+    return ch;
 }
 
-template <int OPK, int T>
-SweepLaunch sweep4_launch(RcCtx *c, const FitPrep &b, int Wmax)
+/* The context's side streams and their events, made on the first fit with
+   several chains and kept. */
+bool fit_side_streams(RcCtx *c)
 {
-    SweepLaunch s;
-    s.fn = (const void *)ft_sweep4<OPK, T>;
-    s.opk = OPK;
-    (void)Wmax;
-    const int bk = ft_base_kind(OPK);
-    const size_t reg = OPK != bk ? b.asm_reg[ft_kind_cls(OPK)]
-                       : (bk == FOP_CASM ? b.asm_region : b.asm_reg[0]);
-    s.smem = ft_sweep4_smem(OPK, b.fmaxins, b.fslots, reg, T);
-    rc_raise_smem(s.fn, s.smem);
-    s.grid = c->sm_count * occupancy(s.fn, T, s.smem);
-    s.threads = T;
-    return s;
+    if (c->fit_side[0]) return true;
+    for (int i = 0; i < FT_MAX_CHAINS; ++i) {
+        if (cudaStreamCreateWithFlags(&c->fit_side[i], cudaStreamNonBlocking) != cudaSuccess ||
+            cudaEventCreateWithFlags(&c->fit_ev[i], cudaEventDisableTiming) != cudaSuccess) {
+            cudaGetLastError();
+            rc_fit_free_streams(c);
+            return false;
+        }
+    }
+    return true;
 }
 
-/* Enqueue the whole fit on the context stream: init, the bounded steps, the
-   flush. */
-unsigned long long enqueue_fit(cudaStream_t s_, int sm_count, const FitArgs &a, int steps,
-                               const SweepLaunch *sw, int nkinds)
+/* Enqueue the whole fit: the subtree cache and the start on stream s_, the
+   bounded steps of each chain (the first on s_, the others on side streams
+   forked from it), the flush when all have joined. `a` is the whole batch
+   with the first chain's queues; the queues of all chains are `qbytes` from
+   a.counts on. */
+unsigned long long enqueue_fit(RcCtx *c, cudaStream_t s_, const FitArgs &a, int steps,
+                               const std::vector<FitChain> &chains, size_t qbytes)
 {
-    /* persistent grids take their items from work counters, so a grid no
-       larger than the items that can exist (a small batch) answers the
-       same and launches no idle blocks */
-    const int ctrl_grid = std::min(sm_count * 8, std::max(a.nprog, 1));
-    const int max_items = (int)std::min<long long>((long long)a.nprog * a.ntiles, 1LL << 30);
     unsigned long long k = 0;
     if (a.nsub > 0) {
         const size_t smem = 8 * (size_t)((a.sub_maxins + 1) & ~1) +
@@ -2447,23 +2502,38 @@ unsigned long long enqueue_fit(cudaStream_t s_, int sm_count, const FitArgs &a, 
             k = 2;
         }
     }
-    ft_step_reset<<<1, 32, 0, s_>>>(a, 1);
-    cudaMemsetAsync(a.work + 1 * FOP_COUNT, 0, sizeof(int) * FOP_COUNT, s_);
-    ft_control<<<ctrl_grid, FT_CTRL_T, 0, s_>>>(a, 1, 1);
+    cudaMemsetAsync(a.counts, 0, qbytes, s_);
+    ft_control<<<std::min(c->sm_count * 8, std::max(a.nprog, 1)), FT_CTRL_T, 0, s_>>>(a, 1, 1);
+    const int nch = (int)chains.size();
+    if (nch > 1) {
+        cudaEventRecord(c->fit_ev[0], s_);
+        for (int i = 1; i < nch; ++i) cudaStreamWaitEvent(c->fit_side[i], c->fit_ev[0], 0);
+    }
     for (int s = 0; s < steps; ++s) {
         const int q = s & 1;
-        ft_step_reset<<<1, 32, 0, s_>>>(a, q);
-        for (int k = 0; k < nkinds; ++k) {
-            const SweepLaunch &L = sw[k];
-            void *args[] = {(void *)&a, (void *)&q};
-            const int grid = std::max(1, std::min(L.grid, max_items));
-            cudaLaunchKernel(L.fn, dim3(grid), dim3(L.threads), args, L.smem, s_);
+        for (int i = 0; i < nch; ++i) {
+            const FitChain &ch = chains[i];
+            cudaStream_t cs = i == 0 ? s_ : c->fit_side[i];
+            for (int w = 0; w < ch.nk; ++w) {
+                const SweepLaunch &L = ch.sw[w];
+                void *args[] = {(void *)&ch.a, (void *)&q};
+                cudaLaunchKernel(L.fn, dim3(L.grid), dim3(L.threads), args, L.smem, cs);
+            }
+            ft_control<<<std::min(c->sm_count * 8, ch.ncand), FT_CTRL_T, 0, cs>>>(ch.a, q, 0);
+            k += 1ULL + (unsigned long long)ch.nk;
         }
-        ft_control<<<ctrl_grid, FT_CTRL_T, 0, s_>>>(a, q, 0);
+    }
+    for (int i = 1; i < nch; ++i) {
+        cudaEventRecord(c->fit_ev[i], c->fit_side[i]);
+        cudaStreamWaitEvent(s_, c->fit_ev[i], 0);
     }
     ft_flush<<<(a.nprog + 127) / 128, 128, 0, s_>>>(a);
-    return k + 3ULL + (unsigned long long)steps * (2ULL + (unsigned long long)nkinds);
+    return k + 2ULL;
 }
+
+/* At most this many (candidate, tile) items per SM: every kind of a step in
+   one launch, on one chain. */
+#define FT_SMALL_ITEMS_PER_SM 8
 
 float fit_run(RcCtx *c, const unsigned int *prog, const unsigned int *off, const int *pcount,
               int nprog, int kmax, const double *c0, const int *gauge, int iters, int metric,
@@ -2523,9 +2593,12 @@ float fit_run(RcCtx *c, const unsigned int *prog, const unsigned int *off, const
     const size_t io_end = rc_take(&cur, 0);
     const size_t o_state = rc_take(&cur, sizeof(FitState) * nprog);
     const size_t o_part = rc_take(&cur, sizeof(double) * (size_t)nprog * ntiles * FT_PART_STRIDE);
-    const size_t o_lists = rc_take(&cur, sizeof(int) * 2 * FOP_COUNT * (size_t)nprog);
-    const size_t o_counts = rc_take(&cur, sizeof(int) * 2 * FOP_COUNT);
-    const size_t o_work = rc_take(&cur, sizeof(int) * 2 * FOP_COUNT);
+    /* every chain's queues; counts and work counters, zeroed together */
+    const size_t o_lists =
+        rc_take(&cur, sizeof(int) * 2 * FOP_COUNT * (size_t)nprog * FT_MAX_CHAINS);
+    const size_t o_counts = rc_take(&cur, sizeof(int) * 2 * FOP_COUNT * FT_MAX_CHAINS);
+    const size_t o_work = rc_take(&cur, sizeof(int) * 2 * FOP_COUNT * FT_MAX_CHAINS);
+    const size_t q_end = rc_take(&cur, 0);
     const size_t o_cache = rc_take(&cur, sizeof(float) * (size_t)c->npad * (size_t)b.ncache);
     /* the f64 twin of the cache for the polish, when it fits the same cap */
     const bool use64 = use_cache && b.ncache > 0 && !(flags & 1) &&
@@ -2537,6 +2610,30 @@ float fit_run(RcCtx *c, const unsigned int *prog, const unsigned int *off, const
     st->alloc_ms += rc_now_ms() - t;
     unsigned char *dev = c->dev, *host = c->host;
     t = rc_now_ms();
+    /* the chains: a small batch is one; else one per assembly class, or an
+       implicit batch split by program length */
+    const bool small = (long long)nprog * ntiles <= (long long)c->sm_count * FT_SMALL_ITEMS_PER_SM;
+    std::vector<std::vector<int>> groups(FT_MAX_CHAINS);
+    std::vector<int> group_cls;
+    if (mode == 0) {
+        const int split = metric == FM_IMPLICIT && !small ? ijac_split(c, b, Wmax) : 0;
+        for (int i = 0; i < nprog; ++i) {
+            int g = 0;
+            if (!small)
+                g = metric == FM_IMPLICIT ? (b.node_off[i + 1] - b.node_off[i] <= split ? 1 : 0)
+                                          : b.finfo[i].z >> 16;
+            groups[g].push_back(i);
+        }
+        std::vector<std::vector<int>> used;
+        for (int g = 0; g < FT_MAX_CHAINS; ++g)
+            if (!groups[g].empty()) {
+                for (int i : groups[g]) b.finfo[i].z |= (int)used.size() << 24;
+                used.push_back(groups[g]);
+                group_cls.push_back(g);
+            }
+        groups.swap(used);
+        if (groups.size() > 1 && !fit_side_streams(c)) return -1.0f;
+    }
     memcpy(host + o_rec, prog, sizeof(uint32_t) * words);
     memcpy(host + o_noff, b.node_off.data(), sizeof(int) * (nprog + 1));
     memcpy(host + o_p, pcount, sizeof(int) * nprog);
@@ -2592,20 +2689,11 @@ float fit_run(RcCtx *c, const unsigned int *prog, const unsigned int *off, const
     a.xfins = reinterpret_cast<const FOp *>(dev + o_xfins);
     a.xfins_off = reinterpret_cast<const int *>(dev + o_xoff);
     a.xinfo = reinterpret_cast<const int4 *>(dev + o_xinfo);
-    a.xmaxins = xp.maxins;
-    a.xslots = xp.slots;
-    a.xtape = xp.tape;
-    a.asm_region = b.asm_region;
-    for (int k = 0; k < FT_NCLS; ++k) a.asm_reg[k] = b.asm_reg[k];
-    a.fslots = b.fslots;
     a.ftape = b.ftape;
-    a.fmaxins = b.fmaxins;
     a.iters = iters;
     a.metric = metric;
     a.flags = flags;
     a.ntiles = ntiles;
-    a.mmax = b.mmax;
-    a.Wmax = Wmax;
     a.nprog = nprog;
     a.state = reinterpret_cast<FitState *>(dev + o_state);
     a.part = reinterpret_cast<double *>(dev + o_part);
@@ -2616,43 +2704,16 @@ float fit_run(RcCtx *c, const unsigned int *prog, const unsigned int *off, const
     a.outsse = reinterpret_cast<double *>(dev + o_sse);
     a.outstatus = reinterpret_cast<int *>(dev + o_status);
 
-    SweepLaunch sw[16];
-    int nk = 0;
-    if (metric == FM_IMPLICIT) {
-        const IjacSplit js = ijac_split(c, b, Wmax);
-        a.ijac_small = js.small;
-        a.ijac_tape = js.tape;
-        a.ijac_tape_small = js.tape_small;
-        if (a.ijac_small > 0) {
-            sw[nk] = sweep_launch<FOP_IJACS>(c, a.ijac_small, a.ijac_tape_small, Wmax); ++nk;
+    std::vector<FitChain> chains;
+    if (mode == 0)
+        for (size_t g = 0; g < groups.size(); ++g) {
+            FitChain ch = make_chain(c, a, b, xp, groups[g], group_cls[g], small);
+            ch.a.lists = a.lists + g * 2 * FOP_COUNT * (size_t)nprog;
+            ch.a.counts = a.counts + g * 2 * FOP_COUNT;
+            ch.a.work = a.work + g * 2 * FOP_COUNT;
+            chains.push_back(ch);
         }
-        sw[nk] = sweep_launch<FOP_IJAC>(c, b.mmax, a.ijac_tape, Wmax); ++nk;
-        sw[nk] = icost_launch(c, xp); ++nk;
-    } else if (corr) {
-        sw[nk] = sweep4_launch<FOP_CASM, FT_ASM_T>(c, b, Wmax); ++nk;
-        sw[nk] = sweep4_launch<FOP_CSCORE, 128>(c, b, Wmax); ++nk;
-    } else {
-        /* one assembly launch per active-thread class present in the batch,
-           each in blocks of that many threads */
-        if (b.nclass[0]) { sw[nk] = sweep4_launch<FOP_ASM32, FT_ASM_T>(c, b, Wmax); ++nk; }
-        if (b.nclass[1]) { sw[nk] = sweep4_launch<FOP_ASM32_64A, 64>(c, b, Wmax); ++nk; }
-        if (b.nclass[2]) { sw[nk] = sweep4_launch<FOP_ASM32_64B, 64>(c, b, Wmax); ++nk; }
-        if (b.nclass[3]) { sw[nk] = sweep4_launch<FOP_ASM32_64, 64>(c, b, Wmax); ++nk; }
-        if (b.nclass[4]) { sw[nk] = sweep4_launch<FOP_ASM32_32, 32>(c, b, Wmax); ++nk; }
-        if (b.nclass[5]) { sw[nk] = sweep4_launch<FOP_ASM32_128L, 128>(c, b, Wmax); ++nk; }
-        sw[nk] = sweep4_launch<FOP_LOSS32, 128>(c, b, Wmax); ++nk;
-        /* the f64 sweeps serve the polish and the f64 rescue */
-        if ((flags & (FT_FLAG_NO_POLISH | FT_FLAG_NO_RESCUE)) !=
-            (FT_FLAG_NO_POLISH | FT_FLAG_NO_RESCUE)) {
-            if (b.nclass[0]) { sw[nk] = sweep4_launch<FOP_ASM64, FT_ASM_T>(c, b, Wmax); ++nk; }
-            if (b.nclass[1]) { sw[nk] = sweep4_launch<FOP_ASM64_64A, 64>(c, b, Wmax); ++nk; }
-            if (b.nclass[2]) { sw[nk] = sweep4_launch<FOP_ASM64_64B, 64>(c, b, Wmax); ++nk; }
-            if (b.nclass[3]) { sw[nk] = sweep4_launch<FOP_ASM64_64, 64>(c, b, Wmax); ++nk; }
-            if (b.nclass[4]) { sw[nk] = sweep4_launch<FOP_ASM64_32, 32>(c, b, Wmax); ++nk; }
-            if (b.nclass[5]) { sw[nk] = sweep4_launch<FOP_ASM64_128L, 128>(c, b, Wmax); ++nk; }
-            sw[nk] = sweep4_launch<FOP_LOSS64, 128>(c, b, Wmax); ++nk;
-        }
-    }
+    const size_t qbytes = q_end - o_counts;
     const int steps = max_steps(iters, metric);
 
     t = rc_now_ms();
@@ -2683,33 +2744,32 @@ float fit_run(RcCtx *c, const unsigned int *prog, const unsigned int *off, const
             one.outc = a.outc + (size_t)i * kmax;
             one.outsse = a.outsse + i;
             one.outstatus = a.outstatus + i;
-            /* only the assembly launches of this candidate's class */
-            SweepLaunch swc[16];
-            int nkc = 0;
-            const int cls = b.finfo[i].z >> 16;
-            for (int k = 0; k < nk; ++k) {
-                const int o = sw[k].opk;
-                const int bk = ft_base_kind(o);
-                if ((bk == FOP_ASM32 || bk == FOP_ASM64) && ft_kind_cls(o) != cls) continue;
-                swc[nkc++] = sw[k];
-            }
-            c->launches += enqueue_fit(c->s, c->sm_count, one, steps, swc, nkc);
+            /* one chain of this candidate's launch shapes */
+            const bool tiny = ntiles <= c->sm_count * FT_SMALL_ITEMS_PER_SM;
+            const std::vector<FitChain> own{
+                make_chain(c, one, b, xp, std::vector<int>(1, i), b.finfo[i].z >> 16, tiny)};
+            c->launches += enqueue_fit(c, c->s, one, steps, own, qbytes);
             ok = cudaGetLastError() == cudaSuccess;
         }
     } else {
-        char key[1024];
-        snprintf(key, sizeof(key), "%p|%d|%d|%d|%d|%d|%d|%d|%d|%d|%zu|%d|%d|%d|%zu", (void *)dev,
-                 nprog, kmax, ntiles, b.mmax, Wmax, iters, metric, flags, steps, io_end, b.fslots,
-                 b.ftape, b.fmaxins, b.asm_region);
-        const size_t kl = strlen(key);
-        snprintf(key + kl, sizeof(key) - kl,
-                 "|%d|%d|%d|%d|%d|%d|%d|%d|%d|%d|%d|%zu|%zu|%zu|%d|%d|%d", b.ncache, a.nsub,
-                 b.sub_slots, b.sub_maxins, xp.maxins, xp.slots, xp.tape, use64 ? 1 : 0,
-                 a.ijac_small, a.ijac_tape, a.ijac_tape_small, b.asm_reg[0], b.asm_reg[1],
-                 b.asm_reg[2], b.nclass[0], b.nclass[1], b.nclass[2]);
-        const size_t kl2 = strlen(key);
-        snprintf(key + kl2, sizeof(key) - kl2, "|%zu|%zu|%zu|%d|%d|%d", b.asm_reg[3],
-                 b.asm_reg[4], b.asm_reg[5], b.nclass[3], b.nclass[4], b.nclass[5]);
+        std::string key;
+        auto add = [&](unsigned long long v) { key += std::to_string(v) + "|"; };
+        add((unsigned long long)(uintptr_t)dev);
+        for (int v : {nprog, kmax, ntiles, iters, metric, flags, steps, b.ftape, b.ncache, a.nsub,
+                      b.sub_slots, b.sub_maxins, use64 ? 1 : 0})
+            add((unsigned long long)(unsigned)v);
+        add(io_end);
+        for (const FitChain &ch : chains) {
+            for (int v : {ch.ncand, ch.nk, ch.a.fslots, ch.a.fmaxins, ch.a.mmax, ch.a.Wmax,
+                          ch.a.ijac_tape, ch.a.xslots, ch.a.xtape, ch.a.xmaxins})
+                add((unsigned long long)(unsigned)v);
+            add(ch.a.asm_region);
+            for (int w = 0; w < ch.nk; ++w) {
+                add((unsigned long long)(uintptr_t)ch.sw[w].fn);
+                add(ch.sw[w].smem);
+                add((unsigned long long)ch.sw[w].grid);
+            }
+        }
         const bool replay = c->fit_graph && c->fit_graph_key == key;
         if (!replay && c->fit_seen_key != key) {
             /* a batch shape seen for the first time runs its steps directly:
@@ -2717,7 +2777,7 @@ float fit_run(RcCtx *c, const unsigned int *prog, const unsigned int *off, const
                instantiating the graph costs more than launching it once.
                The second call of a shape captures it, later ones replay. */
             c->fit_seen_key = key;
-            c->launches += enqueue_fit(c->s, c->sm_count, a, steps, sw, nk);
+            c->launches += enqueue_fit(c, c->s, a, steps, chains, qbytes);
             ok = cudaGetLastError() == cudaSuccess;
         } else {
             if (!replay) {
@@ -2730,7 +2790,7 @@ float fit_run(RcCtx *c, const unsigned int *prog, const unsigned int *off, const
                 cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking);
                 ok = cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
                 if (ok) {
-                    c->fit_graph_kernels = enqueue_fit(cap, c->sm_count, a, steps, sw, nk);
+                    c->fit_graph_kernels = enqueue_fit(c, cap, a, steps, chains, qbytes);
                     ok = cudaStreamEndCapture(cap, &g) == cudaSuccess && g;
                 }
                 if (ok) ok = cudaGraphInstantiate(&c->fit_graph, g, 0) == cudaSuccess;
@@ -2751,6 +2811,8 @@ float fit_run(RcCtx *c, const unsigned int *prog, const unsigned int *off, const
     st->launch_ms += rc_now_ms() - t;
     if (!ok || cudaGetLastError() != cudaSuccess) {
         cudaStreamSynchronize(c->s);
+        for (int i = 0; i < FT_MAX_CHAINS; ++i)
+            if (c->fit_side[i]) cudaStreamSynchronize(c->fit_side[i]);
         cudaGetLastError();
         return -1.0f;
     }

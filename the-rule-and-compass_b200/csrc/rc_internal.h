@@ -178,6 +178,8 @@ struct RcCtx {
     std::string fit_graph_key;
     std::string fit_seen_key;             /* the last batch shape run without a graph */
     unsigned long long fit_graph_kernels; /* kernel nodes in one replay */
+    cudaStream_t fit_side[6];             /* the fit's chains past the first, made on first use */
+    cudaEvent_t fit_ev[6];
 
     /* kernels this context has launched (graph replays count their nodes) */
     unsigned long long launches;
@@ -208,6 +210,8 @@ int rc_raise_smem(const void *fn, size_t bytes);
 /* Make sure the f64 twins exist (cast from the f32 rows when the caller never
    uploaded exact rows). */
 int rc_ensure_f64(RcCtx *c);
+/* Destroy the fit's side streams and their events. */
+void rc_fit_free_streams(RcCtx *c);
 /* Stream-ordered event synchronisation of the context's stream. */
 int rc_finish(RcCtx *c);
 
