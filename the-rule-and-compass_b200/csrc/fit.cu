@@ -247,22 +247,31 @@ __host__ __device__ inline size_t ft_rows_bytes(int Wmax, int T)
     return rows > part ? rows : part;
 }
 
-/* Threads of the implicit sweeps: every thread carries one row. */
+/* Threads of a group of the implicit sweeps (every thread carries one row)
+   and of their largest block. */
 #define FT_ITHREADS 64
+#define FT_IMAXT 512
 
-/* Dynamic shared memory of an exact-Jacobian sweep: the compact records
-   and their reference scratch for `mrec` records, the constants, the two
-   f64 tapes ([slot][T], `tcap` internal-node slots each), the Jacobian row
-   buffer and a reduction buffer. */
-__host__ __device__ inline size_t ft_ijac_smem(int mrec, int tcap, int Wmax, int T)
+/* Dynamic shared memory of an exact-Jacobian sweep of G groups: the compact
+   records and their reference scratch for `mrec` records, the constants, a
+   reduction buffer, and per group the two f64 tapes ([slot][FT_ITHREADS],
+   `tcap` internal-node slots each) and the Jacobian row buffer. */
+__host__ __device__ inline size_t ft_ijac_smem(int mrec, int tcap, int Wmax, int G)
 {
     return 16 * (size_t)mrec + 16 * (size_t)((mrec + 3) / 4) + 8 * (size_t)FT_MAX_CONST +
-           16 * (size_t)tcap * T + ft_rows_bytes(Wmax, T) + 8 * (size_t)T;
+           8 * (size_t)FT_ITHREADS * G +
+           (size_t)G * (16 * (size_t)tcap * FT_ITHREADS + ft_rows_bytes(Wmax, FT_ITHREADS));
+}
+
+/* ... and of a cost sweep. */
+inline size_t ft_icost_smem(int maxins, int slots, int tape, int v, int G)
+{
+    return 8 * (size_t)((maxins + 1) & ~1) + 8 * FT_MAX_CONST + 8 * (size_t)FT_ITHREADS * G +
+           8 * (size_t)FT_ITHREADS * G * (slots + tape + v);
 }
 
 /* Fixed-order reduction of the per-thread SYRK blocks over the row groups,
    written packed ([block][16]) to the tile's partial. */
-template <int T>
 __device__ __forceinline__ void ft_tile_gram_out(const Syrk &sy, const double acc[16],
                                                  double *buf, double *pt)
 {
@@ -272,7 +281,7 @@ __device__ __forceinline__ void ft_tile_gram_out(const Syrk &sy, const double ac
         for (int e = 0; e < 16; ++e) buf[(sy.rg * sy.nblk + sy.blk) * 16 + e] = acc[e];
     }
     __syncthreads();
-    for (int q = tid; q < sy.nblk * 16; q += T) {
+    for (int q = tid; q < sy.nblk * 16; q += blockDim.x) {
         const int blk = q >> 4, e = q & 15;
         double s = 0.0;
         for (int g = 0; g < sy.RG; ++g) s += buf[(g * sy.nblk + blk) * 16 + e];
@@ -285,28 +294,34 @@ __device__ __forceinline__ void ft_tile_gram_out(const Syrk &sy, const double ac
    sum w d^2 at `cd`, the Jacobian rows of sqrt(w) d (exact,
    forward-over-reverse, where the reference takes central differences
    with h = 1e-6 (1 + |c_j|)) and their J^T J / J^T r. An undefined row
-   marks the tile bad. `rec` holds the ni compact records of ij_compact;
-   `tape64` and `tan64` are the two f64 tapes. */
-template <int T>
+   marks the tile bad. `rec` holds the ni compact records of ij_compact. Each
+   group of FT_ITHREADS threads takes a chunk of that many rows a round, with
+   its own two f64 tapes of `tcap` slots and Jacobian rows (`gstride` doubles
+   apart from `groups` on); the chunks are then folded in ascending order, so
+   the sums do not depend on the groups of the launch. */
 __device__ void ft_tile_implicit(const FitArgs &a, const uint4 *rec, int ni, int p,
-                                 const double *cd, double *tape64, double *tan64, double *rows,
+                                 const double *cd, double *groups, size_t gstride, int tcap,
                                  double *red, int r0, int r1, double *pt)
 {
-    constexpr int TS = T;
-    const int tid = threadIdx.x;
+    constexpr int TS = FT_ITHREADS;
+    const int tid = threadIdx.x, grp = tid / TS, lt = tid % TS, G = blockDim.x / TS;
     const int W = 4 * ((p + 1 + 3) / 4);
-    const Syrk sy = ft_syrk_setup<T>(W);
+    const Syrk sy = ft_syrk_setup<TS>(W);
+    double *tape64 = groups + grp * gstride;
+    double *tan64 = tape64 + (size_t)tcap * TS;
+    double *rows = tan64 + (size_t)tcap * TS;
+    const size_t rows_at = 2 * (size_t)tcap * TS;
     double acc[16];
 #pragma unroll
     for (int e = 0; e < 16; ++e) acc[e] = 0.0;
     double cost = 0.0;
     int bad = 0;
-    double *tp = tape64 + tid;
-    double *myrow = rows + (size_t)tid * W;
+    double *tp = tape64 + lt;
+    double *myrow = rows + (size_t)lt * W;
     double x[FT_IMPLICIT_MAXV];
-    for (int base = r0; base < r1; base += TS) {
-        const int row = base + tid;
-        if (tid < TS) {
+    for (int base0 = r0; base0 < r1; base0 += G * TS) {
+        const int base = base0 + grp * TS, row = base + lt;
+        if (base < r1) {
             for (int j = 0; j < W; ++j) myrow[j] = 0.0;
             const double wr = (row < r1 && a.w) ? a.w[row] : 1.0;
             if (row < r1 && !(isfinite(wr) && wr >= 0.0)) bad = 1;
@@ -316,24 +331,28 @@ __device__ void ft_tile_implicit(const FitArgs &a, const uint4 *rec, int ni, int
                 double d;
                 const double sw = sqrt(wr);
                 const bool ok =
-                    ft_implicit_jac<TS>(rec, ni, x, a.v, cd, p, sw, tp, tan64 + tid, d, myrow);
+                    ft_implicit_jac<TS>(rec, ni, x, a.v, cd, p, sw, tp, tan64 + lt, d, myrow);
                 if (!ok) {
                     bad = 1;
                     for (int j = 0; j < p; ++j) myrow[j] = 0.0;
                 } else {
-                    const double r = sw * d;
-                    cost += r * r;
-                    myrow[p] = r;
+                    myrow[p] = sw * d;
                 }
             }
         }
         __syncthreads();
-        ft_syrk_chunk(sy, rows, W, TS, acc);
+        /* the chunks in ascending order, on the first group's threads */
+        for (int g = 0; grp == 0 && g < G && base0 + g * TS < r1; ++g) {
+            const double *rg = groups + g * gstride + rows_at;
+            const double r = rg[(size_t)lt * W + p];
+            cost += r * r;
+            ft_syrk_chunk(sy, rg, W, TS, acc);
+        }
         __syncthreads();
     }
     bad = __syncthreads_or(bad);
-    cost = ft_block_sum<T>(cost, red);
-    ft_tile_gram_out<T>(sy, acc, rows, pt);
+    cost = ft_sum_first(cost, red, TS);
+    ft_tile_gram_out(sy, acc, groups + rows_at, pt);
     if (tid == 0) {
         pt[FT_PART_LOSS] = cost;
         pt[FT_PART_BAD] = bad ? 1.0 : 0.0;
@@ -347,55 +366,65 @@ __device__ void ft_tile_implicit(const FitArgs &a, const uint4 *rec, int ni, int
    reverse sweep (fi_reverse_x). A row with a non-finite value or input
    gradient, or a zero gradient norm, marks the tile undefined
    (implicit.rs:156-174). */
-template <int T>
 __device__ void ft_tile_icost_x(const FitArgs &a, const FOp *fwd, const FOp *rev,
                                 const double *cd, FiV<double, 1>::V4 *stk,
                                 FiV<double, 1>::V4 *tape, FiV<double, 1>::V4 *ig, double *red,
                                 int r0, int r1, double *pt)
 {
-    const int tid = threadIdx.x;
+    constexpr int TS = FT_ITHREADS;
+    const int tid = threadIdx.x, grp = tid / TS, lt = tid % TS, G = blockDim.x / TS;
     double cost = 0.0;
     int bad = 0;
-    for (int base = r0; base < r1; base += T) {
-        const int row = base + tid;
+    /* sqrt(w) d of one row, 0 for a row that counts for nothing */
+    auto residual = [&](int row) {
         double fv;
-        fi_forward<double, 1, true>(fwd, cd, a.cols64 + row, a.npad, stk + tid, tape + tid, T, &fv);
-        if (row >= r1) continue;
+        fi_forward<double, 1, true>(fwd, cd, a.cols64 + row, a.npad, stk + lt, tape + lt, TS, &fv);
+        if (row >= r1) return 0.0;
         const double wr = a.w ? a.w[row] : 1.0;
         if (!(isfinite(wr) && wr >= 0.0)) {
             bad = 1;
-            continue;
+            return 0.0;
         }
-        if (wr == 0.0) continue;
+        if (wr == 0.0) return 0.0;
         if (!isfinite(fv)) {
             bad = 1;
-            continue;
+            return 0.0;
         }
-        for (int k = 0; k < a.v; ++k) ig[k * T + tid].v[0] = 0.0;
+        for (int k = 0; k < a.v; ++k) ig[k * TS + lt].v[0] = 0.0;
         double seed = 1.0;
-        fi_reverse_x<double, 1>(rev, stk + tid, tape + tid, T, ig + tid, &seed);
+        fi_reverse_x<double, 1>(rev, stk + lt, tape + lt, TS, ig + lt, &seed);
         double nsq = 0.0;
         bool ok = true;
         for (int k = 0; k < a.v; ++k) {
-            const double g = ig[k * T + tid].v[0];
+            const double g = ig[k * TS + lt].v[0];
             if (!isfinite(g)) ok = false;
             nsq += g * g;
         }
         const double norm = sqrt(nsq);
         if (!ok || !(isfinite(norm) && norm > 0.0)) {
             bad = 1;
-            continue;
+            return 0.0;
         }
         const double d = fv / norm;
         if (!isfinite(d)) {
             bad = 1;
-            continue;
+            return 0.0;
         }
-        const double r = sqrt(wr) * d;
-        cost += r * r;
+        return sqrt(wr) * d;
+    };
+    for (int base0 = r0; base0 < r1; base0 += G * TS) {
+        const int base = base0 + grp * TS;
+        red[tid] = base < r1 ? residual(base + lt) : 0.0;
+        __syncthreads();
+        /* the chunks in ascending order, on the first group's threads */
+        for (int g = 0; grp == 0 && g < G && base0 + g * TS < r1; ++g) {
+            const double r = red[g * TS + lt];
+            cost += r * r;
+        }
+        __syncthreads();
     }
     bad = __syncthreads_or(bad);
-    cost = ft_block_sum<T>(cost, red);
+    cost = ft_sum_first(cost, red, TS);
     if (tid == 0) {
         pt[FT_PART_LOSS] = cost;
         pt[FT_PART_BAD] = bad ? 1.0 : 0.0;
@@ -405,57 +434,54 @@ __device__ void ft_tile_icost_x(const FitArgs &a, const FOp *fwd, const FOp *rev
 
 /* The implicit cost sweep over every queued (candidate, tile) item of step
    parity q. */
-template <int OPK, int T>
-__global__ void __launch_bounds__(T) ft_sweep(FitArgs a, int q)
+__global__ void __launch_bounds__(FT_IMAXT, 1) ft_cost_sweep(FitArgs a, int q)
 {
     extern __shared__ __align__(16) unsigned char sm[];
-    static_assert(OPK == FOP_ICOST, "ft_sweep runs the cost kind");
-    {
-        /* [instructions | constants | spill slots | tape | input gradients | reduction] */
-        using V4 = FiV<double, 1>::V4;
-        FOp *ins = reinterpret_cast<FOp *>(sm);
-        double *cd = reinterpret_cast<double *>(sm + 8 * (size_t)((a.xmaxins + 1) & ~1));
-        V4 *stk = reinterpret_cast<V4 *>(cd + FT_MAX_CONST);
-        V4 *tape = stk + (size_t)a.xslots * T;
-        V4 *ig = tape + (size_t)a.xtape * T;
-        double *red = reinterpret_cast<double *>(ig + (size_t)a.v * T);
-        __shared__ int s_item;
-        const int tid = threadIdx.x;
-        ft_clear_other(a, q);
-        const int *list = a.lists + ((size_t)q * FOP_COUNT + OPK) * a.nprog;
-        const int total = a.counts[q * FOP_COUNT + OPK] * a.ntiles;
-        int *work = a.work + q * FOP_COUNT + OPK;
-        for (;;) {
-            if (tid == 0) s_item = atomicAdd(work, 1);
-            __syncthreads();
-            const int item = s_item;
-            __syncthreads();
-            if (item >= total) break;
-            const int cand = list[item / a.ntiles];
-            const int tile = item % a.ntiles;
-            const FitState *st = a.state + cand;
-            const int4 info = a.xinfo[cand];
-            const int ib = a.xfins_off[cand];
-            const int p = a.pcount[cand];
-            const int sel = st->sel;
-            for (int i = tid; i < info.x + info.y; i += T) ins[i] = a.xfins[ib + i];
-            if (tid < p) cd[tid] = sel ? st->trial[tid] : st->c[tid];
-            __syncthreads();
-            const int r0 = tile * FT_TILE_ROWS;
-            const int r1 = min(a.n, r0 + FT_TILE_ROWS);
-            double *pt = a.part + ((size_t)cand * a.ntiles + tile) * FT_PART_STRIDE;
-            ft_tile_icost_x<T>(a, ins, ins + info.x, cd, stk, tape, ig, red, r0, r1, pt);
-            __syncthreads();
-        }
+    /* [instructions | constants | reduction | per group: spill slots | tape |
+       input gradients] */
+    using V4 = FiV<double, 1>::V4;
+    const int tid = threadIdx.x, T = blockDim.x, grp = tid / FT_ITHREADS;
+    FOp *ins = reinterpret_cast<FOp *>(sm);
+    double *cd = reinterpret_cast<double *>(sm + 8 * (size_t)((a.xmaxins + 1) & ~1));
+    double *red = cd + FT_MAX_CONST;
+    V4 *stk = reinterpret_cast<V4 *>(red + T) +
+              (size_t)grp * FT_ITHREADS * (a.xslots + a.xtape + a.v);
+    V4 *tape = stk + (size_t)a.xslots * FT_ITHREADS;
+    V4 *ig = tape + (size_t)a.xtape * FT_ITHREADS;
+    __shared__ int s_item;
+    ft_clear_other(a, q);
+    const int *list = a.lists + ((size_t)q * FOP_COUNT + FOP_ICOST) * a.nprog;
+    const int total = a.counts[q * FOP_COUNT + FOP_ICOST] * a.ntiles;
+    int *work = a.work + q * FOP_COUNT + FOP_ICOST;
+    for (;;) {
+        if (tid == 0) s_item = atomicAdd(work, 1);
+        __syncthreads();
+        const int item = s_item;
+        __syncthreads();
+        if (item >= total) break;
+        const int cand = list[item / a.ntiles];
+        const int tile = item % a.ntiles;
+        const FitState *st = a.state + cand;
+        const int4 info = a.xinfo[cand];
+        const int ib = a.xfins_off[cand];
+        const int p = a.pcount[cand];
+        const int sel = st->sel;
+        for (int i = tid; i < info.x + info.y; i += T) ins[i] = a.xfins[ib + i];
+        if (tid < p) cd[tid] = sel ? st->trial[tid] : st->c[tid];
+        __syncthreads();
+        const int r0 = tile * FT_TILE_ROWS;
+        const int r1 = min(a.n, r0 + FT_TILE_ROWS);
+        double *pt = a.part + ((size_t)cand * a.ntiles + tile) * FT_PART_STRIDE;
+        ft_tile_icost_x(a, ins, ins + info.x, cd, stk, tape, ig, red, r0, r1, pt);
+        __syncthreads();
     }
 }
 
 /* The exact-Jacobian sweep over every queued (candidate, tile) item of step
-   parity q: eight 64-thread blocks per SM fit beside the compact tapes, so
+   parity q: eight groups of 64 threads per SM fit beside the compact tapes, so
    registers are held to that. A chain's launch is laid out for its own record
    and tape bounds. */
-template <int T>
-__global__ void __launch_bounds__(T, 8) ft_jac_sweep(FitArgs a, int q)
+__global__ void __launch_bounds__(FT_IMAXT, 1) ft_jac_sweep(FitArgs a, int q)
 {
     extern __shared__ __align__(16) unsigned char sm[];
     constexpr int OPK = FOP_IJAC;
@@ -464,12 +490,11 @@ __global__ void __launch_bounds__(T, 8) ft_jac_sweep(FitArgs a, int q)
     uint4 *rec = reinterpret_cast<uint4 *>(sm);
     unsigned *refs = reinterpret_cast<unsigned *>(sm + 16 * (size_t)mcap);
     double *cd = reinterpret_cast<double *>(sm + 16 * (size_t)mcap + 16 * (size_t)((mcap + 3) / 4));
-    double *tape64 = cd + FT_MAX_CONST;
-    double *tan64 = tape64 + (size_t)tcap * T;
-    double *rows = tan64 + (size_t)tcap * T;
-    double *red = rows + ft_rows_bytes(a.Wmax, T) / 8;
+    const int tid = threadIdx.x, T = blockDim.x;
+    double *red = cd + FT_MAX_CONST;
+    double *groups = red + T;
+    const size_t gstride = 2 * (size_t)tcap * FT_ITHREADS + ft_rows_bytes(a.Wmax, FT_ITHREADS) / 8;
     __shared__ int s_item, s_ni;
-    const int tid = threadIdx.x;
     ft_clear_other(a, q);
     const int *list = a.lists + ((size_t)q * FOP_COUNT + OPK) * a.nprog;
     const int total = a.counts[q * FOP_COUNT + OPK] * a.ntiles;
@@ -495,7 +520,7 @@ __global__ void __launch_bounds__(T, 8) ft_jac_sweep(FitArgs a, int q)
         const int r0 = tile * FT_TILE_ROWS;
         const int r1 = min(a.n, r0 + FT_TILE_ROWS);
         double *pt = a.part + ((size_t)cand * a.ntiles + tile) * FT_PART_STRIDE;
-        ft_tile_implicit<T>(a, rec, s_ni, p, cd, tape64, tan64, rows, red, r0, r1, pt);
+        ft_tile_implicit(a, rec, s_ni, p, cd, groups, gstride, tcap, red, r0, r1, pt);
         __syncthreads();
     }
 }
@@ -515,6 +540,7 @@ __global__ void __launch_bounds__(T, 8) ft_jac_sweep(FitArgs a, int q)
 #define FT_ASM64_NR 1
 #define FT_LOSS32_NR 4
 #define FT_LOSS64_NR 2
+#define FT_LOSS_T 128 /* threads of an objective group */
 
 /* Per-candidate shared region of an assembly sweep at A active threads:
    spill slots and partial tape ([slot][A] 8-byte row vectors), then the
@@ -664,12 +690,12 @@ __device__ __forceinline__ FtRow ft_row_f64(const FitArgs &a, int rr, int r1, do
     return o;
 }
 
-/* Fold the warp's NR * 32 rows of the column-major Jacobian into its
-   J^T J | J^T r blocks with f64 tensor-core MMAs (f32 values widen
-   exactly, so products are exact and sums f64). */
-template <int NB, typename V, int NR>
+/* Fold NR * 32 rows (logical warp w) of the column-major Jacobian into the
+   8x8 blocks of J^T J | J^T r that `own` names, with f64 tensor-core MMAs
+   (f32 values widen exactly, so products are exact and sums f64). */
+template <int NB, bool ALL, typename V, int NR>
 __device__ __forceinline__ void ft_fold(const V *g, int R, int A, int w, int gid, int tig,
-                                        double (*acc)[2])
+                                        unsigned own, double (*acc)[2])
 {
 #pragma unroll 4
     for (int s = 0; s < 8 * NR; ++s) {
@@ -682,46 +708,68 @@ __device__ __forceinline__ void ft_fold(const V *g, int R, int A, int w, int gid
 #pragma unroll
         for (int I = 0; I < NB; ++I)
 #pragma unroll
-            for (int J = 0; J <= I; ++J, ++b) fi_dmma(acc[b][0], acc[b][1], x[I], x[J]);
+            for (int J = 0; J <= I; ++J, ++b)
+                if (ALL || (own >> b) & 1u) fi_dmma(acc[b][0], acc[b][1], x[I], x[J]);
     }
 }
 
 /* Assembly of one tile in f32 or f64: the forward sweep of the thread's
    rows, the reverse sweep seeded with each row's square-root weight (so it
    yields the weighted Jacobian row), the weighted residual as column p, and
-   the warp's rows folded into the augmented Gram matrix. Warps work
-   independently over their own rows; the tile's sum is a fixed-order sum
-   over warps, written in the packed 4x4-block layout the controller reads. */
-template <typename V, int NR, int T, bool CORR>
+   the rows folded into the augmented Gram matrix, written in the packed
+   4x4-block layout the controller reads.
+   A tile is a sequence of chunks of NR * A rows, folded per logical warp (32
+   of the A threads) in ascending order, and the tile's sum is a fixed-order
+   sum over logical warps. A block of A threads takes the chunks one by one,
+   its warps independent of each other. A larger block takes G chunks a
+   round, one per group of A threads with its own region; the round's chunks
+   are then folded in order, each group folding its share of the Gram's 8x8
+   blocks. Every block's MMAs and every row's loss keep their order, so the
+   bits do not depend on G. */
+template <typename V, int NR, bool CORR, bool GROUPED>
 __device__ void ft_tile_asm(const FitArgs &a, const FOp *fwd, const FOp *rev, int p, int A,
-                            int slots, int ntape, const V *cv, unsigned char *region,
+                            int slots, int ntape, const V *cv, unsigned char *regions,
                             double *red, int r0, int r1, double *pt, const V *ccols)
 {
     using F = FiV<V, NR>;
     using V4 = typename F::V4;
     constexpr bool F64 = sizeof(V) == 8;
-    const int tid = threadIdx.x;
-    const int lane = tid & 31, w = tid >> 5, gid = lane >> 2, tig = lane & 3;
+    const int tid = threadIdx.x, T = blockDim.x;
     const int ncols = p + (CORR ? 3 : 1);
-    const int NB = (ncols + 7) / 8;
+    const int NB = (ncols + 7) / 8, NBLK = NB * (NB + 1) / 2;
     const int W8 = 8 * NB, R = NR * A + 4;
+    /* groups of A threads, each with its region and (with several) its rows'
+       losses of the round */
+    const size_t reg1 = ft_asm_region(A, slots, ntape, W8);
+    const int la = 31 - __clz(A); /* A is a power of two */
+    const size_t gstride = GROUPED ? reg1 + 16 * (size_t)A : 0;
+    const int G = GROUPED ? max(1, min(T >> la, (int)(a.asm_region / gstride))) : 1;
+    const int grp = GROUPED ? tid >> la : 0, at = GROUPED ? tid & (A - 1) : tid;
+    const int lane = tid & 31, w = at >> 5, gid = lane >> 2, tig = lane & 3;
+    const bool mine = !GROUPED || grp < G;
+    const size_t g_at = (size_t)(slots + ntape) * A * sizeof(V4);
+    unsigned char *region = regions + grp * gstride;
     V4 *stk = reinterpret_cast<V4 *>(region);
     V4 *tape = stk + slots * A;
-    V *g = reinterpret_cast<V *>(tape + ntape * A);
+    V *g = reinterpret_cast<V *>(region + g_at);
     const V *cols = F64 ? reinterpret_cast<const V *>(a.cols64) : reinterpret_cast<const V *>(a.cols);
-    for (int i = tid; i < W8 * R; i += T) g[i] = V(0);
+    if (mine)
+        for (int i = at; i < W8 * R; i += A) g[i] = V(0);
+    unsigned own = 0;
+    for (int b = grp; b < NBLK; b += G) own |= 1u << b;
     __syncthreads();
     double acc[6][2];
 #pragma unroll
     for (int b = 0; b < 6; ++b) acc[b][0] = acc[b][1] = 0.0;
     double loss = 0.0;
     int bad = 0, skipped = 0;
-    if (tid < A) {
-        V *gt = g + tid;
-        for (int base = r0; base < r1; base += NR * A) {
-            const int row = base + NR * tid;
+    const int nchunk = (r1 - r0 + NR * A - 1) / (NR * A);
+    for (int c0 = 0; c0 < nchunk; c0 += G) {
+        if (mine && c0 + grp < nchunk) {
+            V *gt = g + at;
+            const int row = r0 + (c0 + grp) * NR * A + NR * at;
             V pr[NR];
-            fi_forward<V, NR, true>(fwd, cv, cols + row, a.npad, stk + tid, tape + tid, A, pr,
+            fi_forward<V, NR, true>(fwd, cv, cols + row, a.npad, stk + at, tape + at, A, pr,
                                     ccols + row);
             FtRow rw[NR];
             V seed[NR];
@@ -734,7 +782,7 @@ __device__ void ft_tile_asm(const FitArgs &a, const FOp *fwd, const FOp *rev, in
                 seed[i] = (V)rw[i].seed;
                 special = special || rw[i].s_zero != 0.0f;
             }
-            const bool fin = fi_reverse<V, NR>(rev, stk + tid, tape + tid, A, gt, R, A, seed);
+            const bool fin = fi_reverse<V, NR>(rev, stk + at, tape + at, A, gt, R, A, seed);
             if (!fin || special) {
                 /* rare rows: a non-finite Jacobian entry (the row is dropped
                    from the Jacobian; in f32 it counts as failed), or a zero
@@ -770,23 +818,46 @@ __device__ void ft_tile_asm(const FitArgs &a, const FOp *fwd, const FOp *rev, in
                     const bool jac = rw[i].ok && rw[i].seed != 0.0;
                     gt[p * R + i * A] = jac ? (V)rw[i].res : V(0);
                 }
-                if (rw[i].ok) loss += rw[i].loss;
-                else if (rw[i].use) bad = 1;
+                if (!GROUPED) {
+                    if (rw[i].ok) loss += rw[i].loss;
+                } else {
+                    reinterpret_cast<double *>(region + reg1)[i * A + at] =
+                        rw[i].ok ? rw[i].loss : 0.0;
+                }
+                if (!rw[i].ok && rw[i].use) bad = 1;
             }
+        }
+        if constexpr (!GROUPED) {
             __syncwarp();
-            if (NB <= 1) ft_fold<1, V, NR>(g, R, A, w, gid, tig, acc);
-            else if (NB == 2) ft_fold<2, V, NR>(g, R, A, w, gid, tig, acc);
-            else ft_fold<3, V, NR>(g, R, A, w, gid, tig, acc);
+            if (NB <= 1) ft_fold<1, true, V, NR>(g, R, A, w, gid, tig, own, acc);
+            else if (NB == 2) ft_fold<2, true, V, NR>(g, R, A, w, gid, tig, own, acc);
+            else ft_fold<3, true, V, NR>(g, R, A, w, gid, tig, own, acc);
             __syncwarp();
+        } else {
+            __syncthreads();
+            const int nc = mine ? min(G, nchunk - c0) : 0;
+            for (int k = 0; k < nc; ++k) {
+                const V *gk = reinterpret_cast<const V *>(regions + k * gstride + g_at);
+                if (own) {
+                    if (NB <= 1) ft_fold<1, true, V, NR>(gk, R, A, w, gid, tig, own, acc);
+                    else if (NB == 2) ft_fold<2, false, V, NR>(gk, R, A, w, gid, tig, own, acc);
+                    else ft_fold<3, false, V, NR>(gk, R, A, w, gid, tig, own, acc);
+                }
+                if (grp == 0) {
+                    const double *lk = reinterpret_cast<const double *>(regions + k * gstride + reg1);
+#pragma unroll
+                    for (int i = 0; i < NR; ++i) loss += lk[i * A + at];
+                }
+            }
+            __syncthreads();
         }
     }
     __syncthreads();
-    const int NBLK = NB * (NB + 1) / 2;
-    double *gb = reinterpret_cast<double *>(region);
-    if (tid < A) {
+    double *gb = reinterpret_cast<double *>(regions);
+    if (mine) {
 #pragma unroll
         for (int b = 0; b < 6; ++b) {
-            if (b >= NBLK) break;
+            if (b >= NBLK || !((own >> b) & 1u)) continue;
             gb[(w * NBLK + b) * 64 + gid * 8 + 2 * tig] = acc[b][0];
             gb[(w * NBLK + b) * 64 + gid * 8 + 2 * tig + 1] = acc[b][1];
         }
@@ -809,7 +880,7 @@ __device__ void ft_tile_asm(const FitArgs &a, const FOp *fwd, const FOp *rev, in
     }
     bad = __syncthreads_or(bad);
     skipped = __syncthreads_or(skipped);
-    loss = ft_block_sum<T>(loss, red);
+    loss = ft_sum_first(loss, red, A);
     if (tid == 0) {
         pt[FT_PART_LOSS] = loss;
         pt[FT_PART_BAD] = bad ? 1.0 : 0.0;
@@ -818,19 +889,23 @@ __device__ void ft_tile_asm(const FitArgs &a, const FOp *fwd, const FOp *rev, in
 }
 
 /* Objective of one tile in f32 or f64 (eval.cu:1808-1855): the forward
-   sweep only; a row that is not finite costs 1e30. */
-template <typename V, int NR, int T>
+   sweep only; a row that is not finite costs 1e30. Each group of FT_LOSS_T
+   threads takes a chunk of NR * FT_LOSS_T rows a round, with its own `slots`
+   spill slots (`stk` is this thread's group's); rows add up in one order
+   whatever the groups. */
+template <typename V, int NR, bool GROUPED>
 __device__ void ft_tile_loss(const FitArgs &a, const FOp *ins, const V *cv,
-                             typename FiV<V, NR>::V4 *stk, double *red, int r0, int r1, double *pt,
-                             const V *ccols)
+                             typename FiV<V, NR>::V4 *stk, int slots, double *red, int r0, int r1,
+                             double *pt, const V *ccols)
 {
     constexpr bool F64 = sizeof(V) == 8;
     const V *cols = F64 ? reinterpret_cast<const V *>(a.cols64) : reinterpret_cast<const V *>(a.cols);
-    const int tid = threadIdx.x;
+    using F = FiV<V, NR>;
+    constexpr int TS = FT_LOSS_T;
+    const int tid = threadIdx.x, grp = GROUPED ? tid / TS : 0, lt = GROUPED ? tid % TS : tid;
+    const int G = GROUPED ? blockDim.x / TS : 1;
     double local = 0.0;
-    for (int row = r0 + NR * tid; row < r1; row += NR * T) {
-        V pr[NR];
-        fi_forward<V, NR, false>(ins, cv, cols + row, a.npad, stk + tid, nullptr, T, pr, ccols + row);
+    auto add_rows = [&](int row, const V *pr) {
 #pragma unroll
         for (int i = 0; i < NR; ++i) {
             const int rr = row + i;
@@ -858,8 +933,30 @@ __device__ void ft_tile_loss(const FitArgs &a, const FOp *ins, const V *cv,
                 else local += wr * (double)ft_row_loss_f(r, a.metric);
             }
         }
+    };
+    for (int base = r0; base < r1; base += G * NR * TS) {
+        const int row = base + grp * NR * TS + NR * lt;
+        V pr[NR];
+        if (row < r1)
+            fi_forward<V, NR, false>(ins, cv, cols + row, a.npad, stk + lt, nullptr, TS, pr,
+                                     ccols + row);
+        if constexpr (!GROUPED) {
+            if (row < r1) add_rows(row, pr);
+        } else {
+            /* the round's chunks in ascending order, on the first group's
+               threads: each prediction waits in its thread's first spill slot */
+            if (row < r1) stk[lt] = F::pack(pr);
+            __syncthreads();
+            for (int g = 0; grp == 0 && g < G; ++g) {
+                const int rk = base + g * NR * TS + NR * lt;
+                if (rk >= r1) break;
+                F::unpack(stk[(size_t)g * slots * TS + lt], pr);
+                add_rows(rk, pr);
+            }
+            __syncthreads();
+        }
     }
-    const double total = ft_block_sum<T>(local, red);
+    const double total = ft_sum_first(local, red, TS);
     if (tid == 0) {
         pt[FT_PART_LOSS] = total;
         pt[FT_PART_BAD] = 0.0;
@@ -871,15 +968,16 @@ __device__ void ft_tile_loss(const FitArgs &a, const FOp *ins, const V *cv,
    sum w y^2 in f64 from the f32 forward sweep, in pt[0..5]. A row whose
    prediction or target is not finite marks the tile bad, which rejects the
    trial. */
-template <int NR, int T>
+template <int NR>
 __device__ void ft_tile_corr_score(const FitArgs &a, const FOp *ins, const float *cv,
                                    typename FiV<float, NR>::V4 *stk, double *red, int r0, int r1,
                                    double *pt, const float *ccols)
 {
+    constexpr int T = FT_LOSS_T; /* a larger block's other threads wait */
     const int tid = threadIdx.x;
     double m[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
     int bad = 0;
-    for (int row = r0 + NR * tid; row < r1; row += NR * T) {
+    for (int row = r0 + NR * tid; tid < T && row < r1; row += NR * T) {
         float pr[NR];
         fi_forward<float, NR, false>(ins, cv, a.cols + row, a.npad, stk + tid, nullptr, T, pr,
                                      ccols + row);
@@ -905,14 +1003,15 @@ __device__ void ft_tile_corr_score(const FitArgs &a, const FOp *ins, const float
     bad = __syncthreads_or(bad);
 #pragma unroll
     for (int k = 0; k < 6; ++k) {
-        const double s = ft_block_sum<T>(m[k], red);
+        const double s = ft_sum_first(m[k], red, T);
         if (tid == 0) pt[k] = s;
     }
     if (tid == 0) pt[FT_PART_BAD] = bad ? 1.0 : 0.0;
 }
 
-/* One (candidate, tile) item of a sweep of kind OPK in a block of T threads. */
-template <int OPK, int T>
+/* One (candidate, tile) item of a sweep of kind OPK (GROUPED: in a block of
+   several groups). */
+template <int OPK, bool GROUPED>
 __device__ void ft_sweep_item(const FitArgs &a, unsigned char *sm, int cand, int tile)
 {
     using V = typename std::conditional<OPK == FOP_ASM64 || OPK == FOP_LOSS64, double, float>::type;
@@ -924,10 +1023,10 @@ __device__ void ft_sweep_item(const FitArgs &a, unsigned char *sm, int cand, int
     FOp *ins = reinterpret_cast<FOp *>(sm);
     V *cv = reinterpret_cast<V *>(sm + 8 * (size_t)((a.fmaxins + 1) & ~1));
     unsigned char *region = sm + 8 * (size_t)((a.fmaxins + 1) & ~1) + 8 * FT_MAX_CONST;
+    const int tid = threadIdx.x, T = blockDim.x;
+    const int slots = a.fslots > 0 ? a.fslots : 1;
     double *red = reinterpret_cast<double *>(
-        region + (ft_op_assembles(OPK) ? a.asm_region
-                                       : 16 * (size_t)(a.fslots > 0 ? a.fslots : 1) * T));
-    const int tid = threadIdx.x;
+        region + (ft_op_assembles(OPK) ? a.asm_region : 16 * (size_t)slots * T));
     const FitState *st = a.state + cand;
     const int ib = a.fins_off[cand];
     const int4 info = a.finfo[cand];
@@ -953,12 +1052,14 @@ __device__ void ft_sweep_item(const FitArgs &a, unsigned char *sm, int cand, int
     const int r1 = min(a.n, r0 + FT_TILE_ROWS);
     double *pt = a.part + ((size_t)cand * a.ntiles + tile) * FT_PART_STRIDE;
     if constexpr (ft_op_assembles(OPK))
-        ft_tile_asm<V, NR, T, OPK == FOP_CASM>(a, ins, ins + nf, p, info.z & 0xffff, info.w & 0xffff,
-                                               info.w >> 16, cv, region, red, r0, r1, pt, ccols);
+        ft_tile_asm<V, NR, OPK == FOP_CASM, GROUPED>(a, ins, ins + nf, p, info.z & 0xffff, info.w & 0xffff,
+                                            info.w >> 16, cv, region, red, r0, r1, pt, ccols);
     else if constexpr (OPK == FOP_CSCORE)
-        ft_tile_corr_score<NR, T>(a, ins, cv, reinterpret_cast<V4 *>(region), red, r0, r1, pt, ccols);
+        ft_tile_corr_score<NR>(a, ins, cv, reinterpret_cast<V4 *>(region), red, r0, r1, pt, ccols);
     else
-        ft_tile_loss<V, NR, T>(a, ins, cv, reinterpret_cast<V4 *>(region), red, r0, r1, pt, ccols);
+        ft_tile_loss<V, NR, GROUPED>(a, ins, cv,
+                            reinterpret_cast<V4 *>(region) + (size_t)(tid / FT_LOSS_T) * slots * FT_LOSS_T,
+                            slots, red, r0, r1, pt, ccols);
 }
 
 /* The sweeps of kinds K0, K1, ... of step parity q in one launch: a
@@ -967,9 +1068,8 @@ __device__ void ft_sweep_item(const FitArgs &a, unsigned char *sm, int cand, int
    run beside the next kind's. Registers are held to 640 threads an SM for the
    assemblies, what their shared memory allows (5 blocks of 128 threads at
    40 KB), and to 1,024 for the objective sweeps. */
-template <int T, int K0, int... KS>
-__global__ void __launch_bounds__(T, ft_op_assembles(K0) ? 640 / T : 1024 / T)
-    ft_sweep4(FitArgs a, int q)
+template <bool GROUPED, int K0, int... KS>
+__global__ void __launch_bounds__(ft_op_assembles(K0) ? 640 : 1024, 1) ft_sweep4(FitArgs a, int q)
 {
     extern __shared__ __align__(16) unsigned char sm[];
     constexpr int kinds[] = {K0, KS...};
@@ -1009,10 +1109,10 @@ __global__ void __launch_bounds__(T, ft_op_assembles(K0) ? 640 / T : 1024 / T)
             }
         }
         if constexpr (NK == 1) {
-            ft_sweep_item<K0, T>(a, sm, cand, tile);
+            ft_sweep_item<K0, GROUPED>(a, sm, cand, tile);
         } else {
             auto run = [&](auto K) {
-                if (kind == decltype(K)::value) ft_sweep_item<decltype(K)::value, T>(a, sm, cand, tile);
+                if (kind == decltype(K)::value) ft_sweep_item<decltype(K)::value, GROUPED>(a, sm, cand, tile);
             };
             run(std::integral_constant<int, K0>{});
             (run(std::integral_constant<int, KS>{}), ...);
@@ -2350,13 +2450,13 @@ int ijac_split(RcCtx *c, const FitPrep &b, int Wmax)
             tape = std::max(tape, b.ninternal[i]);
         }
     if (ms.size() < 2) return out;
-    const void *fn = (const void *)ft_jac_sweep<FT_ITHREADS>;
+    const void *fn = (const void *)ft_jac_sweep;
     /* occupancy queries up to the largest layout the split can choose */
-    const size_t smax = ft_ijac_smem(b.mmax, tape, Wmax, FT_ITHREADS);
+    const size_t smax = ft_ijac_smem(b.mmax, tape, Wmax, 1);
     if (rc_raise_smem(fn, smax) != 0) return out;
     std::sort(ms.begin(), ms.end());
     auto occ = [&](int mrec, int tcap) {
-        return (double)occupancy(fn, FT_ITHREADS, ft_ijac_smem(mrec, tcap, Wmax, FT_ITHREADS));
+        return (double)occupancy(fn, FT_ITHREADS, ft_ijac_smem(mrec, tcap, Wmax, 1));
     };
     double total = 0.0;
     for (const auto &e : ms) total += e.second + 1;
@@ -2378,21 +2478,18 @@ int ijac_split(RcCtx *c, const FitPrep &b, int Wmax)
     return best <= 0.95 * one ? out : 0;
 }
 
-/* The assembly and objective launches of a class, one per block width. */
-template <int K64, int K32>
-const void *asm_kernel(int threads)
-{
-    return threads == 128  ? (const void *)ft_sweep4<128, K64, K32>
-           : threads == 64 ? (const void *)ft_sweep4<64, K64, K32>
-                           : (const void *)ft_sweep4<32, K64, K32>;
-}
-
-const void *casm_kernel(int threads)
-{
-    return threads == 128  ? (const void *)ft_sweep4<128, FOP_CASM>
-           : threads == 64 ? (const void *)ft_sweep4<64, FOP_CASM>
-                           : (const void *)ft_sweep4<32, FOP_CASM>;
-}
+/* Shared memory a block may ask for; threads of a grouped block; a chain whose
+   (candidate, tile) items are fewer than this many waves of one-group blocks
+   takes grouped ones. A grouped block holds 4 to 8 chunks of a tile where a
+   one-group block holds one, so the last tile of a step ends that much
+   sooner: 131 candidates x 16,827 rows 21.4 -> 11.8 ms, 40 x 131,072 (four
+   waves) 14.2 -> 13.2 ms. It fits fewer threads an SM (512 against 640 of
+   A = 128), so full waves prefer one group: the classes of A = 128 take
+   grouped blocks below one wave (200 short candidates x 60,000 rows: 6.5 ms
+   with one group, 7.7 grouped). */
+#define FT_SMEM_MAX ((size_t)226 * 1024)
+#define FT_GROUP_T 512
+#define FT_GROUP_WAVES 4
 
 /* The chain of the candidates `ids` (indexes into the batch; `cls` their
    assembly class): the batch's arguments `a` with the chain's launch shapes.
@@ -2436,33 +2533,81 @@ FitChain make_chain(RcCtx *c, const FitArgs &a, const FitPrep &b, const XPrep &x
     ch.a.xmaxins = xmaxins;
     const long long items = (long long)ch.ncand * a.ntiles;
     if (a.metric == FM_IMPLICIT) {
-        ch.sw[ch.nk++] = sweep_shape(c, (const void *)ft_jac_sweep<FT_ITHREADS>, FT_ITHREADS,
-                                     ft_ijac_smem(mmax, ninternal, ch.a.Wmax, FT_ITHREADS), items);
-        const size_t xs = 8 * (size_t)((xmaxins + 1) & ~1) + 8 * FT_MAX_CONST +
-                          8 * (size_t)FT_ITHREADS * (xslots + xtape + a.v) + 8 * (size_t)FT_ITHREADS;
-        ch.sw[ch.nk++] = sweep_shape(c, (const void *)ft_sweep<FOP_ICOST, FT_ITHREADS>, FT_ITHREADS,
-                                     xs, items);
+        /* groups a block: as many rows in flight an SM as the shared memory
+           allows, then as many groups as that leaves (a tile's latency) */
+        auto groups = [&](const void *fn, auto smem) {
+            int best = 1, rows = 0;
+            for (int g = 1; g <= FT_IMAXT / FT_ITHREADS; ++g) {
+                const size_t s = smem(g);
+                if (s > FT_SMEM_MAX || rc_raise_smem(fn, s) != 0) break;
+                const int r = occupancy(fn, g * FT_ITHREADS, s) * g;
+                if (r >= rows) {
+                    rows = r;
+                    best = g;
+                }
+            }
+            return best;
+        };
+        const void *jac = (const void *)ft_jac_sweep, *cost = (const void *)ft_cost_sweep;
+        auto jsm = [&](int g) { return ft_ijac_smem(mmax, ninternal, ch.a.Wmax, g); };
+        auto csm = [&](int g) { return ft_icost_smem(xmaxins, xslots, xtape, a.v, g); };
+        const int gj = groups(jac, jsm), gc = groups(cost, csm);
+        ch.sw[ch.nk++] = sweep_shape(c, jac, gj * FT_ITHREADS, jsm(gj), items);
+        ch.sw[ch.nk++] = sweep_shape(c, cost, gc * FT_ITHREADS, csm(gc), items);
         return ch;
     }
-    const int T = small ? 128 : ft_cls_threads(cls);
-    const size_t sa = ft_sweep4_smem(FOP_ASM32, maxins, slots, region, T);
-    const size_t sl = ft_sweep4_smem(FOP_LOSS32, maxins, slots, region, 128);
-    if (extra) {
-        if (small) {
-            ch.sw[ch.nk++] = sweep_shape(c, (const void *)ft_sweep4<128, FOP_CASM, FOP_CSCORE>, 128,
-                                         std::max(sa, sl), items);
-        } else {
-            ch.sw[ch.nk++] = sweep_shape(c, casm_kernel(T), T, sa, items);
-            ch.sw[ch.nk++] = sweep_shape(c, (const void *)ft_sweep4<128, FOP_CSCORE>, 128, sl, items);
-        }
-    } else if (small) {
-        ch.sw[ch.nk++] = sweep_shape(
-            c, (const void *)ft_sweep4<128, FOP_ASM64, FOP_ASM32, FOP_LOSS64, FOP_LOSS32>, 128,
-            std::max(sa, sl), items);
+    auto kernels = [&](auto grp) {
+        constexpr bool GR = decltype(grp)::value;
+        struct {
+            const void *asm_fn, *loss_fn;
+        } k;
+        k.asm_fn = extra ? (const void *)ft_sweep4<GR, FOP_CASM>
+                         : (const void *)ft_sweep4<GR, FOP_ASM64, FOP_ASM32>;
+        k.loss_fn = extra ? (const void *)ft_sweep4<false, FOP_CSCORE>
+                          : (const void *)ft_sweep4<GR, FOP_LOSS64, FOP_LOSS32>;
+        return k;
+    };
+    const void *all_fn = extra
+                             ? (const void *)ft_sweep4<true, FOP_CASM, FOP_CSCORE>
+                             : (const void *)ft_sweep4<true, FOP_ASM64, FOP_ASM32, FOP_LOSS64, FOP_LOSS32>;
+    auto fns = kernels(std::false_type{});
+    int T = ft_cls_threads(cls);
+    size_t sa = ft_sweep4_smem(FOP_ASM32, maxins, slots, region, T);
+    bool grouped = small;
+    if (!small) {
+        rc_raise_smem(fns.asm_fn, sa);
+        grouped = items < (long long)(T == 128 ? 1 : FT_GROUP_WAVES) * c->sm_count *
+                              occupancy(fns.asm_fn, T, sa);
+    }
+    int TL = FT_LOSS_T;
+    if (grouped) {
+        /* several chunks of a tile at once (a tile's latency bounds these
+           fits): blocks of 512 threads with the regions that fit */
+        const auto gf = kernels(std::true_type{});
+        fns.asm_fn = gf.asm_fn;
+        fns.loss_fn = gf.loss_fn;
+        T = FT_GROUP_T;
+        size_t want = 0;
+        for (int i : ids)
+            if (b.valid[i]) {
+                const int4 f = b.finfo[i];
+                const int A = f.z & 0xffff;
+                want = std::max(want, (size_t)(T / A) *
+                                          (ft_asm_region(A, f.w & 0xffff, f.w >> 16,
+                                                         8 * ((b.pcount[i] + 1 + extra + 7) / 8)) +
+                                           16 * (size_t)A));
+            }
+        const size_t fixed = ft_sweep4_smem(FOP_ASM32, maxins, slots, 0, T);
+        ch.a.asm_region = std::max(region + 16 * 128, std::min(want, FT_SMEM_MAX - fixed));
+        sa = fixed + ch.a.asm_region;
+        TL = extra ? FT_LOSS_T : FT_GROUP_T;
+    }
+    const size_t sl = ft_sweep4_smem(FOP_LOSS32, maxins, slots, region, small ? T : TL);
+    if (small) {
+        ch.sw[ch.nk++] = sweep_shape(c, all_fn, T, std::max(sa, sl), items);
     } else {
-        ch.sw[ch.nk++] = sweep_shape(c, asm_kernel<FOP_ASM64, FOP_ASM32>(T), T, sa, items);
-        ch.sw[ch.nk++] = sweep_shape(c, (const void *)ft_sweep4<128, FOP_LOSS64, FOP_LOSS32>, 128, sl,
-                                     items);
+        ch.sw[ch.nk++] = sweep_shape(c, fns.asm_fn, T, sa, items);
+        ch.sw[ch.nk++] = sweep_shape(c, fns.loss_fn, TL, sl, items);
     }
     return ch;
 }

@@ -174,6 +174,22 @@ __device__ __forceinline__ double ft_block_sum(double v, double *red)
     return total;
 }
 
+/* Sum over the block's first n threads (n a power of two; the others' values
+   are not read): the tree of ft_block_sum<n>. Every thread gets it. */
+__device__ __forceinline__ double ft_sum_first(double v, double *red, int n)
+{
+    const int tid = threadIdx.x;
+    if (tid < n) red[tid] = v;
+    __syncthreads();
+    for (int st = n / 2; st > 0; st >>= 1) {
+        if (tid < st) red[tid] += red[tid + st];
+        __syncthreads();
+    }
+    const double total = red[0];
+    __syncthreads();
+    return total;
+}
+
 /* SYRK block assignment: the (W/4)x(W/4) block lower triangle of the
    augmented Gram [J | r]^T [J | r] is split into nblk 4x4 blocks; thread t
    owns block t % nblk and rows r == t / nblk (mod RG). */
