@@ -115,8 +115,10 @@ __device__ __forceinline__ void rs_count_keys(const u64 *src, long long r0, long
    not finite or exceeds 1e30 (eval.cu:4388-4418). A non-finite key marks
    the segment's status 2. The block then counts the eight digits of the
    keys it wrote (still in L2) into count[local segment][pass][256], which
-   the caller zeroed, so the sort needs no counting read of its own (with
-   count NULL it counts nothing). */
+   the caller zeroed, so the sort needs no counting read of its own. With
+   count NULL it counts nothing, and a segment known to have failed (its
+   keys are not read) is left: blocks take the segments of one tile after
+   another, so a failure is known early. */
 static_assert(RK_T == RS_T, "the digit count runs on the key kernel's blocks");
 template <int MODE>
 __global__ void __launch_bounds__(RK_T) rk_keys(const FOp *fins, const int *fins_off,
@@ -133,11 +135,18 @@ __global__ void __launch_bounds__(RK_T) rk_keys(const FOp *fins, const int *fins
     FOp *ins = reinterpret_cast<FOp *>(sm);
     double *cv = reinterpret_cast<double *>(sm + 8 * (size_t)((maxins + 1) & ~1));
     V4 *stk = reinterpret_cast<V4 *>(cv + FT_MAX_CONST);
-    const int ls = blockIdx.x / tiles;
+    const int nseg = (int)(gridDim.x / (unsigned)tiles);
+    const int ls = blockIdx.x % nseg;
     const int seg = seg0 + ls;
-    const int tile = blockIdx.x % tiles;
+    const int tile = blockIdx.x / nseg;
     const int cand = seg / ntrials;
     const int tid = threadIdx.x;
+    __shared__ int s_failed;
+    if (!count) {
+        if (tid == 0) s_failed = *(volatile const int *)(status + seg);
+        __syncthreads();
+        if (s_failed) return;
+    }
     const bool ok = valid[cand] != 0;
     const int nf = finfo[cand].x;
 #pragma unroll
@@ -151,7 +160,7 @@ __global__ void __launch_bounds__(RK_T) rk_keys(const FOp *fins, const int *fins
     u64 *kseg = keys + (size_t)ls * n;
     unsigned int *rseg = rows ? rows + (size_t)ls * n : nullptr;
     bool bad = !ok;
-    for (int row = r0 + 2 * tid; row < r1; row += 2 * RK_T) {
+    for (int row = r0 + 2 * tid; row < r1 && (count || !bad); row += 2 * RK_T) {
         double pr[2] = {CUDART_NAN, CUDART_NAN};
         if (ok)
             fi_forward<double, 2, false>(ins, cv, cols + row, npad, stk + tid, nullptr, RK_T, pr);
@@ -729,10 +738,12 @@ __device__ __forceinline__ unsigned rb_hash(unsigned a, unsigned b)
 /* Keys of S sample rows per segment: S / 2 row pairs, pair p at rows 2q and
    2q + 1 with q drawn by a fixed hash from the p-th of S / 2 equal strata of
    the n / 2 pairs; the f64 sweep and the keys of rk_keys. */
+template <int MODE>
 __global__ void __launch_bounds__(RK_T) rb_sample(const FOp *fins, const int *fins_off,
                                                   const int4 *finfo, const int *valid,
                                                   const double *c0, int kmax, const double *cols,
-                                                  int npad, int n, int ntrials, int seg0,
+                                                  const double *y, int npad, int n, int ntrials,
+                                                  int seg0,
                                                   int sblocks, int S, int maxins, u64 *samp)
 {
     using V4 = FiV<double, 2>::V4;
@@ -759,8 +770,16 @@ __global__ void __launch_bounds__(RK_T) rb_sample(const FOp *fins, const int *fi
     if (ok)
         fi_forward<double, 2, false>(ins, cv, cols + 2 * q, npad, stk + tid, nullptr, RK_T, pr);
 #pragma unroll
-    for (int i = 0; i < 2; ++i)
-        samp[(size_t)ls * RB_MAXS + 2 * p + i] = isfinite(pr[i]) ? rk_key(pr[i]) : ~0ULL;
+    for (int i = 0; i < 2; ++i) {
+        u64 k = ~0ULL;
+        if (MODE == RK_RANK) {
+            if (isfinite(pr[i])) k = rk_key(pr[i]);
+        } else {
+            const double r = pr[i] - y[2 * q + i];
+            if (isfinite(r)) k = rk_abs_key(r);
+        }
+        samp[(size_t)ls * RB_MAXS + 2 * p + i] = k;
+    }
 }
 
 /* One block per segment: the S samples sorted (bitonic, padded to P2 with the
@@ -816,12 +835,14 @@ __global__ void __launch_bounds__(RB_CTT, 3) rb_scatter(const u64 *keys, int n, 
                                                    int cap, const long long *B, const u64 *spl,
                                                    const int *nspl, unsigned *rcur,
                                                    unsigned *ecnt, unsigned long long *esum,
-                                                   u64 *bkey, int *bval, int *ovf)
+                                                   u64 *bkey, int *bval, int *ovf,
+                                                   const int *status)
 {
     __shared__ u64 sspl[RB_MAXB];
     __shared__ unsigned hist[2 * RB_MAXB];
     __shared__ unsigned long long ssum[RB_MAXB];
     const int ls = blockIdx.x / ctiles, tile = blockIdx.x % ctiles, tid = threadIdx.x;
+    if (status[ls]) return; /* its keys were not all made */
     const int ns = nspl[ls], nb = 2 * ns + 1;
     for (int i = tid; i < ns; i += RB_CTT) {
         sspl[i] = spl[(size_t)ls * RB_MAXB + i];
@@ -905,10 +926,11 @@ __global__ void __launch_bounds__(RB_CTT, 3) rb_scatter(const u64 *keys, int n, 
 __global__ void __launch_bounds__(RB_ST) rb_scan(int n, int cap, const int *nspl,
                                                  const unsigned *rcur, const unsigned *ecnt,
                                                  const unsigned long long *esum, unsigned *boff,
-                                                 __int128 *part, int *ovf)
+                                                 __int128 *part, int *ovf, const int *status)
 {
     __shared__ unsigned wsum[RB_ST / 32];
     const int ls = blockIdx.x, tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    if (status[ls]) return;
     const int nb = 2 * nspl[ls] + 1;
     unsigned sz[4], tot = 0;
     bool bad = false;
@@ -989,7 +1011,8 @@ static_assert(RB_DIG == 2 * RB_LT, "two digit groups per thread");
 __global__ void __launch_bounds__(RB_LT, 2) rb_local(int n, int m, int cap, int gmax,
                                                      const int *nspl, const unsigned *rcur,
                                                      const unsigned *boff, const u64 *bkey,
-                                                     const int *bval, __int128 *part, int *ovf)
+                                                     const int *bval, __int128 *part, int *ovf,
+                                                     const int *status)
 {
     extern __shared__ __align__(16) unsigned char sm[];
     u64 *sk = reinterpret_cast<u64 *>(sm);
@@ -1005,7 +1028,7 @@ __global__ void __launch_bounds__(RB_LT, 2) rb_local(int n, int m, int cap, int 
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     /* other blocks of the segment may raise its flag meanwhile: one read,
        shared, so the whole block takes the same branch */
-    if (tid == 0) s_skip = *(volatile const int *)(ovf + ls) || idx > nspl[ls];
+    if (tid == 0) s_skip = *(volatile const int *)(ovf + ls) || idx > nspl[ls] || status[ls];
     for (int d = tid; d < RB_DIG; d += RB_LT) {
         cur[d] = 0u;
         mixed[d] = 0;
@@ -1162,12 +1185,17 @@ __global__ void __launch_bounds__(RB_LT, 2) rb_local(int n, int m, int cap, int 
 }
 
 /* One block per segment not flagged: the bucket partials summed into the
-   two 128-bit sums, written as rk_final writes them. */
+   two 128-bit sums, written as rk_final writes them (zeros for a failed
+   segment). */
 __global__ void __launch_bounds__(RS_T) rb_final(const int *nspl, const __int128 *part,
-                                                 const int *ovf, u64 *out)
+                                                 const int *ovf, const int *status, u64 *out)
 {
     __shared__ __int128 red[RS_T];
     const int ls = blockIdx.x, tid = threadIdx.x;
+    if (status[ls]) {
+        if (tid < 4) out[(size_t)ls * 4 + tid] = 0ULL;
+        return;
+    }
     if (ovf[ls]) return;
     const int nb = 2 * nspl[ls] + 1;
     __int128 ab = 0, aa = 0;
@@ -1225,6 +1253,255 @@ __global__ void __launch_bounds__(OS_T) os_pick(const u64 *ka, const u64 *kb,
         __syncthreads();
     }
     if (tid == 0) out[seg] = part[0] / (double)(hi - lo);
+}
+
+/* Median by selection. A median needs one or two order statistics, not the
+ * sorted segment: a bracket [lo, hi] around the middle of a sorted sample of
+ * OS_S keys (OS_D sample ranks to either side, six standard deviations of the
+ * middle's sample rank for independent rows), one pass that makes every key,
+ * counts those below lo and lists those inside (about 9 % of them), and a
+ * radix selection inside the list on one block. Up to OS_LIST_ALL rows the
+ * bracket is everything. A middle outside the bracket (rows that the sample
+ * did not stand for) sends the segment to the sort, so the value is exact
+ * either way. The pass writes 0.75 B a key where keys and their sort moved
+ * 8 B and eight times 16. */
+#define OS_S 4096
+#define OS_D 192
+#define OS_LIST_ALL 32768
+#define OS_SEL_T 1024
+#define OS_BINS 2048
+#define OS_SMALL 1024 /* candidates ranked by comparison */
+
+/* The bracket of each segment from its sample; `all`: no sample, everything. */
+__global__ void __launch_bounds__(OS_SEL_T) os_bracket(const u64 *samp, int all, u64 *bracket)
+{
+    __shared__ u64 s[OS_S];
+    const int ls = blockIdx.x, tid = threadIdx.x;
+    if (all) {
+        if (tid < 2) bracket[2 * ls + tid] = tid == 0 ? 0ULL : ~0ULL;
+        return;
+    }
+    for (int i = tid; i < OS_S; i += OS_SEL_T) s[i] = samp[(size_t)ls * RB_MAXS + i];
+    __syncthreads();
+    for (int k = 2; k <= OS_S; k <<= 1)
+        for (int j = k >> 1; j > 0; j >>= 1) {
+            for (int i = tid; i < OS_S; i += OS_SEL_T) {
+                const int l = i ^ j;
+                if (l > i) {
+                    const u64 a = s[i], b = s[l];
+                    if ((a > b) == ((i & k) == 0)) {
+                        s[i] = b;
+                        s[l] = a;
+                    }
+                }
+            }
+            __syncthreads();
+        }
+    if (tid < 2) bracket[2 * ls + tid] = s[OS_S / 2 + (tid == 0 ? -OS_D : OS_D)];
+}
+
+/* The key pass of the selection (the keys and failures of rk_keys<RK_ABS>):
+   below[segment] += keys under the bracket, the keys inside appended to
+   list[segment][...] (cnt of them, in any order). */
+__global__ void __launch_bounds__(RK_T) os_keys(const FOp *fins, const int *fins_off,
+                                                const int4 *finfo, const int *valid,
+                                                const double *c0, int kmax, const double *cols,
+                                                const double *y, int npad, int n, int ntrials,
+                                                int seg0, int tiles, int maxins,
+                                                const u64 *bracket, u64 *list, unsigned *cnt,
+                                                unsigned *below, int *status)
+{
+    using V4 = FiV<double, 2>::V4;
+    extern __shared__ __align__(16) unsigned char sm[];
+    FOp *ins = reinterpret_cast<FOp *>(sm);
+    double *cv = reinterpret_cast<double *>(sm + 8 * (size_t)((maxins + 1) & ~1));
+    V4 *stk = reinterpret_cast<V4 *>(cv + FT_MAX_CONST);
+    __shared__ int s_failed;
+    const int nseg = (int)(gridDim.x / (unsigned)tiles);
+    const int ls = blockIdx.x % nseg, tile = blockIdx.x / nseg;
+    const int seg = seg0 + ls, cand = seg / ntrials;
+    const int tid = threadIdx.x, lane = tid & 31;
+    if (tid == 0) s_failed = *(volatile const int *)(status + seg) || !valid[cand];
+    __syncthreads();
+    if (s_failed) {
+        if (tid == 0) status[seg] = 2;
+        return;
+    }
+    const int nf = finfo[cand].x;
+    for (int i = tid; i < nf; i += RK_T) ins[i] = fins[fins_off[cand] + i];
+    if (tid < FT_MAX_CONST) cv[tid] = tid < kmax ? c0[(size_t)seg * kmax + tid] : 0.0;
+    __syncthreads();
+    const u64 lo = bracket[2 * ls], hi = bracket[2 * ls + 1];
+    u64 *out = list + (size_t)ls * n;
+    const int r0 = tile * RK_TILE, r1 = min(n, r0 + RK_TILE);
+    unsigned under = 0;
+    bool bad = false;
+    /* every lane takes every step: rows past r1 (below n rounded up to a
+       block's rows, which the columns hold) count for nothing */
+    for (int base = r0; base < r1; base += 2 * RK_T) {
+        const int row = base + 2 * tid;
+        double pr[2];
+        fi_forward<double, 2, false>(ins, cv, cols + row, npad, stk + tid, nullptr, RK_T, pr);
+        u64 k[2];
+        bool in[2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const int rr = row + i;
+            in[i] = false;
+            k[i] = 0;
+            if (rr >= r1) continue;
+            const double r = pr[i] - y[rr];
+            if (!isfinite(pr[i]) || fabs(pr[i]) > 1e30 || !isfinite(r)) {
+                bad = true;
+                continue;
+            }
+            k[i] = rk_abs_key(r);
+            under += k[i] < lo;
+            in[i] = k[i] >= lo && k[i] <= hi;
+        }
+        const unsigned m0 = __ballot_sync(0xffffffffu, in[0]), m1 = __ballot_sync(0xffffffffu, in[1]);
+        if (m0 | m1) {
+            unsigned at = 0;
+            if (lane == 0) at = atomicAdd(&cnt[ls], (unsigned)(__popc(m0) + __popc(m1)));
+            at = __shfl_sync(0xffffffffu, at, 0);
+            const unsigned lt = (1u << lane) - 1u;
+            if (in[0]) out[at + __popc(m0 & lt)] = k[0];
+            if (in[1]) out[at + __popc(m0) + __popc(m1 & lt)] = k[1];
+        }
+        if (__any_sync(0xffffffffu, bad)) break; /* the segment's answer is its status */
+    }
+    if (__syncthreads_or(bad)) {
+        if (tid == 0) status[seg] = 2;
+        return;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) under += __shfl_xor_sync(0xffffffffu, under, o);
+    if (lane == 0 && under) atomicAdd(&below[ls], under);
+}
+
+/* The rank-th smallest (from 0) of keys[0, m), all in [lo, hi]; every thread
+   of the block gets it. */
+__device__ u64 os_select(const u64 *keys, unsigned m, unsigned rank, u64 lo, u64 hi, unsigned *bins,
+                         u64 *small, unsigned *sh)
+{
+    const int tid = threadIdx.x;
+    u64 base = lo, width = hi - lo; /* the rank is among keys in [base, base + width] */
+    for (;;) {
+        if (width == 0) return base;
+        const int bits = 64 - __clzll((long long)width);
+        const int shift = bits > 11 ? bits - 11 : 0;
+        for (int b = tid; b < OS_BINS; b += OS_SEL_T) bins[b] = 0u;
+        __syncthreads();
+        for (unsigned q = tid; q < m; q += OS_SEL_T) {
+            const u64 k = keys[q];
+            if (k >= base && k - base <= width) atomicAdd(&bins[(unsigned)((k - base) >> shift)], 1u);
+        }
+        __syncthreads();
+        /* two bins a thread: the bin that holds the rank */
+        const unsigned a0 = bins[2 * tid], a1 = bins[2 * tid + 1];
+        unsigned x = a0 + a1;
+        const int lane = tid & 31, w = tid >> 5;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned v = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += v;
+        }
+        if (lane == 31) sh[w] = x;
+        __syncthreads();
+        unsigned before = x - a0 - a1;
+        for (int k = 0; k < w; ++k) before += sh[k];
+        if (rank >= before && rank < before + a0 + a1) {
+            const bool second = rank >= before + a0;
+            sh[32] = 2 * tid + (second ? 1 : 0);
+            sh[33] = second ? before + a0 : before;
+            sh[34] = second ? a1 : a0;
+        }
+        if (tid == 0) sh[35] = 0;
+        __syncthreads();
+        const unsigned bin = sh[32], first = sh[33], in_bin = sh[34];
+        rank -= first;
+        base += (u64)bin << shift;
+        const u64 span = shift ? ((1ULL << shift) - 1ULL) : 0ULL;
+        width = hi - base < span ? hi - base : span;
+        if (width == 0) return base;
+        if (in_bin <= OS_SMALL) {
+            for (unsigned q = tid; q < m; q += OS_SEL_T) {
+                const u64 k = keys[q];
+                if (k >= base && k - base <= width) small[atomicAdd(&sh[35], 1u)] = k;
+            }
+            __syncthreads();
+            if (tid < in_bin) {
+                const u64 k = small[tid];
+                unsigned lt = 0, le = 0;
+                for (unsigned q = 0; q < in_bin; ++q) {
+                    lt += small[q] < k;
+                    le += small[q] <= k;
+                }
+                /* (equal keys write the same answer) */
+                if (lt <= rank && rank < le) small[OS_SMALL] = k;
+            }
+            __syncthreads();
+            const u64 r = small[OS_SMALL];
+            __syncthreads();
+            return r;
+        }
+        __syncthreads();
+    }
+}
+
+/* One block per segment: the median from the listed keys, or a flag for the
+   sort when the middle is not among them. */
+__global__ void __launch_bounds__(OS_SEL_T) os_median(const u64 *list, const unsigned *cnt,
+                                                      const unsigned *below, int n, int seg0,
+                                                      const int *status, double *out, int *redo)
+{
+    __shared__ unsigned bins[OS_BINS];
+    __shared__ u64 small[OS_SMALL + 1];
+    __shared__ unsigned sh[36];
+    const int ls = blockIdx.x, seg = seg0 + ls, tid = threadIdx.x;
+    if (status[seg] != 0) {
+        if (tid == 0) out[seg] = CUDART_NAN;
+        return;
+    }
+    const unsigned m = cnt[ls], u = below[ls];
+    const unsigned kh = (unsigned)n / 2, kl = (n & 1) ? kh : kh - 1;
+    if (kl < u || kh >= u + m) {
+        if (tid == 0) redo[seg] = 1;
+        return;
+    }
+    const u64 *keys = list + (size_t)ls * n;
+    /* the listed keys' own range, so that the first digit spreads them */
+    u64 lo = ~0ULL, hi = 0ULL;
+    for (unsigned q = tid; q < m; q += OS_SEL_T) {
+        const u64 k = keys[q];
+        lo = k < lo ? k : lo;
+        hi = k > hi ? k : hi;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const u64 x = __shfl_xor_sync(0xffffffffu, lo, o), y = __shfl_xor_sync(0xffffffffu, hi, o);
+        lo = x < lo ? x : lo;
+        hi = y > hi ? y : hi;
+    }
+    if ((tid & 31) == 0) {
+        small[tid >> 5] = lo;
+        small[32 + (tid >> 5)] = hi;
+    }
+    __syncthreads();
+    for (int w = 0; w < OS_SEL_T / 32; ++w) {
+        lo = small[w] < lo ? small[w] : lo;
+        hi = small[32 + w] > hi ? small[32 + w] : hi;
+    }
+    __syncthreads();
+    const u64 a = os_select(keys, m, kl - u, lo, hi, bins, small, sh);
+    u64 b = a;
+    if (kh != kl) {
+        __syncthreads();
+        b = os_select(keys, m, kh - u, lo, hi, bins, small, sh);
+    }
+    if (tid == 0)
+        out[seg] = (n & 1) ? rk_key_abs_value(a)
+                           : 0.5 * (rk_key_abs_value(a) + rk_key_abs_value(b));
 }
 
 /* ---- maximum-error scan ------------------------------------------------- */
@@ -1575,7 +1852,7 @@ float rc_rank_score_batch(void *ctx, const unsigned int *prog, const unsigned in
     cudaMemsetAsync(d_abort, 0, sizeof(int), c->s);
     const size_t smem = key_smem(sp);
     if (rc_raise_smem((const void *)rk_keys<RK_RANK>, smem) != 0) return -1.0f;
-    if (m > 0 && (rc_raise_smem((const void *)rb_sample, smem) != 0 ||
+    if (m > 0 && (rc_raise_smem((const void *)rb_sample<RK_RANK>, smem) != 0 ||
                   rc_raise_smem((const void *)rb_splitters, sizeof(u64) * RB_MAXS) != 0 ||
                   rc_raise_smem((const void *)rb_local, rb_local_smem()) != 0))
         return -1.0f;
@@ -1611,8 +1888,8 @@ float rc_rank_score_batch(void *ctx, const unsigned int *prog, const unsigned in
             int P2 = 1;
             while (P2 < S) P2 <<= 1;
             const int sblocks = (S / 2 + RK_T - 1) / RK_T;
-            rb_sample<<<(unsigned)ns * sblocks, RK_T, smem, c->s>>>(
-                d_fins, d_finsoff, d_finfo, d_valid, d_c0, kmax, c->d_cols64, c->npad, n, ntrials,
+            rb_sample<RK_RANK><<<(unsigned)ns * sblocks, RK_T, smem, c->s>>>(
+                d_fins, d_finsoff, d_finfo, d_valid, d_c0, kmax, c->d_cols64, c->d_y64, c->npad, n, ntrials,
                 s0, sblocks, S, sp.b.fmaxins, r.samp);
             rb_splitters<<<ns, RB_ST, sizeof(u64) * P2, c->s>>>(r.samp, S, P2, m, r.spl, r.nspl);
             c->launches += 2;
@@ -1625,12 +1902,14 @@ float rc_rank_score_batch(void *ctx, const unsigned int *prog, const unsigned in
         const int ctiles = (n + RB_CT - 1) / RB_CT;
         rb_scatter<<<(unsigned)ns * ctiles, RB_CTT, 0, c->s>>>(
             r.keys, n, ctiles, m, cap, c->d_rank_b, r.spl, r.nspl, r.rcur, r.ecnt, r.esum, r.bkey,
-            r.bval, d_ovf + s0);
+            r.bval, d_ovf + s0, d_status + s0);
         rb_scan<<<ns, RB_ST, 0, c->s>>>(n, cap, r.nspl, r.rcur, r.ecnt, r.esum, r.boff, r.part,
-                                        d_ovf + s0);
+                                        d_ovf + s0, d_status + s0);
         rb_local<<<(unsigned)ns * m, RB_LT, rb_local_smem(), c->s>>>(
-            n, m, cap, gmax, r.nspl, r.rcur, r.boff, r.bkey, r.bval, r.part, d_ovf + s0);
-        rb_final<<<ns, RS_T, 0, c->s>>>(r.nspl, r.part, d_ovf + s0, d_out + 4 * (size_t)s0);
+            n, m, cap, gmax, r.nspl, r.rcur, r.boff, r.bkey, r.bval, r.part, d_ovf + s0,
+            d_status + s0);
+        rb_final<<<ns, RS_T, 0, c->s>>>(r.nspl, r.part, d_ovf + s0, d_status + s0,
+                                        d_out + 4 * (size_t)s0);
         c->launches += 5;
     };
     cudaEventRecord(c->t0, c->s);
@@ -1717,45 +1996,93 @@ float rc_order_stat_score_batch(void *ctx, const unsigned int *prog, const unsig
     stat_inputs(c, prog, off, pcount, nsets, nsegs, kmax, c0, &cur, sp);
     const size_t o_val = rc_take(&cur, sizeof(double) * (size_t)nsegs);
     const size_t o_status = rc_take(&cur, sizeof(int) * (size_t)nsegs);
+    const size_t o_redo = rc_take(&cur, sizeof(int) * (size_t)nsegs);
     const size_t o_abort = rc_take(&cur, sizeof(int));
     const size_t io_end = rc_take(&cur, 0);
-    const int wseg = wave_segments(nsegs, n, false);
+    /* a median by selection (a wave's key lists in RK_WAVE_BYTES, a segment
+       it cannot settle sorted alone), the interquartile mean by sorting */
     const size_t work = cur;
-    if (rc_reserve(c, work + rs_bytes((size_t)wseg * n, wseg, n, false) + 4096, io_end) != 0)
-        return -1.0f;
+    const size_t sel_per = sizeof(u64) * ((size_t)n + RB_MAXS + 2) + 2 * sizeof(unsigned);
+    const int wseg = what == 0
+                         ? (int)std::min<size_t>(std::max<size_t>(RK_WAVE_BYTES / sel_per, 1), nsegs)
+                         : wave_segments(nsegs, n, false);
+    const size_t wbytes = what == 0 ? std::max(sel_per * wseg + 8 * 256, rs_bytes((size_t)n, 1, n, false))
+                                    : rs_bytes((size_t)wseg * n, wseg, n, false);
+    if (rc_reserve(c, work + wbytes + 4096, io_end) != 0) return -1.0f;
     stat_copy(c, pcount, nsets, nsegs, kmax, c0, sp);
     unsigned char *dev = c->dev;
     int *d_status = reinterpret_cast<int *>(dev + o_status);
+    int *d_redo = reinterpret_cast<int *>(dev + o_redo);
     int *d_abort = reinterpret_cast<int *>(dev + o_abort);
-    cudaMemsetAsync(d_status, 0, sizeof(int) * nsegs, c->s);
-    cudaMemsetAsync(d_abort, 0, sizeof(int), c->s);
+    double *d_val = reinterpret_cast<double *>(dev + o_val);
+    cudaMemsetAsync(d_status, 0, io_end - o_status, c->s);
     const size_t smem = key_smem(sp);
-    if (rc_raise_smem((const void *)rk_keys<RK_ABS>, smem) != 0) return -1.0f;
+    if (rc_raise_smem((const void *)rk_keys<RK_ABS>, smem) != 0 ||
+        rc_raise_smem((const void *)rb_sample<RK_ABS>, smem) != 0 ||
+        rc_raise_smem((const void *)os_keys, smem) != 0)
+        return -1.0f;
     const int ktiles = (n + RK_TILE - 1) / RK_TILE;
-    cudaEventRecord(c->t0, c->s);
-    for (int s0 = 0; s0 < nsegs; s0 += wseg) {
-        const int ns = std::min(wseg, nsegs - s0);
+    const FOp *d_fins = reinterpret_cast<const FOp *>(dev + sp.o_fins);
+    const int *d_finsoff = reinterpret_cast<const int *>(dev + sp.o_finsoff);
+    const int4 *d_finfo = reinterpret_cast<const int4 *>(dev + sp.o_finfo);
+    const int *d_valid = reinterpret_cast<const int *>(dev + sp.o_valid);
+    const double *d_c0 = reinterpret_cast<const double *>(dev + sp.o_c0);
+    auto sort_wave = [&](int s0, int ns) {
         size_t wc = work;
         __int128 *part = nullptr;
         const RsBuffers b = rs_carve(dev, &wc, ns, n, false, &part);
         cudaMemsetAsync(b.count, 0, sizeof(unsigned int) * RS_PASSES * 256 * (size_t)ns, c->s);
         rk_keys<RK_ABS><<<(unsigned)ns * ktiles, RK_T, smem, c->s>>>(
-            reinterpret_cast<const FOp *>(dev + sp.o_fins),
-            reinterpret_cast<const int *>(dev + sp.o_finsoff),
-            reinterpret_cast<const int4 *>(dev + sp.o_finfo),
-            reinterpret_cast<const int *>(dev + sp.o_valid),
-            reinterpret_cast<const double *>(dev + sp.o_c0), kmax, c->d_cols64, c->d_y64, c->npad,
-            n, ntrials, s0, ktiles, sp.b.fmaxins, b.ka, nullptr, b.count, d_status);
+            d_fins, d_finsoff, d_finfo, d_valid, d_c0, kmax, c->d_cols64, c->d_y64, c->npad, n,
+            ntrials, s0, ktiles, sp.b.fmaxins, b.ka, nullptr, b.count, d_status);
         c->launches += 2 + rs_sort<false>(b, ns, n, d_abort, c->s, true);
-        os_pick<<<ns, OS_T, 0, c->s>>>(b.ka, b.kb, b.par, n, s0, ns, what, d_status,
-                                       reinterpret_cast<double *>(dev + o_val));
+        os_pick<<<ns, OS_T, 0, c->s>>>(b.ka, b.kb, b.par, n, s0, ns, what, d_status, d_val);
+    };
+    auto select_wave = [&](int s0, int ns) {
+        size_t wc = work;
+        u64 *list = reinterpret_cast<u64 *>(dev + rc_take(&wc, sizeof(u64) * (size_t)ns * n));
+        u64 *samp = reinterpret_cast<u64 *>(dev + rc_take(&wc, sizeof(u64) * (size_t)ns * RB_MAXS));
+        u64 *bracket = reinterpret_cast<u64 *>(dev + rc_take(&wc, sizeof(u64) * 2 * (size_t)ns));
+        unsigned *cnt = reinterpret_cast<unsigned *>(dev + rc_take(&wc, sizeof(unsigned) * 2 * (size_t)ns));
+        cudaMemsetAsync(cnt, 0, sizeof(unsigned) * 2 * (size_t)ns, c->s);
+        const int all = n <= OS_LIST_ALL ? 1 : 0;
+        if (!all) {
+            const int sblocks = (OS_S / 2 + RK_T - 1) / RK_T;
+            rb_sample<RK_ABS><<<(unsigned)ns * sblocks, RK_T, smem, c->s>>>(
+                d_fins, d_finsoff, d_finfo, d_valid, d_c0, kmax, c->d_cols64, c->d_y64, c->npad, n,
+                ntrials, s0, sblocks, OS_S, sp.b.fmaxins, samp);
+            c->launches += 1;
+        }
+        os_bracket<<<ns, OS_SEL_T, 0, c->s>>>(samp, all, bracket);
+        os_keys<<<(unsigned)ns * ktiles, RK_T, smem, c->s>>>(
+            d_fins, d_finsoff, d_finfo, d_valid, d_c0, kmax, c->d_cols64, c->d_y64, c->npad, n,
+            ntrials, s0, ktiles, sp.b.fmaxins, bracket, list, cnt, cnt + ns, d_status);
+        os_median<<<ns, OS_SEL_T, 0, c->s>>>(list, cnt, cnt + ns, n, s0, d_status, d_val, d_redo);
+        c->launches += 3;
+    };
+    auto fetch = [&]() {
+        cudaEventRecord(c->t1, c->s);
+        if (cudaGetLastError() != cudaSuccess) return -1;
+        cudaMemcpyAsync(c->host + sp.in_end, dev + sp.in_end, io_end - sp.in_end,
+                        cudaMemcpyDeviceToHost, c->s);
+        if (rc_finish(c) != 0) return -1;
+        return *reinterpret_cast<const int *>(c->host + o_abort) != 0 ? -1 : 0;
+    };
+    cudaEventRecord(c->t0, c->s);
+    for (int s0 = 0; s0 < nsegs; s0 += wseg) {
+        const int ns = std::min(wseg, nsegs - s0);
+        if (what == 0) select_wave(s0, ns);
+        else sort_wave(s0, ns);
     }
-    cudaEventRecord(c->t1, c->s);
-    if (cudaGetLastError() != cudaSuccess) return -1.0f;
-    cudaMemcpyAsync(c->host + sp.in_end, dev + sp.in_end, io_end - sp.in_end,
-                    cudaMemcpyDeviceToHost, c->s);
-    if (rc_finish(c) != 0) return -1.0f;
-    if (*reinterpret_cast<const int *>(c->host + o_abort) != 0) return -1.0f;
+    if (fetch() != 0) return -1.0f;
+    if (what == 0) {
+        const int *h_redo = reinterpret_cast<const int *>(c->host + o_redo);
+        std::vector<int> redo;
+        for (int s = 0; s < nsegs; ++s)
+            if (h_redo[s]) redo.push_back(s);
+        for (int s : redo) sort_wave(s, 1);
+        if (!redo.empty() && fetch() != 0) return -1.0f;
+    }
     memcpy(out_value, c->host + o_val, sizeof(double) * (size_t)nsegs);
     memcpy(out_status, c->host + o_status, sizeof(int) * (size_t)nsegs);
     float ms = -1.0f;
