@@ -34,7 +34,12 @@ enum RcInsKind {
     K_BIN_C = 5,      /* TOS = op(TOS, imm) */
     K_IF = 6,         /* TOS = slot[arg] > 0 ? slot[arg + 1] : TOS */
     K_HALT = 7,       /* result = TOS (depth 1) or slot[0] (depth > 1) */
-    K_NAN = 8         /* the whole program is a hard failure (NaN every row) */
+    K_NAN = 8,        /* the whole program is a hard failure (NaN every row) */
+    /* made from the kinds above for one batch (rc_fold_programs): */
+    K_PUSH_COL = 9,   /* spill TOS; TOS = op(input), read from the batch's column imm */
+    K_PUSH_FOLD = 10  /* spill TOS; TOS = a folded constant subtree: f32 bits of its value here
+                         and of its error bound in the next word's imm (f64 lane: the low
+                         and high halves of its f64 value) */
 };
 
 struct RcIns {
@@ -106,7 +111,20 @@ struct RcPinnedWords {
     ~RcPinnedWords() { release(); }
 };
 
+/* Host lists of a scoring call, kept by the context: they are mapped memory of
+   half a megabyte and more for a large batch, and fresh pages on every call
+   cost as much as decoding the batch. Sizes only grow. */
+struct RcScoreLists {
+    std::vector<RcIns> ins, ins32, ins64;
+    RcIns *grow(std::vector<RcIns> &v, size_t n)
+    {
+        if (v.size() < n) v.resize(n);
+        return v.data();
+    }
+};
+
 struct RcCtx {
+    RcScoreLists score_lists;
     int n;      /* rows */
     int v;      /* columns */
     int npad;   /* padded row stride of the device columns */

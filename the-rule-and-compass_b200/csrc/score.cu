@@ -146,6 +146,181 @@ int rc_decode_postfix(const uint32_t *words, size_t nwords, int v, RcIns *out, i
 
 namespace {
 
+/* Rows x programs from which a batch's constant subtrees and columns are
+   worth their two launches (about 30 us with the host's share; a batch of
+   that many row evaluations runs for 150 us and more). */
+const long long FOLD_MIN = 1LL << 24;
+/* Columns only while the inputs and they stay in L2 (126 MB). */
+const size_t FCOL_BYTES = (size_t)96 << 20;
+/* ... and only for as many uses in the batch. */
+const int FCOL_USES = 8;
+
+/* The f32 and f64 lists of a batch with constant subtrees folded and, in the
+   f32 list, sin / cos / exp of an input read from a column. */
+struct FoldedBatch {
+    const RcIns *ins32 = nullptr, *ins64 = nullptr; /* in the context's lists */
+    std::vector<RcIns> fold_ins;
+    std::vector<int> off32, off64;
+    std::vector<RcFold> folds;
+    std::vector<unsigned> spec; /* columns: input << 8 | operator */
+};
+
+bool column_op(const RcIns &push, const RcIns &un)
+{
+    return push.kind == K_PUSH_VAR && un.kind == K_UNARY &&
+           (un.op == OP_SIN || un.op == OP_COS || un.op == OP_EXP);
+}
+
+/* The maximal constant subtrees (of an operator or more) of one program, as
+   instruction ranges [first, last] in ascending order. A program that ends
+   with more than one entry is left alone (its result is the lowest). */
+void constant_ranges(const RcIns *ins, int n, std::vector<std::pair<int, int>> &out)
+{
+    struct Ent {
+        int first, last;
+        bool c;
+    };
+    Ent st[RC_MAX_STACK + 1];
+    int d = 0;
+    out.clear();
+    auto take = [&](const Ent &e) {
+        if (e.c && e.last > e.first) out.emplace_back(e.first, e.last);
+    };
+    if (n <= 0 || ins[n - 1].kind != K_HALT || ins[n - 1].arg != 1) return;
+    for (int i = 0; i < n; ++i) {
+        const RcIns &in = ins[i];
+        switch (in.kind) {
+            case K_PUSH_VAR: st[d++] = {i, i, false}; break;
+            case K_PUSH_CONST: st[d++] = {i, i, true}; break;
+            case K_UNARY: case K_BIN_C: st[d - 1].last = i; break;
+            case K_BIN_V:
+                take(st[d - 1]);
+                st[d - 1] = {st[d - 1].first, i, false};
+                break;
+            case K_BIN_S: case K_IF: {
+                const int k = in.kind == K_IF ? 3 : 2;
+                bool all = true;
+                for (int j = d - k; j < d; ++j) all = all && st[j].c;
+                if (!all)
+                    for (int j = d - k; j < d; ++j) take(st[j]);
+                d -= k - 1;
+                st[d - 1] = {st[d - 1].first, i, all};
+            } break;
+            case K_HALT: take(st[d - 1]); break;
+            default: out.clear(); return;
+        }
+    }
+    std::sort(out.begin(), out.end());
+}
+
+void fold_programs(RcScoreLists &lists, const RcIns *ins, const std::vector<int> &off, int nprog,
+                   int v, size_t col_bytes, FoldedBatch &f)
+{
+    /* the columns: the most used first, while they fit; three operators an
+       input, inputs past COL_VARS left alone */
+    const int COL_VARS = 256;
+    auto slot = [&](const RcIns &push, const RcIns &un) {
+        return (int)push.imm * 3 + (un.op == OP_SIN ? 0 : (un.op == OP_COS ? 1 : 2));
+    };
+    auto is_col = [&](const RcIns &push, const RcIns &un) {
+        return column_op(push, un) && push.imm < (unsigned)COL_VARS;
+    };
+    const unsigned opc[3] = {OP_SIN, OP_COS, OP_EXP};
+    std::vector<int> uses(3 * (size_t)std::min(v, COL_VARS), 0), col(uses.size(), -1);
+    /* one scan: the columns' uses, and the programs that hold something to
+       fold (the innermost operator of a constant subtree directly follows a
+       constant push) or a column's pair */
+    std::vector<unsigned char> has(nprog, 0);
+    for (int p = 0; p < nprog; ++p) {
+        unsigned char h = 0;
+        const RcIns *s = ins + off[p], *e = ins + off[p + 1] - 1;
+        for (; s < e; ++s) {
+            if (s->kind > K_PUSH_CONST) continue;
+            const unsigned nk = s[1].kind;
+            if (s->kind == K_PUSH_CONST) {
+                if (nk == K_UNARY || nk == K_BIN_C || nk == K_BIN_S || nk == K_IF) h |= 1;
+            } else if (nk == K_UNARY && is_col(s[0], s[1])) {
+                ++uses[slot(s[0], s[1])];
+                h |= 2;
+            }
+        }
+        has[p] = h;
+    }
+    std::vector<std::pair<int, int>> by;
+    for (size_t k = 0; k < uses.size(); ++k)
+        if (uses[k] >= FCOL_USES) by.emplace_back(-uses[k], (int)k);
+    std::sort(by.begin(), by.end());
+    for (const auto &b : by) {
+        if ((size_t)(v + 1 + f.spec.size() + 1) * col_bytes > FCOL_BYTES) break;
+        col[b.second] = (int)f.spec.size();
+        f.spec.push_back(((unsigned)(b.second / 3) << 8) | opc[b.second % 3]);
+    }
+    /* (neither list is ever longer than the program's own) */
+    RcIns *const b32 = lists.grow(lists.ins32, (size_t)off[nprog]);
+    RcIns *const b64 = lists.grow(lists.ins64, (size_t)off[nprog]);
+    f.ins32 = b32;
+    f.ins64 = b64;
+    f.off32.resize(nprog + 1);
+    f.off64.resize(nprog + 1);
+    RcIns *o32 = b32, *o64 = b64;
+    RcIns fold, halt;
+    memset(&fold, 0, sizeof(fold));
+    fold.kind = K_PUSH_FOLD;
+    halt = fold;
+    halt.kind = K_HALT;
+    halt.arg = 1;
+    std::vector<std::pair<int, int>> ranges;
+    for (int p = 0; p < nprog; ++p) {
+        const RcIns *src = ins + off[p];
+        const int n = off[p + 1] - off[p];
+        f.off32[p] = (int)(o32 - b32);
+        f.off64[p] = (int)(o64 - b64);
+        if (!has[p]) {
+            memcpy(o32, src, sizeof(RcIns) * n);
+            memcpy(o64, src, sizeof(RcIns) * n);
+            o32 += n;
+            o64 += n;
+            continue;
+        }
+        ranges.clear();
+        if (has[p] & 1) constant_ranges(src, n, ranges);
+        size_t r = 0;
+        for (int i = 0; i < n; ++i) {
+            if (r < ranges.size() && ranges[r].first == i) {
+                fold.spill = src[i].spill;
+                f.folds.push_back({(int)f.fold_ins.size(), (int)(o32 - b32), (int)(o64 - b64)});
+                for (int k = 0; k < 2; ++k) {
+                    *o32++ = fold;
+                    *o64++ = fold;
+                }
+                f.fold_ins.insert(f.fold_ins.end(), src + i, src + ranges[r].second + 1);
+                f.fold_ins.push_back(halt);
+                i = ranges[r].second;
+                ++r;
+                continue;
+            }
+            if (src[i].kind == K_PUSH_VAR && i + 1 < n && is_col(src[i], src[i + 1])) {
+                const int at = col[slot(src[i], src[i + 1])];
+                if (at >= 0) {
+                    *o32 = src[i];
+                    o32->kind = K_PUSH_COL;
+                    o32->op = src[i + 1].op;
+                    o32->imm = (unsigned)at;
+                    ++o32;
+                    *o64++ = src[i];
+                    *o64++ = src[i + 1];
+                    ++i;
+                    continue;
+                }
+            }
+            *o32++ = src[i];
+            *o64++ = src[i];
+        }
+    }
+    f.off32[nprog] = (int)(o32 - b32);
+    f.off64[nprog] = (int)(o64 - b64);
+}
+
 struct Bucket {
     std::vector<int> cands;
     int nslots = 0;
@@ -184,23 +359,39 @@ int rc_score_tile_rows(int n)
 }
 const int LANE_T = 128;
 
-const void *score_kernel_fn(int T, bool track)
+/* The scoring kernel of a launch: the 256-thread shape has the common modes
+   compiled in. */
+const void *score_kernel_fn(int T, bool track, int mode)
 {
-    if (T == 256) return track ? (const void *)rc_score_kernel<256, true>
-                               : (const void *)rc_score_kernel<256, false>;
-    return track ? (const void *)rc_score_kernel<64, true> : (const void *)rc_score_kernel<64, false>;
+    if (T != 256)
+        return track ? (const void *)rc_score_kernel<64, true, -1>
+                     : (const void *)rc_score_kernel<64, false, -1>;
+    if (!track) return (const void *)rc_score_kernel<256, false, -1>;
+    switch (mode) {
+        case SM_SQUARED: case SM_AIC: case SM_AICC: case SM_BIC: /* the same sums */
+            return (const void *)rc_score_kernel<256, true, SM_SQUARED>;
+        case SM_ABSOLUTE: return (const void *)rc_score_kernel<256, true, SM_ABSOLUTE>;
+        case SM_CORR_PASS1: return (const void *)rc_score_kernel<256, true, SM_CORR_PASS1>;
+        case SM_CORR_PASS2: return (const void *)rc_score_kernel<256, true, SM_CORR_PASS2>;
+        default: return (const void *)rc_score_kernel<256, true, -1>;
+    }
 }
 
-void launch_score_kernel(int T, bool track, int grid, size_t smem, cudaStream_t s,
+const void *lane_kernel_fn(int mode)
+{
+    switch (mode) {
+        case SM_SQUARED: case SM_AIC: case SM_AICC: case SM_BIC:
+            return (const void *)rc_score64_kernel<LANE_T, SM_SQUARED>;
+        case SM_ABSOLUTE: return (const void *)rc_score64_kernel<LANE_T, SM_ABSOLUTE>;
+        default: return (const void *)rc_score64_kernel<LANE_T, -1>;
+    }
+}
+
+void launch_score_kernel(const void *fn, int T, int grid, size_t smem, cudaStream_t s,
                          const ScoreArgs &a)
 {
-    if (T == 256) {
-        if (track) rc_score_kernel<256, true><<<grid, 256, smem, s>>>(a);
-        else rc_score_kernel<256, false><<<grid, 256, smem, s>>>(a);
-    } else {
-        if (track) rc_score_kernel<64, true><<<grid, 64, smem, s>>>(a);
-        else rc_score_kernel<64, false><<<grid, 64, smem, s>>>(a);
-    }
+    void *args[] = {(void *)&a};
+    cudaLaunchKernel(fn, dim3(grid), dim3(T), args, smem, s);
 }
 
 /* The kernel's dynamic shared-memory limit raised to at least `smem`
@@ -232,7 +423,8 @@ float rc_score_run(RcCtx *c, const uint32_t *words, const uint32_t *off, int wid
         const size_t e = width > 0 ? b + (size_t)width : off[p + 1];
         room += std::max<size_t>(e > b ? e - b : 0, 1);
     }
-    std::vector<RcIns> ins(room);
+    RcIns *const decoded = c->score_lists.grow(c->score_lists.ins, room);
+    const RcIns *ins = decoded;
     size_t pos = 0;
     for (int p = 0; p < nprog; ++p) {
         size_t b = width > 0 ? (size_t)p * (size_t)width : off[p];
@@ -244,13 +436,21 @@ float rc_score_run(RcCtx *c, const uint32_t *words, const uint32_t *off, int wid
             q += (words[q] == OP_CONST || words[q] == OP_VAR) ? 2 : 1;
         opw[p] = ops + 2;
         int ns = 0;
-        const int cnt = rc_decode_postfix(words + b, e - b, c->v, ins.data() + pos, &ns);
+        const int cnt = rc_decode_postfix(words + b, e - b, c->v, decoded + pos, &ns);
         ins_off[p] = (int)pos;
         pos += (size_t)cnt;
         nslots[p] = ns;
     }
-    ins.resize(pos);
     ins_off[nprog] = (int)pos;
+    /* constant subtrees and shared columns, for a batch large enough */
+    FoldedBatch fb;
+    if ((long long)nprog * c->n >= FOLD_MIN)
+        fold_programs(c->score_lists, ins, ins_off, nprog, c->v, sizeof(float) * (size_t)c->npad, fb);
+    const bool folded = !fb.folds.empty() || !fb.spec.empty();
+    if (folded) {
+        ins = fb.ins32;
+        ins_off.swap(fb.off32);
+    }
 
     /* 2. bucket by depth; longest program first */
     Bucket bk[2];
@@ -292,10 +492,16 @@ float rc_score_run(RcCtx *c, const uint32_t *words, const uint32_t *off, int wid
        [out | status | out_f32 | rows], work zeroed with rows by one memset
        [bad | bad64 | badrow | counters], work [part | pbar | lane]. */
     size_t cur = 0;
-    const size_t o_ins = rc_take(&cur, sizeof(RcIns) * ins.size());
+    const size_t o_ins = rc_take(&cur, sizeof(RcIns) * (size_t)ins_off[nprog]);
     const size_t o_insoff = rc_take(&cur, sizeof(int) * (nprog + 1));
     const size_t o_order = rc_take(&cur, sizeof(int) * nprog);
     const size_t o_opw = rc_take(&cur, sizeof(int) * nprog);
+    const size_t n64 = folded ? (size_t)fb.off64[nprog] : 0;
+    const size_t o_ins64 = rc_take(&cur, sizeof(RcIns) * n64);
+    const size_t o_off64 = rc_take(&cur, folded ? sizeof(int) * (nprog + 1) : 0);
+    const size_t o_fold = rc_take(&cur, sizeof(RcFold) * fb.folds.size());
+    const size_t o_foldins = rc_take(&cur, sizeof(RcIns) * fb.fold_ins.size());
+    const size_t o_spec = rc_take(&cur, sizeof(unsigned) * fb.spec.size());
     const size_t in_end = rc_take(&cur, 0);
     const size_t o_out = rc_take(&cur, sizeof(double) * nprog);
     const size_t o_status = rc_take(&cur, sizeof(int) * nprog);
@@ -313,6 +519,7 @@ float rc_score_run(RcCtx *c, const uint32_t *words, const uint32_t *off, int wid
     const size_t o_pbar64 = rc_take(&cur, sizeof(double) * nprog);
     const size_t o_flagged = rc_take(&cur, sizeof(int) * nprog);
     const size_t o_part64 = rc_take(&cur, track ? 2 * sizeof(double) * (size_t)nprog * ntiles : 0);
+    const size_t o_fcols = rc_take(&cur, sizeof(float) * (size_t)c->npad * fb.spec.size());
     const size_t o_pred = rc_take(&cur, pred_out ? sizeof(float) * (size_t)nprog * c->n : 0);
     const size_t dev_end = rc_take(&cur, 0);
     double t = rc_now_ms();
@@ -323,10 +530,20 @@ float rc_score_run(RcCtx *c, const uint32_t *words, const uint32_t *off, int wid
     st->alloc_ms += rc_now_ms() - t;
     unsigned char *dev = c->dev, *host = c->host;
     t = rc_now_ms();
-    memcpy(host + o_ins, ins.data(), sizeof(RcIns) * ins.size());
+    memcpy(host + o_ins, ins, sizeof(RcIns) * (size_t)ins_off[nprog]);
     memcpy(host + o_insoff, ins_off.data(), sizeof(int) * (nprog + 1));
     memcpy(host + o_order, order.data(), sizeof(int) * nprog);
     memcpy(host + o_opw, opw.data(), sizeof(int) * nprog);
+    if (folded) {
+        memcpy(host + o_ins64, fb.ins64, sizeof(RcIns) * n64);
+        memcpy(host + o_off64, fb.off64.data(), sizeof(int) * (nprog + 1));
+        if (!fb.folds.empty()) {
+            memcpy(host + o_fold, fb.folds.data(), sizeof(RcFold) * fb.folds.size());
+            memcpy(host + o_foldins, fb.fold_ins.data(), sizeof(RcIns) * fb.fold_ins.size());
+        }
+        if (!fb.spec.empty())
+            memcpy(host + o_spec, fb.spec.data(), sizeof(unsigned) * fb.spec.size());
+    }
     cudaMemcpyAsync(dev, host, in_end, cudaMemcpyHostToDevice, c->s);
     cudaMemsetAsync(dev + o_rows, 0, o_zero_end - o_rows, c->s);
     unsigned long long *d_rows = reinterpret_cast<unsigned long long *>(dev + o_rows);
@@ -347,6 +564,7 @@ float rc_score_run(RcCtx *c, const uint32_t *words, const uint32_t *off, int wid
     a.npad = c->npad;
     a.v = c->v;
     a.staged = staged;
+    a.fcols = reinterpret_cast<const float *>(dev + o_fcols);
     a.ins = reinterpret_cast<const RcIns *>(dev + o_ins);
     a.ins_off = reinterpret_cast<const int *>(dev + o_insoff);
     a.nprog = nprog;
@@ -365,6 +583,26 @@ float rc_score_run(RcCtx *c, const uint32_t *words, const uint32_t *off, int wid
     t = rc_now_ms();
     cudaEventRecord(c->t0, c->s);
     cudaEventRecord(c->sp[0], c->s);
+    if (!fb.folds.empty()) {
+        const int nf = (int)fb.folds.size();
+        const size_t fsmem = (size_t)max_slots * RC_FOLD_T * 24;
+        if (set_smem((const void *)rc_fold, fsmem) != 0) {
+            st->failed = 1;
+            cudaStreamSynchronize(c->s);
+            return -1.0f;
+        }
+        rc_fold<<<(nf + RC_FOLD_T - 1) / RC_FOLD_T, RC_FOLD_T, fsmem, c->s>>>(
+            nf, reinterpret_cast<const RcFold *>(dev + o_fold),
+            reinterpret_cast<const RcIns *>(dev + o_foldins), max_slots,
+            reinterpret_cast<RcIns *>(dev + o_ins), reinterpret_cast<RcIns *>(dev + o_ins64));
+        c->launches += 1;
+    }
+    if (!fb.spec.empty()) {
+        rc_fill_cols<<<dim3((c->npad + 1023) / 1024, (unsigned)fb.spec.size()), 256, 0, c->s>>>(
+            c->d_cols, c->npad, reinterpret_cast<const unsigned *>(dev + o_spec),
+            reinterpret_cast<float *>(dev + o_fcols));
+        c->launches += 1;
+    }
     const int passes = corr ? 2 : 1;
     for (int pass = 0; pass < passes; ++pass) {
         const int kmode = corr ? (pass == 0 ? SM_CORR_PASS1 : SM_CORR_PASS2) : mode;
@@ -398,7 +636,7 @@ float rc_score_run(RcCtx *c, const uint32_t *words, const uint32_t *off, int wid
             const size_t smem = T == 256
                 ? ScoreSmem<256>::total(c->v, staged, a.nslots, group, a.maxins)
                 : ScoreSmem<64>::total(c->v, staged, a.nslots, group, a.maxins);
-            const void *fn = score_kernel_fn(T, track);
+            const void *fn = score_kernel_fn(T, track, kmode);
             if (set_smem(fn, smem) != 0) {
                 st->failed = 1;
                 cudaStreamSynchronize(c->s);
@@ -406,7 +644,7 @@ float rc_score_run(RcCtx *c, const uint32_t *words, const uint32_t *off, int wid
             }
             int grid = c->sm_count * occupancy_blocks(fn, T, smem);
             if (grid > a.nitems) grid = a.nitems;
-            launch_score_kernel(T, track, grid, smem, c->s, a);
+            launch_score_kernel(fn, T, grid, smem, c->s, a);
             c->launches += 1;
             obase += nb;
         }
@@ -430,8 +668,8 @@ float rc_score_run(RcCtx *c, const uint32_t *words, const uint32_t *off, int wid
         l.w = c->d_w64;
         l.n = c->n;
         l.npad = c->npad;
-        l.ins = a.ins;
-        l.ins_off = a.ins_off;
+        l.ins = folded ? reinterpret_cast<const RcIns *>(dev + o_ins64) : a.ins;
+        l.ins_off = folded ? reinterpret_cast<const int *>(dev + o_off64) : a.ins_off;
         l.flagged = reinterpret_cast<const int *>(dev + o_flagged);
         l.nflag = d_nflag;
         l.ntiles = ntiles;
@@ -446,13 +684,6 @@ float rc_score_run(RcCtx *c, const uint32_t *words, const uint32_t *off, int wid
         l.rows = d_rows + 1;
         l.opw = a.opw;
         const size_t smem = lane_smem(max_slots);
-        if (set_smem((const void *)rc_score64_kernel<LANE_T>, smem) != 0) {
-            st->failed = 1;
-            cudaStreamSynchronize(c->s);
-            return -1.0f;
-        }
-        const int grid = c->sm_count *
-                         occupancy_blocks((const void *)rc_score64_kernel<LANE_T>, LANE_T, smem);
         if (a.badrow) {
             /* the f32 failure rows first: most failures are confirmed there */
             l.mode = mode;
@@ -470,7 +701,15 @@ float rc_score_run(RcCtx *c, const uint32_t *words, const uint32_t *off, int wid
             l.counter = d_cnt + 4 + pass;
             l.mode = kmode;
             c->launches += 2;
-            rc_score64_kernel<LANE_T><<<grid, LANE_T, smem, c->s>>>(l);
+            const void *fn = lane_kernel_fn(kmode);
+            if (set_smem(fn, smem) != 0) {
+                st->failed = 1;
+                cudaStreamSynchronize(c->s);
+                return -1.0f;
+            }
+            void *args[] = {(void *)&l};
+            cudaLaunchKernel(fn, dim3(c->sm_count * occupancy_blocks(fn, LANE_T, smem)), dim3(LANE_T),
+                             args, smem, c->s);
             rc_score64_finalize<<<(nprog + 127) / 128, 128, 0, c->s>>>(
                 l.flagged, d_nflag, ntiles, l.part, nprog, ntiles, l.bad, c->n,
                 (corr && pass == 1) ? mode : kmode, c->syy,
@@ -925,24 +1164,24 @@ extern "C" int rc_score_batch_noalloc(const float *cols, const float *y, int n, 
                 return -1;
             }
             const size_t maxsmem = ScoreSmem<256>::total(0, 0, RC_SHALLOW_SLOTS, G, RC_MAX_INS);
-            if (set_smem((const void *)rc_score_kernel<256, true>, maxsmem) != 0 ||
-                set_smem((const void *)rc_score64_kernel<LANE_T>, lsmem) != 0)
+            if (set_smem((const void *)rc_score_kernel<256, true, -1>, maxsmem) != 0 ||
+                set_smem((const void *)rc_score64_kernel<LANE_T, -1>, lsmem) != 0)
                 return -1;
             int sms = 1;
             cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
             d->scratch = (unsigned char *)ptr;
             d->sm_count = sms > 0 ? sms : 1;
             d->grid_per_sm =
-                occupancy_blocks((const void *)rc_score_kernel<256, true>, T, maxsmem);
+                occupancy_blocks((const void *)rc_score_kernel<256, true, -1>, T, maxsmem);
             d->lane_per_sm =
-                occupancy_blocks((const void *)rc_score64_kernel<LANE_T>, LANE_T, lsmem);
+                occupancy_blocks((const void *)rc_score64_kernel<LANE_T, -1>, LANE_T, lsmem);
             d->ready = 1;
         }
     }
     /* the limits only grow, and another path may have launched these
        kernels since; raising them again is a no-op when already high enough */
-    if (set_smem((const void *)rc_score_kernel<256, true>, smem) != 0 ||
-        set_smem((const void *)rc_score64_kernel<LANE_T>, lsmem) != 0) {
+    if (set_smem((const void *)rc_score_kernel<256, true, -1>, smem) != 0 ||
+        set_smem((const void *)rc_score64_kernel<LANE_T, -1>, lsmem) != 0) {
         fprintf(stderr, "rc_score_batch_noalloc: cannot raise the shared-memory limit\n");
         return -1;
     }
@@ -981,7 +1220,7 @@ extern "C" int rc_score_batch_noalloc(const float *cols, const float *y, int n, 
     a.mode = kind;
     int grid = d->sm_count * d->grid_per_sm;
     if (grid > a.nitems) grid = a.nitems;
-    rc_score_kernel<256, true><<<grid, T, smem, s>>>(a);
+    rc_score_kernel<256, true, -1><<<grid, T, smem, s>>>(a);
     {
         /* a failed scoring launch must not let the finalize kernels write
            stale scratch into the caller's outputs */
@@ -1014,7 +1253,7 @@ extern "C" int rc_score_batch_noalloc(const float *cols, const float *y, int n, 
     l.ptiles = ntiles;
     l.bad = reinterpret_cast<int *>(sc + o_bad64);
     l.mode = kind;
-    rc_score64_kernel<LANE_T><<<d->sm_count * d->lane_per_sm, LANE_T, lsmem, s>>>(l);
+    rc_score64_kernel<LANE_T, -1><<<d->sm_count * d->lane_per_sm, LANE_T, lsmem, s>>>(l);
     rc_score64_finalize<<<(nprog + 127) / 128, 128, 0, s>>>(l.flagged, l.nflag, ntiles, l.part,
                                                             nprog, ntiles, l.bad, n, kind, 0.0,
                                                             out, status, nullptr);

@@ -269,7 +269,7 @@ template <int T, bool TRACK>
 __device__ __forceinline__ void rc_run(const RcIns *__restrict__ prog, const float4 *xs,
                                        bool staged, const float *__restrict__ cols, int npad,
                                        int myrow, float4 *stk, uint2 *estk, int tid, float4 &p,
-                                       float4 &pe)
+                                       float4 &pe, const float *__restrict__ fcols = nullptr)
 {
     float t0 = 0.f, t1 = 0.f, t2 = 0.f, t3 = 0.f;
     float e0 = 0.f, e1 = 0.f, e2 = 0.f, e3 = 0.f;
@@ -355,6 +355,38 @@ __device__ __forceinline__ void rc_run(const RcIns *__restrict__ prog, const flo
                     t0 = o.t[0]; t1 = o.t[1]; t2 = o.t[2]; t3 = o.t[3];
                     e0 = o.e[0]; e1 = o.e[1]; e2 = o.e[2]; e3 = o.e[3];
                 } break;
+            }
+            continue;
+        }
+        if (kind >= K_PUSH_COL) {
+            if (in.spill != 0xff) {
+                stk[in.spill * T + tid] = make_float4(t0, t1, t2, t3);
+                if (TRACK) estk[in.spill * T + tid] = rc_pack_err(e0, e1, e2, e3);
+            }
+            if (kind == K_PUSH_COL) {
+                /* sin, cos or exp of an input: its value from the column, its
+                   bound as the operator gives it for an exact operand */
+                const float4 x = __ldg(reinterpret_cast<const float4 *>(
+                    fcols + (size_t)in.imm * (size_t)npad + myrow));
+                t0 = x.x; t1 = x.y; t2 = x.z; t3 = x.w;
+                if (TRACK) {
+                    if (in.op == OP_EXP) {
+                        e0 = rc_un_err<OP_EXP>(0.f, 0.f, t0);
+                        e1 = rc_un_err<OP_EXP>(0.f, 0.f, t1);
+                        e2 = rc_un_err<OP_EXP>(0.f, 0.f, t2);
+                        e3 = rc_un_err<OP_EXP>(0.f, 0.f, t3);
+                    } else {
+                        e0 = rc_un_err<OP_SIN>(0.f, 0.f, t0);
+                        e1 = rc_un_err<OP_SIN>(0.f, 0.f, t1);
+                        e2 = rc_un_err<OP_SIN>(0.f, 0.f, t2);
+                        e3 = rc_un_err<OP_SIN>(0.f, 0.f, t3);
+                    }
+                }
+            } else {
+                const float c = __uint_as_float(in.imm);
+                const float e = __uint_as_float(prog[++pc].imm);
+                t0 = c; t1 = c; t2 = c; t3 = c;
+                e0 = e; e1 = e; e2 = e; e3 = e;
             }
             continue;
         }
@@ -458,6 +490,7 @@ struct ScoreArgs {
     const double *w;
     int n, npad, v;
     int staged;
+    const float *fcols;   /* the batch's columns of op(input) (K_PUSH_COL) */
     const RcIns *ins;
     const int *ins_off;
     const int *ins_len;   /* [P] instructions per program, or null: ins_off[p + 1] - ins_off[p] */
@@ -493,7 +526,7 @@ __device__ __forceinline__ void rc_accumulate(const ScoreArgs &a, int mode, floa
                                               float yv, int row, int cand, double &a0,
                                               double &a1, double &e0, double &e1, int &bad)
 {
-    const bool finite = isfinite(pr) && fabsf(pr) <= 1e30f;
+    const bool finite = fabsf(pr) <= 1e30f; /* (false for NaN and infinities) */
     if (mode >= SM_EVAL_SQUARED && mode <= SM_EVAL_ABSOLUTE) {
         if (!finite) a0 += 1e30;
         else a0 += (double)rc_row_loss(pr - yv, mode - SM_EVAL_SQUARED);
@@ -596,7 +629,13 @@ struct ScoreSmem {
     }
 };
 
-template <int T, bool TRACK>
+/* `MODE` is the scoring mode of the launch, or -1: read it from the
+   arguments. The modes a search scores every candidate under have launches of
+   their own: with the mode known, a row's accumulation is a dozen
+   instructions, where choosing it per row took about ninety, a third of the
+   kernel on programs of a dozen operators (4,096 x 1,048,576 rows: 10.1 ms
+   with the mode read from the arguments, 7.4 ms with it compiled in). */
+template <int T, bool TRACK, int MODE>
 __global__ void __launch_bounds__(T) rc_score_kernel(ScoreArgs a)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -611,7 +650,7 @@ __global__ void __launch_bounds__(T) rc_score_kernel(ScoreArgs a)
     __shared__ unsigned s_bad;
     __shared__ unsigned long long s_rows, s_ops;
     const int SUB = T * 4;
-    const int mode = a.mode;
+    const int mode = MODE >= 0 ? MODE : a.mode;
     const bool skip_bad = rc_mode_tracks(mode);
 
     for (;;) {
@@ -658,7 +697,7 @@ __global__ void __launch_bounds__(T) rc_score_kernel(ScoreArgs a)
                 wrows += max(0, min(128, a.n - (row0 + 128 * warp)));
                 float4 p, pe;
                 rc_run<T, TRACK>(sprog + c * a.maxins, nullptr, false, a.cols, a.npad, myrow, stk,
-                                 estk, tid, p, pe);
+                                 estk, tid, p, pe, a.fcols);
                 const float4 yv4 = __ldg(reinterpret_cast<const float4 *>(a.y + myrow));
                 const float pr[4] = {p.x, p.y, p.z, p.w};
                 const float pq[4] = {pe.x, pe.y, pe.z, pe.w};
@@ -944,6 +983,11 @@ __device__ __forceinline__ double2 rc_run_d(const RcIns *__restrict__ prog,
             t1 = rc_binary_d(in.op, a1, b1);
             continue;
         }
+        if (kind == K_PUSH_FOLD) {
+            if (in.spill != 0xff) stk[in.spill * T + tid] = make_double2(t0, t1);
+            t0 = t1 = __hiloint2double((int)prog[++pc].imm, (int)in.imm);
+            continue;
+        }
         if (kind == K_IF) {
             const double2 cnd = stk[in.arg * T + tid];
             const double2 a = stk[(in.arg + 1) * T + tid];
@@ -983,7 +1027,7 @@ struct Score64Args {
     const int *opw;
 };
 
-template <int T>
+template <int T, int MODE>
 __global__ void __launch_bounds__(T) rc_score64_kernel(Score64Args a)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -994,7 +1038,7 @@ __global__ void __launch_bounds__(T) rc_score64_kernel(Score64Args a)
     const int tid = threadIdx.x;
     const int SUB = 2 * T;
     const int subtiles = a.tile_rows / SUB;
-    const int mode = a.mode;
+    const int mode = MODE >= 0 ? MODE : a.mode;
     for (;;) {
         const int total = *a.nflag * a.ntiles;
         if (tid == 0) {
@@ -1179,4 +1223,67 @@ __global__ void rc_score64_finalize(const int *__restrict__ flagged, const int *
     }
     out[cand] = v;
     status[cand] = st;
+}
+
+/* ---- what a batch's programs share over its rows -------------------------
+ *
+ * Of the operators that a batch of random programs runs on every row, about
+ * 15 % have constant operands only and 22 % are sin, cos or exp of an input
+ * (the commonest leaf of a search's population), and they are among the
+ * dearest. The first are evaluated once per program, the second once per
+ * input for the whole batch, by the same functions, so neither values nor
+ * bounds change; the rows then read a constant or a column. */
+
+/* One constant subtree: its program (closed by K_HALT) in fold_ins, and the
+   K_PUSH_FOLD words it fills in the f32 and f64 lists. */
+struct RcFold {
+    int prog, at32, at64;
+};
+
+#define RC_FOLD_T 32
+__global__ void __launch_bounds__(RC_FOLD_T) rc_fold(int nfold, const RcFold *__restrict__ folds,
+                                                     const RcIns *__restrict__ fold_ins, int nslots,
+                                                     RcIns *ins32, RcIns *ins64)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    float4 *stk = reinterpret_cast<float4 *>(smem_raw);
+    uint2 *estk = reinterpret_cast<uint2 *>(stk + nslots * RC_FOLD_T);
+    const int k = blockIdx.x * RC_FOLD_T + threadIdx.x;
+    if (k >= nfold) return;
+    const RcFold f = folds[k];
+    float4 p, pe;
+    rc_run<RC_FOLD_T, true>(fold_ins + f.prog, nullptr, false, nullptr, 0, 0, stk, estk, threadIdx.x, p,
+                            pe);
+    ins32[f.at32].imm = __float_as_uint(p.x);
+    ins32[f.at32 + 1].imm = __float_as_uint(pe.x);
+    const double2 d = rc_run_d<RC_FOLD_T>(fold_ins + f.prog, nullptr, 0, 0,
+                                          reinterpret_cast<double2 *>(smem_raw), threadIdx.x);
+    ins64[f.at64].imm = (unsigned)__double2loint(d.x);
+    ins64[f.at64 + 1].imm = (unsigned)__double2hiint(d.x);
+}
+
+/* The batch's columns: spec[c] = input << 8 | operator (sin, cos, exp). */
+__global__ void __launch_bounds__(256) rc_fill_cols(const float *__restrict__ cols, int npad,
+                                                    const unsigned *__restrict__ spec, float *fcols)
+{
+    const unsigned s = spec[blockIdx.y];
+    const int row = 4 * (blockIdx.x * 256 + threadIdx.x);
+    if (row >= npad) return;
+    const float4 x = __ldg(reinterpret_cast<const float4 *>(cols + (size_t)(s >> 8) * npad + row));
+    float4 r;
+    switch (s & 255u) {
+        case OP_SIN:
+            r = make_float4(rc_unary_f(OP_SIN, x.x), rc_unary_f(OP_SIN, x.y), rc_unary_f(OP_SIN, x.z),
+                            rc_unary_f(OP_SIN, x.w));
+            break;
+        case OP_COS:
+            r = make_float4(rc_unary_f(OP_COS, x.x), rc_unary_f(OP_COS, x.y), rc_unary_f(OP_COS, x.z),
+                            rc_unary_f(OP_COS, x.w));
+            break;
+        default:
+            r = make_float4(rc_unary_f(OP_EXP, x.x), rc_unary_f(OP_EXP, x.y), rc_unary_f(OP_EXP, x.z),
+                            rc_unary_f(OP_EXP, x.w));
+            break;
+    }
+    *reinterpret_cast<float4 *>(fcols + (size_t)blockIdx.y * npad + row) = r;
 }
