@@ -206,6 +206,7 @@ struct FitArgs {
     int nprog;
     FitState *state;
     double *part;      /* [P][ntiles][FT_PART_STRIDE] */
+    double *run;       /* [P] objective of the trial sweep so far (ft_trial_lost) */
     int *lists;        /* the chain's [2][FOP_COUNT][P] */
     int *counts;       /* the chain's [2][FOP_COUNT] candidates queued per kind */
     int *work;         /* the chain's [2][FOP_COUNT] persistent-grid work counters */
@@ -230,6 +231,20 @@ __device__ __forceinline__ void ft_clear_other(const FitArgs &a, int q)
         a.counts[(q ^ 1) * FOP_COUNT + threadIdx.x] = 0;
         a.work[(q ^ 1) * FOP_COUNT + threadIdx.x] = 0;
     }
+}
+
+/* Whether a trial's sweep can stop. A trial (sel 1) is accepted only when its
+   objective is below the one to beat; the objective is a sum of terms that are
+   not negative, so once the tiles summed so far exceed it (by more than any
+   rounding of the order they add up in) the trial is rejected whatever the
+   others hold. `run` is the candidate's running sum, cleared with each
+   request, and an item's tile is left out (it counts 0) when this holds. The
+   objective sweeps take tile after tile over all their candidates, so that
+   most of a rejected trial (half of the trials of a fit) is still ahead. */
+__device__ __forceinline__ bool ft_trial_lost(const FitArgs &a, int cand)
+{
+    const FitState *st = a.state + cand;
+    return st->sel == 1 && *(volatile const double *)(a.run + cand) > st->best * (1.0 + 1e-9);
 }
 
 /* Columns of a sweep's augmented Gram: the Jacobian and the residual, or for
@@ -448,10 +463,10 @@ __global__ void __launch_bounds__(FT_IMAXT, 1) ft_cost_sweep(FitArgs a, int q)
               (size_t)grp * FT_ITHREADS * (a.xslots + a.xtape + a.v);
     V4 *tape = stk + (size_t)a.xslots * FT_ITHREADS;
     V4 *ig = tape + (size_t)a.xtape * FT_ITHREADS;
-    __shared__ int s_item;
+    __shared__ int s_item, s_lost;
     ft_clear_other(a, q);
     const int *list = a.lists + ((size_t)q * FOP_COUNT + FOP_ICOST) * a.nprog;
-    const int total = a.counts[q * FOP_COUNT + FOP_ICOST] * a.ntiles;
+    const int ncand = a.counts[q * FOP_COUNT + FOP_ICOST], total = ncand * a.ntiles;
     int *work = a.work + q * FOP_COUNT + FOP_ICOST;
     for (;;) {
         if (tid == 0) s_item = atomicAdd(work, 1);
@@ -459,9 +474,18 @@ __global__ void __launch_bounds__(FT_IMAXT, 1) ft_cost_sweep(FitArgs a, int q)
         const int item = s_item;
         __syncthreads();
         if (item >= total) break;
-        const int cand = list[item / a.ntiles];
-        const int tile = item % a.ntiles;
+        const int cand = list[item % ncand];
+        const int tile = item / ncand;
         const FitState *st = a.state + cand;
+        if (tid == 0) s_lost = ft_trial_lost(a, cand);
+        __syncthreads();
+        if (s_lost) {
+            if (tid == 0) {
+                double *pt = a.part + ((size_t)cand * a.ntiles + tile) * FT_PART_STRIDE;
+                pt[FT_PART_LOSS] = pt[FT_PART_BAD] = pt[FT_PART_SKIP] = 0.0;
+            }
+            continue;
+        }
         const int4 info = a.xinfo[cand];
         const int ib = a.xfins_off[cand];
         const int p = a.pcount[cand];
@@ -473,6 +497,8 @@ __global__ void __launch_bounds__(FT_IMAXT, 1) ft_cost_sweep(FitArgs a, int q)
         const int r1 = min(a.n, r0 + FT_TILE_ROWS);
         double *pt = a.part + ((size_t)cand * a.ntiles + tile) * FT_PART_STRIDE;
         ft_tile_icost_x(a, ins, ins + info.x, cd, stk, tape, ig, red, r0, r1, pt);
+        /* (an undefined row rejects the trial too) */
+        if (tid == 0) atomicAdd(a.run + cand, pt[FT_PART_BAD] != 0.0 ? INFINITY : pt[FT_PART_LOSS]);
         __syncthreads();
     }
 }
@@ -1056,10 +1082,12 @@ __device__ void ft_sweep_item(const FitArgs &a, unsigned char *sm, int cand, int
                                             info.w >> 16, cv, region, red, r0, r1, pt, ccols);
     else if constexpr (OPK == FOP_CSCORE)
         ft_tile_corr_score<NR>(a, ins, cv, reinterpret_cast<V4 *>(region), red, r0, r1, pt, ccols);
-    else
+    else {
         ft_tile_loss<V, NR, GROUPED>(a, ins, cv,
                             reinterpret_cast<V4 *>(region) + (size_t)(tid / FT_LOSS_T) * slots * FT_LOSS_T,
                             slots, red, r0, r1, pt, ccols);
+        if (tid == 0) atomicAdd(a.run + cand, pt[FT_PART_LOSS]);
+    }
 }
 
 /* The sweeps of kinds K0, K1, ... of step parity q in one launch: a
@@ -1074,7 +1102,7 @@ __global__ void __launch_bounds__(ft_op_assembles(K0) ? 640 : 1024, 1) ft_sweep4
     extern __shared__ __align__(16) unsigned char sm[];
     constexpr int kinds[] = {K0, KS...};
     constexpr int NK = 1 + sizeof...(KS);
-    __shared__ int s_item;
+    __shared__ int s_item, s_lost;
     const int tid = threadIdx.x;
     ft_clear_other(a, q);
     int counts[NK], total = 0;
@@ -1091,21 +1119,33 @@ __global__ void __launch_bounds__(ft_op_assembles(K0) ? 640 : 1024, 1) ft_sweep4
         const int item = s_item;
         __syncthreads();
         if (item >= total) break;
-        int c = item / a.ntiles;
-        const int tile = item - c * a.ntiles;
-        int kind = K0;
+        int left = item, kind = K0, cand = 0, tile = 0;
         const int *lists = a.lists + (size_t)q * FOP_COUNT * a.nprog;
         bool found = false;
-        int cand = 0;
 #pragma unroll
         for (int k = 0; k < NK; ++k) {
             if (found) continue;
-            if (c < counts[k]) {
+            if (left < counts[k] * a.ntiles) {
+                /* assemblies candidate by candidate, objectives tile by tile */
+                const bool obj = kinds[k] == FOP_LOSS32 || kinds[k] == FOP_LOSS64;
+                const int c = obj ? left % counts[k] : left / a.ntiles;
+                tile = obj ? left / counts[k] : left - c * a.ntiles;
                 kind = kinds[k];
                 cand = lists[(size_t)kind * a.nprog + c];
                 found = true;
             } else {
-                c -= counts[k];
+                left -= counts[k] * a.ntiles;
+            }
+        }
+        if (kind == FOP_LOSS32 || kind == FOP_LOSS64) {
+            if (tid == 0) s_lost = ft_trial_lost(a, cand);
+            __syncthreads();
+            if (s_lost) {
+                if (tid == 0) {
+                    double *pt = a.part + ((size_t)cand * a.ntiles + tile) * FT_PART_STRIDE;
+                    pt[FT_PART_LOSS] = pt[FT_PART_BAD] = 0.0;
+                }
+                continue;
             }
         }
         if constexpr (NK == 1) {
@@ -1928,6 +1968,7 @@ __global__ void __launch_bounds__(FT_CTRL_T) ft_control(FitArgs a, int q, int in
         if (tid == 0 && sst.op != FOP_NONE) {
             /* the start of a fit serves every chain: its arguments are the
                first chain's */
+            a.run[cand] = 0.0;
             const size_t ch = init ? (size_t)((unsigned)a.finfo[cand].z >> 24) : 0;
             int *counts = a.counts + ch * 2 * FOP_COUNT;
             int *lists = a.lists + ch * 2 * FOP_COUNT * (size_t)a.nprog;
@@ -2738,6 +2779,7 @@ float fit_run(RcCtx *c, const unsigned int *prog, const unsigned int *off, const
     const size_t io_end = rc_take(&cur, 0);
     const size_t o_state = rc_take(&cur, sizeof(FitState) * nprog);
     const size_t o_part = rc_take(&cur, sizeof(double) * (size_t)nprog * ntiles * FT_PART_STRIDE);
+    const size_t o_run = rc_take(&cur, sizeof(double) * nprog);
     /* every chain's queues; counts and work counters, zeroed together */
     const size_t o_lists =
         rc_take(&cur, sizeof(int) * 2 * FOP_COUNT * (size_t)nprog * FT_MAX_CHAINS);
@@ -2842,6 +2884,7 @@ float fit_run(RcCtx *c, const unsigned int *prog, const unsigned int *off, const
     a.nprog = nprog;
     a.state = reinterpret_cast<FitState *>(dev + o_state);
     a.part = reinterpret_cast<double *>(dev + o_part);
+    a.run = reinterpret_cast<double *>(dev + o_run);
     a.lists = reinterpret_cast<int *>(dev + o_lists);
     a.counts = reinterpret_cast<int *>(dev + o_counts);
     a.work = reinterpret_cast<int *>(dev + o_work);
@@ -2886,6 +2929,7 @@ float fit_run(RcCtx *c, const unsigned int *prog, const unsigned int *off, const
             one.nsub = b.sub_cand_off[i + 1] - b.sub_cand_off[i];
             one.state = a.state + i;
             one.part = a.part + (size_t)i * ntiles * FT_PART_STRIDE;
+            one.run = a.run + i;
             one.outc = a.outc + (size_t)i * kmax;
             one.outsse = a.outsse + i;
             one.outstatus = a.outstatus + i;
