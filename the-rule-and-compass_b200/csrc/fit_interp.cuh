@@ -215,7 +215,12 @@ inline bool fi_decode(const uint32_t *rec, int m, std::vector<FIns> &fwd, std::v
         }
     }
     /* a constant slot met again (in reverse order) accumulates */
-    std::vector<char> seen(65536, 0);
+    unsigned slots = 0;
+    for (const FIns &r : rev) {
+        const unsigned k = r.kind & FI_KIND_MASK;
+        if (k == FI_PUSH_PARAM || k == FI_BIN_P) slots = slots > r.imm + 1u ? slots : r.imm + 1u;
+    }
+    std::vector<char> seen(slots, 0);
     for (int j = (int)rev.size() - 1; j >= 0; --j) {
         const unsigned k = rev[j].kind & FI_KIND_MASK;
         if (k == FI_PUSH_PARAM || k == FI_BIN_P) {
