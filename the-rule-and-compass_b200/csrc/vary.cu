@@ -251,6 +251,11 @@ extern "C" float rc_pool_vary(void *ctx, int which, int islands, int pop, int wi
     rv_parents<<<(nslots + RV_T - 1) / RV_T, RV_T, 0, c->s>>>(c->d_pool[b], width, nslots, d_plen,
                                                              d_pcost, d_pcost16, d_phash, d_bad);
 
+    /* read back while the children are built: the parents' hashes and the
+       elites are ready when the items arrive */
+    cudaMemcpyAsync(host + o_plen, dev + o_plen, o_items - o_plen, cudaMemcpyDeviceToHost, c->s);
+    cudaEventRecord(c->sp[0], c->s);
+
     /* 2. the first RV_K attempts of every child slot */
     RvParents dpar;
     dpar.words = c->d_pool[b];
@@ -262,11 +267,19 @@ extern "C" float rc_pool_vary(void *ctx, int which, int islands, int pop, int wi
     uint32_t *d_progs = reinterpret_cast<uint32_t *>(dev + o_progs);
     rv_children<<<(nitems + RV_T - 1) / RV_T, RV_T, 0, c->s>>>(
         cfg, dpar, reinterpret_cast<const uint8_t *>(dev + o_restart), d_bad, d_items, d_progs);
-    cudaMemcpyAsync(host + o_plen, dev + o_plen, meta_end - o_plen, cudaMemcpyDeviceToHost, c->s);
+    cudaMemcpyAsync(host + o_items, dev + o_items, meta_end - o_items, cudaMemcpyDeviceToHost, c->s);
     c->launches += 2;
-    if (rc_finish(c) != 0) return -1.0f;
-    /* a parent slot that is not a valid program fails the call */
-    if (*reinterpret_cast<const int *>(host + o_bad) != 0) return -1.0f;
+    if (cudaGetLastError() != cudaSuccess || cudaEventSynchronize(c->sp[0]) != cudaSuccess) {
+        cudaStreamSynchronize(c->s);
+        cudaGetLastError();
+        return -1.0f;
+    }
+    /* a parent slot that is not a valid program fails the call (its children
+       are not built) */
+    if (*reinterpret_cast<const int *>(host + o_bad) != 0) {
+        rc_finish(c);
+        return -1.0f;
+    }
     const uint16_t *cost16 = reinterpret_cast<const uint16_t *>(host + o_pcost16);
 
     /* 3. the duplicate rule, in slot order */
@@ -291,10 +304,10 @@ extern "C" float rc_pool_vary(void *ctx, int which, int islands, int pop, int wi
     HashSet64 seen((size_t)2 * nslots);
     if (dedup)
         for (int k = 0; k < nslots; ++k) seen.insert(phash[k]);
+    std::vector<int> elites(islands, 0);
     for (int i = 0; i < islands; ++i) {
-        const bool rs = restart && restart[i];
         int elite = i * pop;
-        if (!rs) {
+        if (!(restart && restart[i])) {
             RvKey kb = rv_key(err, cost16, elite);
             for (int k = i * pop + 1; k < (i + 1) * pop; ++k) {
                 const RvKey kk = rv_key(err, cost16, k);
@@ -304,6 +317,12 @@ extern "C" float rc_pool_vary(void *ctx, int which, int islands, int pop, int wi
                 }
             }
         }
+        elites[i] = elite;
+    }
+    if (rc_finish(c) != 0) return -1.0f; /* the items are here */
+    for (int i = 0; i < islands; ++i) {
+        const bool rs = restart && restart[i];
+        const int elite = elites[i];
         for (int j = 0; j < pop; ++j) {
             const int k = i * pop + j;
             RvChoice &ch = choice[k];
@@ -385,13 +404,13 @@ extern "C" float rc_pool_vary(void *ctx, int which, int islands, int pop, int wi
     if (out_words)
         cudaMemcpyAsync(out_words, c->d_pool[b ^ 1], sizeof(uint32_t) * total,
                         cudaMemcpyDeviceToHost, c->s);
-    if (rc_finish(c) != 0) return -1.0f;
     for (int k = 0; k < nslots; ++k) {
         if (out_len) out_len[k] = choice[k].len;
         if (out_cost) out_cost[k] = choice[k].cost;
         if (out_hash) out_hash[k] = choice[k].hash;
         if (out_err) out_err[k] = choice[k].err;
     }
+    if (rc_finish(c) != 0) return -1.0f;
     float ms = -1.0f;
     cudaEventElapsedTime(&ms, c->t0, c->t1);
     return ms;
