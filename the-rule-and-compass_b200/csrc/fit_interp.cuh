@@ -463,7 +463,7 @@ __device__ __forceinline__ void fi_partials(unsigned op, V x, V y, V r, V &d0, V
    16-byte vector (spill slots, tape, column loads). */
 template <typename V, int NR>
 struct FiV {
-    struct alignas(sizeof(V) * NR) V4 {
+    struct alignas(sizeof(V) * NR > 16 ? 16 : sizeof(V) * NR) V4 {
         V v[NR];
     };
     __device__ __forceinline__ static void unpack(const V4 &x, V *v)
@@ -481,6 +481,11 @@ struct FiV {
     /* read-only load of NR consecutive column values */
     __device__ __forceinline__ static void ldg(const V *p, V *v)
     {
+        if constexpr (sizeof(V4) == 32) {
+            FiV<V, NR / 2>::ldg(p, v);
+            FiV<V, NR / 2>::ldg(p + NR / 2, v + NR / 2);
+            return;
+        }
         V4 x;
         if constexpr (sizeof(V4) == 16) {
             const float4 t = __ldg(reinterpret_cast<const float4 *>(p));
