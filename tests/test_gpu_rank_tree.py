@@ -27,3 +27,28 @@ def test_bucketed_sums_equal_the_sorted_ones(pkg, E, n):
     assert ev.rank_fallbacks() == len(trees)
     assert sums == want
     ev.close()
+
+
+@pytest.mark.parametrize("n,values", [(20001, 2000), (65536, 20000), (300007, 6000), (300007, 150000)])
+def test_groups_of_ties_equal_the_sorted_ones(pkg, E, n, values):
+    """Digit groups of equal keys, of a few distinct ones and of both, and
+    buckets of more keys than the block holds in registers; a comparison bound
+    of one sorts every bucket with a mixed group."""
+    rng = np.random.Generator(np.random.PCG64(values))
+    x = rng.integers(0, values, n) / 64.0
+    x[: n // 3] = x[: n // 3] % 8.0  # a third of the rows in few buckets
+    y = np.round(rng.standard_normal(n), 3)
+    ev = pkg.GpuEvaluator(x.astype(np.float32), n, 1, y.astype(np.float32))
+    ev.set_fit_data(x, y)
+    trees = [E.node(E.ADD, [E.node(E.MUL, [E.constant(c), E.input(0)]), E.constant(1.0)])
+             for c in (1.0, -0.3)]
+    plans = [pkg.gpu_fit_plan(t, allow_no_constants=True) for t in trees]
+    prog, off, pcount, c0, _, kmax = pkg.pack_plans(plans)
+    got = []
+    for cap, gmax in ((0, 0), (0, 1), (-1, 0)):
+        ev.rank_tuning(cap, gmax)
+        sums, status, _, _ = ev.rank_sums(prog, off, pcount, c0, kmax)
+        assert list(status) == [0, 0]
+        got.append(sums)
+    assert got[0] == got[2] and got[1] == got[2]
+    ev.close()

@@ -994,12 +994,11 @@ __global__ void __launch_bounds__(RB_ST) rb_scan(int n, int cap, const int *nspl
     if (bad) ovf[ls] = 1;
 }
 
-/* Shared layout of rb_local: the bucket's keys and B in digit order, the
-   digit groups' first positions (RB_DIG + 1), their cursors and flags. */
+/* Shared layout of rb_local: the bucket's keys in digit order, the digit
+   groups' cursors and flags. */
 __host__ __device__ constexpr size_t rb_local_smem()
 {
-    return (size_t)RB_CAP * (sizeof(u64) + sizeof(int)) + (2 * RB_DIG + 1) * sizeof(unsigned) +
-           RB_DIG;
+    return (size_t)RB_CAP * sizeof(u64) + RB_DIG * (sizeof(unsigned) + 1);
 }
 
 /* Sum of a 64-bit integer over a block of NT threads: warp butterflies, then
@@ -1020,13 +1019,21 @@ __device__ __forceinline__ long long rb_block_sum64(long long v, long long *ws)
 }
 
 #define RB_LT 512 /* rb_local threads */
-static_assert(RB_DIG == 2 * RB_LT, "two digit groups per thread");
+#define RB_LR 4   /* keys each holds in registers */
+static_assert(RB_DIG % RB_LT == 0, "whole digit groups per thread");
 
 /* One block per (segment, range bucket): runs and partial sums of its c
    keys, which hold positions [O, O + c) of the segment's order. A thread
    holds at most RB_CAP / RB_LT keys, each |A * B| and A^2 at most n^2, so
-   per-thread and block sums fit 64 bits for the n this path takes. */
-__global__ void __launch_bounds__(RB_LT, 2) rb_local(int n, int m, int cap, int gmax,
+   per-thread and block sums fit 64 bits for the n this path takes.
+
+   A bucket is a short chain of passes with a barrier after each, so its time
+   is latency and the blocks an SM holds decide: shared memory keeps the keys
+   alone, as each thread ranks the keys that it holds itself and reads their B
+   where it uses them (keys and B, one thread for each position, allow two
+   blocks instead of three: 32 segments of 2,097,152 rows, 24 of them live,
+   1.07 -> 0.89 ms; three blocks of 256 threads 1.1, two of 1,024 1.4). */
+__global__ void __launch_bounds__(RB_LT, 3) rb_local(int n, int m, int cap, int gmax,
                                                      const int *nspl, const unsigned *rcur,
                                                      const unsigned *boff, const u64 *bkey,
                                                      const int *bval, __int128 *part, int *ovf,
@@ -1034,9 +1041,7 @@ __global__ void __launch_bounds__(RB_LT, 2) rb_local(int n, int m, int cap, int 
 {
     extern __shared__ __align__(16) unsigned char sm[];
     u64 *sk = reinterpret_cast<u64 *>(sm);
-    int *sv = reinterpret_cast<int *>(sk + RB_CAP);
-    unsigned *gst = reinterpret_cast<unsigned *>(sv + RB_CAP);
-    unsigned *cur = gst + RB_DIG + 1;
+    unsigned *cur = reinterpret_cast<unsigned *>(sk + RB_CAP);
     unsigned char *mixed = reinterpret_cast<unsigned char *>(cur + RB_DIG);
     __shared__ u64 s_lo[RB_LT / 32], s_hi[RB_LT / 32];
     __shared__ unsigned wsum[RB_LT / 32];
@@ -1061,12 +1066,22 @@ __global__ void __launch_bounds__(RB_LT, 2) rb_local(int n, int m, int cap, int 
     const int *bv = bval + base;
     __int128 *pp = part + ((size_t)ls * 2 * RB_MAXB + 2 * idx) * 2;
 
+    /* a thread's first RB_LR keys stay in registers over the passes; those
+       of a larger bucket are read again */
+    u64 kr[RB_LR];
+#pragma unroll
+    for (int r = 0; r < RB_LR; ++r) kr[r] = r * RB_LT + tid < c ? bk[r * RB_LT + tid] : 0ULL;
+    const auto each = [&](auto &&f) {
+#pragma unroll
+        for (int r = 0; r < RB_LR; ++r)
+            if (r * RB_LT + tid < c) f(kr[r], r * RB_LT + tid);
+        for (int q = RB_LR * RB_LT + tid; q < c; q += RB_LT) f(bk[q], q);
+    };
     u64 lo = ~0ULL, hi = 0ULL;
-    for (int q = tid; q < c; q += RB_LT) {
-        const u64 k = bk[q];
+    each([&](u64 k, int) {
         lo = k < lo ? k : lo;
         hi = k > hi ? k : hi;
-    }
+    });
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         const u64 a = __shfl_xor_sync(0xffffffffu, lo, o), b = __shfl_xor_sync(0xffffffffu, hi, o);
@@ -1096,10 +1111,15 @@ __global__ void __launch_bounds__(RB_LT, 2) rb_local(int n, int m, int cap, int 
     }
     const int nbits = 64 - __clzll((long long)(hi - lo));
     const int shift = nbits > 10 ? nbits - 10 : 0;
-    for (int q = tid; q < c; q += RB_LT) atomicAdd(&cur[(unsigned)((bk[q] - lo) >> shift)], 1u);
+    each([&](u64 k, int) { atomicAdd(&cur[(unsigned)((k - lo) >> shift)], 1u); });
     __syncthreads();
     {
-        const unsigned a0 = cur[2 * tid], a1 = cur[2 * tid + 1], t = a0 + a1;
+        unsigned t = 0, a[RB_DIG / RB_LT];
+#pragma unroll
+        for (int e = 0; e < RB_DIG / RB_LT; ++e) {
+            a[e] = cur[RB_DIG / RB_LT * tid + e];
+            t += a[e];
+        }
         unsigned x = t;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -1110,62 +1130,53 @@ __global__ void __launch_bounds__(RB_LT, 2) rb_local(int n, int m, int cap, int 
         __syncthreads();
         unsigned run = x - t;
         for (int k = 0; k < w; ++k) run += wsum[k];
-        gst[2 * tid] = run;
-        cur[2 * tid] = run;
-        gst[2 * tid + 1] = run + a0;
-        cur[2 * tid + 1] = run + a0;
-        if (tid == 0) gst[RB_DIG] = (unsigned)c;
+#pragma unroll
+        for (int e = 0; e < RB_DIG / RB_LT; ++e) {
+            cur[RB_DIG / RB_LT * tid + e] = run;
+            run += a[e];
+        }
     }
     __syncthreads();
-    for (int q = tid; q < c; q += RB_LT) {
-        const u64 k = bk[q];
-        const unsigned p = atomicAdd(&cur[(unsigned)((k - lo) >> shift)], 1u);
-        sk[p] = k;
-        sv[p] = bv[q];
-    }
+    each([&](u64 k, int) { sk[atomicAdd(&cur[(unsigned)((k - lo) >> shift)], 1u)] = k; });
     __syncthreads();
-    for (int q = tid; q < c; q += RB_LT) {
-        const u64 k = sk[q];
+    /* each cursor now stands at its group's end; a group is one run unless a
+       key of it differs from its first one */
+    each([&](u64 k, int) {
         const unsigned d = (unsigned)((k - lo) >> shift);
-        if (k != sk[gst[d]]) mixed[d] = 1;
-    }
+        const unsigned gs = d ? cur[d - 1] : 0u;
+        if (k != sk[gs]) mixed[d] = 1;
+    });
     __syncthreads();
     long long ab = 0, aa = 0;
     bool big = false;
-    for (int q = tid; q < c; q += RB_LT) {
-        const u64 k = sk[q];
+    each([&](u64 k, int q) {
         const unsigned d = (unsigned)((k - lo) >> shift);
-        const unsigned gs = gst[d], ge = gst[d + 1];
-        long long i = gs, j = ge;
+        const unsigned gs = d ? cur[d - 1] : 0u, ge = cur[d];
+        unsigned lt = 0, le = ge - gs;
         if (mixed[d]) {
-            if (ge - gs <= (unsigned)gmax) {
-                unsigned lt = 0, le = 0;
+            if (le <= (unsigned)gmax) {
+                le = 0;
                 for (unsigned t = gs; t < ge; ++t) {
                     const u64 o = sk[t];
                     lt += o < k;
                     le += o <= k;
                 }
-                i = gs + lt;
-                j = gs + le;
             } else {
                 big = true;
             }
         }
-        const long long A = 2 * O + i + j - n;
-        ab += A * (long long)sv[q];
+        const long long A = 2 * (O + gs) + lt + le - n;
+        ab += A * (long long)bv[q];
         aa += A * A;
-    }
+    });
     if (__syncthreads_or(big)) {
         /* the digit could not tell a large group apart (keys spread over many
            binades, as in a tail bucket): sort the bucket (bitonic, padded to
-           a power of two by entries that order after every key, B marked
-           INT_MIN) and take each key's run by binary search */
+           a power of two by the largest key) and take each key's run among
+           the c by binary search */
         int P2 = 1;
         while (P2 < c) P2 <<= 1;
-        for (int q = c + tid; q < P2; q += RB_LT) {
-            sk[q] = ~0ULL;
-            sv[q] = INT_MIN;
-        }
+        for (int q = c + tid; q < P2; q += RB_LT) sk[q] = ~0ULL;
         __syncthreads();
         for (int k = 2; k <= P2; k <<= 1)
             for (int j = k >> 1; j > 0; j >>= 1) {
@@ -1173,13 +1184,9 @@ __global__ void __launch_bounds__(RB_LT, 2) rb_local(int n, int m, int cap, int 
                     const int l = i ^ j;
                     if (l > i) {
                         const u64 a = sk[i], b = sk[l];
-                        const int va = sv[i], vb = sv[l];
-                        const bool agt = a > b || (a == b && va == INT_MIN && vb != INT_MIN);
-                        if (agt == ((i & k) == 0)) {
+                        if ((a > b) == ((i & k) == 0)) {
                             sk[i] = b;
                             sk[l] = a;
-                            sv[i] = vb;
-                            sv[l] = va;
                         }
                     }
                 }
@@ -1187,12 +1194,11 @@ __global__ void __launch_bounds__(RB_LT, 2) rb_local(int n, int m, int cap, int 
             }
         ab = 0;
         aa = 0;
-        for (int q = tid; q < c; q += RB_LT) {
-            const u64 k = sk[q];
+        each([&](u64 k, int q) {
             const long long A = 2 * O + rk_lower(sk, 0, c, k) + rk_upper(sk, 0, c, k) - n;
-            ab += A * (long long)sv[q];
+            ab += A * (long long)bv[q];
             aa += A * A;
-        }
+        });
     }
     const long long sab = rb_block_sum64<RB_LT>(ab, ws);
     const long long saa = rb_block_sum64<RB_LT>(aa, ws);
