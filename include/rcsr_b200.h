@@ -157,7 +157,8 @@ int rc_fit_kernel_info(int kmax, int *threads, int *smem_bytes, int *max_constan
 
 /* eval.cu:4270 rc_rank_score_batch: exact 128-bit rank sums per segment
    (seg = set * ntrials + trial): out[4*seg] = (ab_hi, ab_lo, aa_hi, aa_lo);
-   out_bb = (hi, lo) of the target's sum B^2. */
+   out_bb = (hi, lo) of the target's sum B^2. A segment whose status is not 0
+   has no ranks: its four words are zeros. */
 float rc_rank_score_batch(void *ctx, const unsigned int *prog, const unsigned int *off,
                           const int *pcount, int nsets, int ntrials, int kmax, const double *c0,
                           unsigned long long *out, int *out_status, unsigned long long *out_bb);
@@ -236,7 +237,8 @@ int rc_fit_budgets(void *ctx, int *out_kb);
    call on the context), out[4 * cand + k]: k = 0 f32 assembly sweeps, 1 f32
    objective sweeps, 2 f64 assembly sweeps (implicit: Jacobian sweeps), 3 f64
    objective sweeps (implicit: cost sweeps); the correlation arm's assembly
-   and trial sweeps count as 0 and 1. Returns 0, or -1 when the last call was
+   and trial sweeps count as 0 and 1. A trial's objective sweep counts although
+   it ends early once its sum exceeds the objective to beat. Returns 0, or -1 when the last call was
    not a fit of nprog candidates. No counterpart in the reference ABI. */
 int rc_last_fit_sweeps(void *ctx, int nprog, int *out);
 /* Per-row gradients of fit-record programs from the fused adjoint sweep, over

@@ -20,9 +20,9 @@
  * bit-identical to the CPU's `RankTarget::sums` (metrics.rs:1359-1416) for
  * the same predictions.
  *
- * Order statistics sort the bit patterns of |pred - y| (non-negative, so
- * they order like the values) and pick the median or average the
- * interquartile window by rank. The maximum scan is an integer max over the
+ * Order statistics rank the bit patterns of |pred - y| (non-negative, so
+ * they order like the values): the median is selected between two sampled
+ * keys around the middle, the interquartile window is sorted and averaged. The maximum scan is an integer max over the
  * same patterns with the lowest attaining row, plus the per-row feasibility
  * interval of a level along one constant (reverse sweep for dr/dc).
  */
