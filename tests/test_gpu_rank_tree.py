@@ -1,14 +1,16 @@
 """The bucketed rank sums against the radix sort's where the splitters' search
 tree changes its depth: row counts that give one splitter fewer, as many and
 one more than a power of two, and columns of one to nine values (as few
-splitters, all of them with equality buckets). Whole numbers: equal."""
+splitters, all of them with equality buckets), and samples of 1 to 16 keys a
+sorting thread. Whole numbers: equal."""
 import numpy as np
 import pytest
 
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n", [8193, 14336, 16384, 16385, 32769, 34817, 131073, 2097152, 2099201])
+@pytest.mark.parametrize("n", [8193, 14336, 16384, 16385, 32769, 34817, 131073, 300007, 700001, 2097152,
+                               2099201])
 def test_bucketed_sums_equal_the_sorted_ones(pkg, E, n):
     rng = np.random.Generator(np.random.PCG64(n))
     cols = np.stack([rng.standard_normal(n)] +
