@@ -2415,21 +2415,25 @@ struct FitChain {
     SweepLaunch sw[2];
     int nk = 0;
     int ncand = 0;
+    bool fits = true; /* the device grants every sweep its shared memory */
 };
 
-SweepLaunch sweep_shape(RcCtx *c, const void *fn, int threads, size_t smem, long long items)
+void add_sweep(RcCtx *c, FitChain &ch, const void *fn, int threads, size_t smem, long long items)
 {
     /* persistent grids take their items from work counters, so a grid no
        larger than the items that can exist answers the same and launches no
        idle blocks */
-    SweepLaunch s;
+    SweepLaunch &s = ch.sw[ch.nk++];
     s.fn = fn;
     s.smem = smem;
-    rc_raise_smem(fn, smem);
+    if (rc_raise_smem(fn, smem) != 0) {
+        fprintf(stderr, "fit: the batch's deepest program needs %zu bytes of shared memory a block, "
+                        "more than the device has\n", smem);
+        ch.fits = false;
+    }
     s.grid = (int)std::max<long long>(
         1, std::min<long long>((long long)c->sm_count * occupancy(fn, threads, smem), items));
     s.threads = threads;
-    return s;
 }
 
 /* Input-mode translation (fi_decode with `inputs`) of every valid candidate:
@@ -2527,14 +2531,16 @@ int ijac_split(RcCtx *c, const FitPrep &b, int Wmax)
    waves) 14.2 -> 13.2 ms. It fits fewer threads an SM (512 against 640 of
    A = 128), so full waves prefer one group: the classes of A = 128 take
    grouped blocks below one wave (200 short candidates x 60,000 rows: 6.5 ms
-   with one group, 7.7 grouped). */
+   with one group, 7.7 grouped). A block has fewer groups, down to one of 128
+   threads, where a deep program's spill slots (8 KB each for the objective of
+   512 threads) would not fit. */
 #define FT_SMEM_MAX ((size_t)226 * 1024)
 #define FT_GROUP_T 512
 #define FT_GROUP_WAVES 4
 
 /* The chain of the candidates `ids` (indexes into the batch; `cls` their
    assembly class): the batch's arguments `a` with the chain's launch shapes.
-   `small`: every kind of a step in one launch of 128-thread blocks. */
+   `small`: every kind of a step in one launch of grouped blocks. */
 FitChain make_chain(RcCtx *c, const FitArgs &a, const FitPrep &b, const XPrep &xp,
                     const std::vector<int> &ids, int cls, bool small)
 {
@@ -2593,8 +2599,8 @@ FitChain make_chain(RcCtx *c, const FitArgs &a, const FitPrep &b, const XPrep &x
         auto jsm = [&](int g) { return ft_ijac_smem(mmax, ninternal, ch.a.Wmax, g); };
         auto csm = [&](int g) { return ft_icost_smem(xmaxins, xslots, xtape, a.v, g); };
         const int gj = groups(jac, jsm), gc = groups(cost, csm);
-        ch.sw[ch.nk++] = sweep_shape(c, jac, gj * FT_ITHREADS, jsm(gj), items);
-        ch.sw[ch.nk++] = sweep_shape(c, cost, gc * FT_ITHREADS, csm(gc), items);
+        add_sweep(c, ch, jac, gj * FT_ITHREADS, jsm(gj), items);
+        add_sweep(c, ch, cost, gc * FT_ITHREADS, csm(gc), items);
         return ch;
     }
     auto kernels = [&](auto grp) {
@@ -2621,34 +2627,39 @@ FitChain make_chain(RcCtx *c, const FitArgs &a, const FitPrep &b, const XPrep &x
                               occupancy(fns.asm_fn, T, sa);
     }
     int TL = FT_LOSS_T;
+    auto loss_smem = [&](int t) { return ft_sweep4_smem(FOP_LOSS32, maxins, slots, region, t); };
     if (grouped) {
         /* several chunks of a tile at once (a tile's latency bounds these
            fits): blocks of 512 threads with the regions that fit */
         const auto gf = kernels(std::true_type{});
         fns.asm_fn = gf.asm_fn;
         fns.loss_fn = gf.loss_fn;
+        auto regions = [&](int t) {
+            size_t want = 0;
+            for (int i : ids)
+                if (b.valid[i]) {
+                    const int4 f = b.finfo[i];
+                    const int A = f.z & 0xffff;
+                    want = std::max(want, (size_t)(t / A) *
+                                              (ft_asm_region(A, f.w & 0xffff, f.w >> 16,
+                                                             8 * ((b.pcount[i] + 1 + extra + 7) / 8)) +
+                                               16 * (size_t)A));
+                }
+            const size_t fixed = ft_sweep4_smem(FOP_ASM32, maxins, slots, 0, t);
+            return std::max(region + 16 * 128, std::min(want, FT_SMEM_MAX - fixed));
+        };
         T = FT_GROUP_T;
-        size_t want = 0;
-        for (int i : ids)
-            if (b.valid[i]) {
-                const int4 f = b.finfo[i];
-                const int A = f.z & 0xffff;
-                want = std::max(want, (size_t)(T / A) *
-                                          (ft_asm_region(A, f.w & 0xffff, f.w >> 16,
-                                                         8 * ((b.pcount[i] + 1 + extra + 7) / 8)) +
-                                           16 * (size_t)A));
-            }
-        const size_t fixed = ft_sweep4_smem(FOP_ASM32, maxins, slots, 0, T);
-        ch.a.asm_region = std::max(region + 16 * 128, std::min(want, FT_SMEM_MAX - fixed));
-        sa = fixed + ch.a.asm_region;
+        while (small && T > FT_LOSS_T && loss_smem(T) > FT_SMEM_MAX) T /= 2;
+        ch.a.asm_region = regions(T);
+        sa = ft_sweep4_smem(FOP_ASM32, maxins, slots, ch.a.asm_region, T);
         TL = extra ? FT_LOSS_T : FT_GROUP_T;
+        while (TL > FT_LOSS_T && loss_smem(TL) > FT_SMEM_MAX) TL /= 2;
     }
-    const size_t sl = ft_sweep4_smem(FOP_LOSS32, maxins, slots, region, small ? T : TL);
     if (small) {
-        ch.sw[ch.nk++] = sweep_shape(c, all_fn, T, std::max(sa, sl), items);
+        add_sweep(c, ch, all_fn, T, std::max(sa, loss_smem(T)), items);
     } else {
-        ch.sw[ch.nk++] = sweep_shape(c, fns.asm_fn, T, sa, items);
-        ch.sw[ch.nk++] = sweep_shape(c, fns.loss_fn, TL, sl, items);
+        add_sweep(c, ch, fns.asm_fn, T, sa, items);
+        add_sweep(c, ch, fns.loss_fn, TL, loss_smem(TL), items);
     }
     return ch;
 }
@@ -2899,6 +2910,7 @@ float fit_run(RcCtx *c, const unsigned int *prog, const unsigned int *off, const
             ch.a.lists = a.lists + g * 2 * FOP_COUNT * (size_t)nprog;
             ch.a.counts = a.counts + g * 2 * FOP_COUNT;
             ch.a.work = a.work + g * 2 * FOP_COUNT;
+            if (!ch.fits) return -1.0f;
             chains.push_back(ch);
         }
     const size_t qbytes = q_end - o_counts;
@@ -2937,6 +2949,8 @@ float fit_run(RcCtx *c, const unsigned int *prog, const unsigned int *off, const
             const bool tiny = ntiles <= c->sm_count * FT_SMALL_ITEMS_PER_SM;
             const std::vector<FitChain> own{
                 make_chain(c, one, b, xp, std::vector<int>(1, i), b.finfo[i].z >> 16, tiny)};
+            ok = own[0].fits;
+            if (!ok) break;
             c->launches += enqueue_fit(c, c->s, one, steps, own, qbytes);
             ok = cudaGetLastError() == cudaSuccess;
         }
