@@ -45,8 +45,12 @@ typedef unsigned long long u64;
 #define RK_T 256                  /* key threads */
 /* Rows per thread of the key sweeps. They are bound by issue (80 % of the
    cycles with two rows), and four halve the decoding a row pays: rank sums of
-   32 x 2,097,152 rows 4.55 -> 4.31 ms, medians of 33 x 300,007 0.65 -> 0.55. */
+   32 x 2,097,152 rows 4.55 -> 4.31 ms, medians of 33 x 300,007 0.65 -> 0.55.
+   A spill slot of a block takes RK_T * 8 bytes a row, so a batch whose deepest
+   program does not fit at RK_NR rows (28 slots and more) is swept at
+   RK_NR_DEEP; the keys do not depend on it. */
 #define RK_NR 4
+#define RK_NR_DEEP 2
 #define RK_TILE 8192              /* rows per key block */
 #define RK_WAVE_BYTES ((size_t)3 << 30)
 #define RS_PASSES 8               /* 8-bit digits of a u64 key */
@@ -114,7 +118,7 @@ __device__ __forceinline__ void rs_count_keys(const u64 *src, long long r0, long
 
 /* Keys of segments [seg0, seg0 + gridDim.x / tiles) over all rows: the f64
    forward sweep of the segment's candidate at its constants
-   (c0[seg * kmax + slot]), RK_NR rows per thread. RK_RANK keys the
+   (c0[seg * kmax + slot]), NR rows per thread. RK_RANK keys the
    prediction; RK_ABS keys |pred - y| and flags a row whose prediction is
    not finite or exceeds 1e30 (eval.cu:4388-4418). A non-finite key marks
    the segment's status 2. The block then counts the eight digits of the
@@ -124,7 +128,7 @@ __device__ __forceinline__ void rs_count_keys(const u64 *src, long long r0, long
    keys are not read) is left: blocks take the segments of one tile after
    another, so a failure is known early. */
 static_assert(RK_T == RS_T, "the digit count runs on the key kernel's blocks");
-template <int MODE>
+template <int MODE, int NR>
 __global__ void __launch_bounds__(RK_T) rk_keys(const FOp *fins, const int *fins_off,
                                                 const int4 *finfo, const int *valid,
                                                 const double *c0, int kmax, const double *cols,
@@ -134,7 +138,7 @@ __global__ void __launch_bounds__(RK_T) rk_keys(const FOp *fins, const int *fins
                                                 int *status)
 {
     __shared__ unsigned int cnt[RS_PASSES][256];
-    using V4 = FiV<double, RK_NR>::V4;
+    using V4 = typename FiV<double, NR>::V4;
     extern __shared__ __align__(16) unsigned char sm[];
     FOp *ins = reinterpret_cast<FOp *>(sm);
     double *cv = reinterpret_cast<double *>(sm + 8 * (size_t)((maxins + 1) & ~1));
@@ -164,14 +168,14 @@ __global__ void __launch_bounds__(RK_T) rk_keys(const FOp *fins, const int *fins
     u64 *kseg = keys + (size_t)ls * n;
     unsigned int *rseg = rows ? rows + (size_t)ls * n : nullptr;
     bool bad = !ok;
-    for (int row = r0 + RK_NR * tid; row < r1 && (count || !bad); row += RK_NR * RK_T) {
-        double pr[RK_NR];
+    for (int row = r0 + NR * tid; row < r1 && (count || !bad); row += NR * RK_T) {
+        double pr[NR];
 #pragma unroll
-        for (int i = 0; i < RK_NR; ++i) pr[i] = CUDART_NAN;
+        for (int i = 0; i < NR; ++i) pr[i] = CUDART_NAN;
         if (ok)
-            fi_forward<double, RK_NR, false>(ins, cv, cols + row, npad, stk + tid, nullptr, RK_T, pr);
+            fi_forward<double, NR, false>(ins, cv, cols + row, npad, stk + tid, nullptr, RK_T, pr);
 #pragma unroll
-        for (int i = 0; i < RK_NR; ++i) {
+        for (int i = 0; i < NR; ++i) {
             const int rr = row + i;
             if (rr >= r1) continue;
             u64 k;
@@ -1357,6 +1361,7 @@ __global__ void __launch_bounds__(OS_SEL_T) os_bracket(const u64 *samp, int all,
 /* The key pass of the selection (the keys and failures of rk_keys<RK_ABS>):
    below[segment] += keys under the bracket, the keys inside appended to
    list[segment][...] (cnt of them, in any order). */
+template <int NR>
 __global__ void __launch_bounds__(RK_T) os_keys(const FOp *fins, const int *fins_off,
                                                 const int4 *finfo, const int *valid,
                                                 const double *c0, int kmax, const double *cols,
@@ -1365,7 +1370,7 @@ __global__ void __launch_bounds__(RK_T) os_keys(const FOp *fins, const int *fins
                                                 const u64 *bracket, u64 *list, unsigned *cnt,
                                                 unsigned *below, int *status)
 {
-    using V4 = FiV<double, RK_NR>::V4;
+    using V4 = typename FiV<double, NR>::V4;
     extern __shared__ __align__(16) unsigned char sm[];
     FOp *ins = reinterpret_cast<FOp *>(sm);
     double *cv = reinterpret_cast<double *>(sm + 8 * (size_t)((maxins + 1) & ~1));
@@ -1392,14 +1397,14 @@ __global__ void __launch_bounds__(RK_T) os_keys(const FOp *fins, const int *fins
     bool bad = false;
     /* every lane takes every step: rows past r1 (below n rounded up to a
        block's rows, which the columns hold) count for nothing */
-    for (int base = r0; base < r1; base += RK_NR * RK_T) {
-        const int row = base + RK_NR * tid;
-        double pr[RK_NR];
-        fi_forward<double, RK_NR, false>(ins, cv, cols + row, npad, stk + tid, nullptr, RK_T, pr);
-        u64 k[RK_NR];
-        bool in[RK_NR];
+    for (int base = r0; base < r1; base += NR * RK_T) {
+        const int row = base + NR * tid;
+        double pr[NR];
+        fi_forward<double, NR, false>(ins, cv, cols + row, npad, stk + tid, nullptr, RK_T, pr);
+        u64 k[NR];
+        bool in[NR];
 #pragma unroll
-        for (int i = 0; i < RK_NR; ++i) {
+        for (int i = 0; i < NR; ++i) {
             const int rr = row + i;
             in[i] = false;
             k[i] = 0;
@@ -1413,9 +1418,9 @@ __global__ void __launch_bounds__(RK_T) os_keys(const FOp *fins, const int *fins
             under += k[i] < lo;
             in[i] = k[i] >= lo && k[i] <= hi;
         }
-        unsigned m[RK_NR], all = 0;
+        unsigned m[NR], all = 0;
 #pragma unroll
-        for (int i = 0; i < RK_NR; ++i) {
+        for (int i = 0; i < NR; ++i) {
             m[i] = __ballot_sync(0xffffffffu, in[i]);
             all += __popc(m[i]);
         }
@@ -1424,7 +1429,7 @@ __global__ void __launch_bounds__(RK_T) os_keys(const FOp *fins, const int *fins
             if (lane == 0) at = atomicAdd(&cnt[ls], all);
             at = __shfl_sync(0xffffffffu, at, 0);
 #pragma unroll
-            for (int i = 0; i < RK_NR; ++i) {
+            for (int i = 0; i < NR; ++i) {
                 if (in[i]) out[at + __popc(m[i] & ((1u << lane) - 1u))] = k[i];
                 at += __popc(m[i]);
             }
@@ -1787,10 +1792,22 @@ void stat_copy(RcCtx *c, const int *pcount, int nsets, int nsegs, int kmax, cons
     cudaMemcpyAsync(c->dev, h, sp.in_end, cudaMemcpyHostToDevice, c->s);
 }
 
-size_t key_smem(const StatPrep &sp)
+/* Shared memory of a key sweep of `rows` rows per thread. */
+size_t key_smem(const StatPrep &sp, int rows)
 {
     return 8 * (size_t)((sp.b.fmaxins + 1) & ~1) + 8 * FT_MAX_CONST +
-           8 * RK_NR * (size_t)(sp.b.fslots > 0 ? sp.b.fslots : 1) * RK_T;
+           8 * rows * (size_t)(sp.b.fslots > 0 ? sp.b.fslots : 1) * RK_T;
+}
+
+/* The key kernel of a batch (`wide`: RK_NR rows per thread, `deep`:
+   RK_NR_DEEP) and its shared memory, or null when neither fits. */
+template <typename F>
+F *key_kernel(const StatPrep &sp, F *wide, F *deep, size_t *smem)
+{
+    *smem = key_smem(sp, RK_NR);
+    if (rc_raise_smem((const void *)wide, *smem) == 0) return wide;
+    *smem = key_smem(sp, RK_NR_DEEP);
+    return rc_raise_smem((const void *)deep, *smem) == 0 ? deep : nullptr;
 }
 
 /* Segments per wave so that a wave's sort buffers stay within the budget. */
@@ -1911,9 +1928,11 @@ float rc_rank_score_batch(void *ctx, const unsigned int *prog, const unsigned in
     cudaMemsetAsync(d_status, 0, sizeof(int) * nsegs, c->s);
     cudaMemsetAsync(d_ovf, 0, sizeof(int) * nsegs, c->s);
     cudaMemsetAsync(d_abort, 0, sizeof(int), c->s);
-    const size_t smem = key_smem(sp);
-    if (rc_raise_smem((const void *)rk_keys<RK_RANK>, smem) != 0) return -1.0f;
-    if (m > 0 && (rc_raise_smem((const void *)rb_sample<RK_RANK>, smem) != 0 ||
+    size_t smem = 0;
+    const size_t sample_smem = key_smem(sp, 2);
+    const auto keys = key_kernel(sp, rk_keys<RK_RANK, RK_NR>, rk_keys<RK_RANK, RK_NR_DEEP>, &smem);
+    if (!keys) return -1.0f;
+    if (m > 0 && (rc_raise_smem((const void *)rb_sample<RK_RANK>, sample_smem) != 0 ||
                   rc_raise_smem((const void *)rb_splitters, sizeof(u64) * RB_MAXS) != 0 ||
                   rc_raise_smem((const void *)rb_local, rb_local_smem()) != 0))
         return -1.0f;
@@ -1930,7 +1949,7 @@ float rc_rank_score_batch(void *ctx, const unsigned int *prog, const unsigned in
         __int128 *part = nullptr;
         const RsBuffers b = rs_carve(dev, &wc, ns, n, true, &part);
         cudaMemsetAsync(b.count, 0, sizeof(unsigned int) * RS_PASSES * 256 * (size_t)ns, c->s);
-        rk_keys<RK_RANK><<<(unsigned)ns * ktiles, RK_T, smem, c->s>>>(
+        keys<<<(unsigned)ns * ktiles, RK_T, smem, c->s>>>(
             d_fins, d_finsoff, d_finfo, d_valid, d_c0, kmax, c->d_cols64, c->d_y64, c->npad, n,
             ntrials, s0, ktiles, sp.b.fmaxins, b.ka, b.va, b.count, d_status);
         c->launches += 3 + rs_sort<true>(b, ns, n, d_abort, c->s, true);
@@ -1949,7 +1968,7 @@ float rc_rank_score_batch(void *ctx, const unsigned int *prog, const unsigned in
             int P2 = RB_ST;
             while (P2 < S) P2 <<= 1;
             const int sblocks = (S / 2 + RK_T - 1) / RK_T;
-            rb_sample<RK_RANK><<<(unsigned)ns * sblocks, RK_T, smem, c->s>>>(
+            rb_sample<RK_RANK><<<(unsigned)ns * sblocks, RK_T, sample_smem, c->s>>>(
                 d_fins, d_finsoff, d_finfo, d_valid, d_c0, kmax, c->d_cols64, c->d_y64, c->npad, n, ntrials,
                 s0, sblocks, S, sp.b.fmaxins, r.samp);
             rb_splitters<<<ns, RB_ST, sizeof(u64) * P2, c->s>>>(r.samp, S, P2, m, r.spl, r.nspl);
@@ -1957,7 +1976,7 @@ float rc_rank_score_batch(void *ctx, const unsigned int *prog, const unsigned in
         } else {
             cudaMemsetAsync(r.nspl, 0, sizeof(int) * ns, c->s);
         }
-        rk_keys<RK_RANK><<<(unsigned)ns * ktiles, RK_T, smem, c->s>>>(
+        keys<<<(unsigned)ns * ktiles, RK_T, smem, c->s>>>(
             d_fins, d_finsoff, d_finfo, d_valid, d_c0, kmax, c->d_cols64, c->d_y64, c->npad, n,
             ntrials, s0, ktiles, sp.b.fmaxins, r.keys, nullptr, nullptr, d_status);
         const int ctiles = (n + RB_CT - 1) / RB_CT;
@@ -2077,10 +2096,12 @@ float rc_order_stat_score_batch(void *ctx, const unsigned int *prog, const unsig
     int *d_abort = reinterpret_cast<int *>(dev + o_abort);
     double *d_val = reinterpret_cast<double *>(dev + o_val);
     cudaMemsetAsync(d_status, 0, io_end - o_status, c->s);
-    const size_t smem = key_smem(sp);
-    if (rc_raise_smem((const void *)rk_keys<RK_ABS>, smem) != 0 ||
-        rc_raise_smem((const void *)rb_sample<RK_ABS>, smem) != 0 ||
-        rc_raise_smem((const void *)os_keys, smem) != 0)
+    size_t smem = 0, select_smem = 0;
+    const size_t sample_smem = key_smem(sp, 2);
+    const auto keys = key_kernel(sp, rk_keys<RK_ABS, RK_NR>, rk_keys<RK_ABS, RK_NR_DEEP>, &smem);
+    const auto select_keys = key_kernel(sp, os_keys<RK_NR>, os_keys<RK_NR_DEEP>, &select_smem);
+    if (!keys || !select_keys ||
+        rc_raise_smem((const void *)rb_sample<RK_ABS>, sample_smem) != 0)
         return -1.0f;
     const int ktiles = (n + RK_TILE - 1) / RK_TILE;
     const FOp *d_fins = reinterpret_cast<const FOp *>(dev + sp.o_fins);
@@ -2093,7 +2114,7 @@ float rc_order_stat_score_batch(void *ctx, const unsigned int *prog, const unsig
         __int128 *part = nullptr;
         const RsBuffers b = rs_carve(dev, &wc, ns, n, false, &part);
         cudaMemsetAsync(b.count, 0, sizeof(unsigned int) * RS_PASSES * 256 * (size_t)ns, c->s);
-        rk_keys<RK_ABS><<<(unsigned)ns * ktiles, RK_T, smem, c->s>>>(
+        keys<<<(unsigned)ns * ktiles, RK_T, smem, c->s>>>(
             d_fins, d_finsoff, d_finfo, d_valid, d_c0, kmax, c->d_cols64, c->d_y64, c->npad, n,
             ntrials, s0, ktiles, sp.b.fmaxins, b.ka, nullptr, b.count, d_status);
         c->launches += 2 + rs_sort<false>(b, ns, n, d_abort, c->s, true);
@@ -2109,13 +2130,13 @@ float rc_order_stat_score_batch(void *ctx, const unsigned int *prog, const unsig
         const int all = n <= OS_LIST_ALL ? 1 : 0;
         if (!all) {
             const int sblocks = (OS_S / 2 + RK_T - 1) / RK_T;
-            rb_sample<RK_ABS><<<(unsigned)ns * sblocks, RK_T, smem, c->s>>>(
+            rb_sample<RK_ABS><<<(unsigned)ns * sblocks, RK_T, sample_smem, c->s>>>(
                 d_fins, d_finsoff, d_finfo, d_valid, d_c0, kmax, c->d_cols64, c->d_y64, c->npad, n,
                 ntrials, s0, sblocks, OS_S, sp.b.fmaxins, samp);
             c->launches += 1;
         }
         os_bracket<<<ns, OS_SEL_T, 0, c->s>>>(samp, all, bracket);
-        os_keys<<<(unsigned)ns * ktiles, RK_T, smem, c->s>>>(
+        select_keys<<<(unsigned)ns * ktiles, RK_T, select_smem, c->s>>>(
             d_fins, d_finsoff, d_finfo, d_valid, d_c0, kmax, c->d_cols64, c->d_y64, c->npad, n,
             ntrials, s0, ktiles, sp.b.fmaxins, bracket, list, cnt, cnt + ns, d_status);
         os_median<<<ns, OS_SEL_T, 0, c->s>>>(list, cnt, cnt + ns, n, s0, d_status, d_val, d_redo);
