@@ -57,3 +57,31 @@ def test_deep_statistics(pkg, E, slots, n, radix):
                 s[lo:hi].sum() / (hi - lo)
             assert val[k] == want, (slots, n, k, what)
     ev.close()
+
+
+@pytest.mark.parametrize("n", [9001, 70003])
+def test_wide_batches(pkg, E, n):
+    """More than eight key blocks an SM: a sort's keys two rows a thread."""
+    rng = np.random.Generator(np.random.PCG64(n))
+    x = rng.integers(-4096, 4097, (3, n)) / 8.0
+    y = rng.integers(-4096, 4097, n) / 8.0
+    ev = pkg.GpuEvaluator(x.astype(np.float32).reshape(-1), n, 3, y.astype(np.float32))
+    ev.set_fit_data(x.reshape(-1), y)
+    trees = [E.input(1), _deep(E, 5), E.node(E.LOG, [E.constant(-1.0)])]
+    preds = [x[1], sum(x[k % 3] for k in range(4)) + 2.0 * x[0], None]
+    reps = 1 + 8 * 160 // (3 * ((n + 8191) // 8192))
+    plans = [pkg.gpu_fit_plan(t, allow_no_constants=True) for t in trees] * reps
+    prog, off, pcount, c0, _, kmax = pkg.pack_plans(plans)
+    lo, hi = n // 4, 3 * n // 4
+    val, status, _ = ev.order_stat(prog, off, pcount, c0, kmax, 1)
+    assert status.tolist() == [0, 0, 2] * reps
+    for k in (0, 1):
+        s = np.sort(np.abs(preds[k] - y))
+        assert (val[k::3] == s[lo:hi].sum() / (hi - lo)).all(), (n, k)
+    ev.rank_tuning(-1, 0)
+    sums, status, _, _ = ev.rank_sums(prog, off, pcount, c0, kmax)
+    b = _centred(y)
+    for k in (0, 1):
+        a = _centred(preds[k])
+        assert set(sums[k::3]) == {(int(a @ b), int(a @ a))}, (n, k)
+    ev.close()

@@ -46,9 +46,9 @@ typedef unsigned long long u64;
 /* Rows per thread of the key sweeps. They are bound by issue (80 % of the
    cycles with two rows), and four halve the decoding a row pays: rank sums of
    32 x 2,097,152 rows 4.55 -> 4.31 ms, medians of 33 x 300,007 0.65 -> 0.55.
-   A spill slot of a block takes RK_T * 8 bytes a row, so a batch whose deepest
-   program does not fit at RK_NR rows (28 slots and more) is swept at
-   RK_NR_DEEP; the keys do not depend on it. */
+   A spill slot of a block takes RK_T * 8 bytes a row, so a batch of deep
+   programs is swept at RK_NR_DEEP rows (key_kernel); the keys do not depend
+   on it. */
 #define RK_NR 4
 #define RK_NR_DEEP 2
 #define RK_TILE 8192              /* rows per key block */
@@ -1799,15 +1799,41 @@ size_t key_smem(const StatPrep &sp, int rows)
            8 * rows * (size_t)(sp.b.fslots > 0 ? sp.b.fslots : 1) * RK_T;
 }
 
-/* The key kernel of a batch (`wide`: RK_NR rows per thread, `deep`:
-   RK_NR_DEEP) and its shared memory, or null when neither fits. */
+/* The key kernel of a batch of `blocks` blocks (`wide`: RK_NR rows per thread,
+   `deep`: RK_NR_DEEP) and its shared memory, or null when neither fits. Two
+   rows where that puts more rows in flight on an SM, or as many in two blocks
+   instead of one: 24 programs x 300,007 rows of 14 slots, rank sums 0.76 ms
+   with four rows and 0.70 with two; of 20 slots, as many rows, 0.78 and 0.75,
+   medians 0.48 and 0.43; but of 12 slots, as many rows in two blocks of four,
+   medians 0.28 and 0.31. `sorted`: the keys of a sort, whose kernel also
+   counts digits; a grid of more than RK_SORT_WIDE blocks an SM takes them two
+   rows a thread (interquartile means of 32 candidates x 1,048,576 rows
+   3.89 ms with four, 3.62 with two; of 48 x 300,007, twelve blocks an SM, 1.84
+   and 1.77; but of 64 x 10,007, one block an SM, 0.51 and 0.57, and of 24
+   shallow ones x 300,007, six, 0.73 and 0.76). */
+#define RK_SORT_WIDE 8
 template <typename F>
-F *key_kernel(const StatPrep &sp, F *wide, F *deep, size_t *smem)
+F *key_kernel(RcCtx *c, const StatPrep &sp, F *wide, F *deep, long long blocks, bool sorted,
+              size_t *smem)
 {
-    *smem = key_smem(sp, RK_NR);
-    if (rc_raise_smem((const void *)wide, *smem) == 0) return wide;
-    *smem = key_smem(sp, RK_NR_DEEP);
-    return rc_raise_smem((const void *)deep, *smem) == 0 ? deep : nullptr;
+    const size_t sw = key_smem(sp, RK_NR), sd = key_smem(sp, RK_NR_DEEP);
+    const bool fits = rc_raise_smem((const void *)wide, sw) == 0;
+    if (rc_raise_smem((const void *)deep, sd) != 0) return nullptr;
+    const long long per_sm = (blocks + c->sm_count - 1) / c->sm_count;
+    auto resident = [&](F *fn, size_t s) {
+        int b = 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, fn, RK_T, s) != cudaSuccess) {
+            cudaGetLastError();
+            b = 1;
+        }
+        return std::min<long long>(b, per_sm);
+    };
+    *smem = sd;
+    if (!fits || (sorted && per_sm > RK_SORT_WIDE)) return deep;
+    const long long bw = resident(wide, sw), rw = RK_NR * bw, rd = RK_NR_DEEP * resident(deep, sd);
+    if (rw < rd || (rw == rd && bw == 1)) return deep;
+    *smem = sw;
+    return wide;
 }
 
 /* Segments per wave so that a wave's sort buffers stay within the budget. */
@@ -1930,13 +1956,14 @@ float rc_rank_score_batch(void *ctx, const unsigned int *prog, const unsigned in
     cudaMemsetAsync(d_abort, 0, sizeof(int), c->s);
     size_t smem = 0;
     const size_t sample_smem = key_smem(sp, 2);
-    const auto keys = key_kernel(sp, rk_keys<RK_RANK, RK_NR>, rk_keys<RK_RANK, RK_NR_DEEP>, &smem);
+    const int ktiles = (n + RK_TILE - 1) / RK_TILE;
+    const auto keys = key_kernel(c, sp, rk_keys<RK_RANK, RK_NR>, rk_keys<RK_RANK, RK_NR_DEEP>,
+                                 (long long)wseg * ktiles, m == 0, &smem);
     if (!keys) return -1.0f;
     if (m > 0 && (rc_raise_smem((const void *)rb_sample<RK_RANK>, sample_smem) != 0 ||
                   rc_raise_smem((const void *)rb_splitters, sizeof(u64) * RB_MAXS) != 0 ||
                   rc_raise_smem((const void *)rb_local, rb_local_smem()) != 0))
         return -1.0f;
-    const int ktiles = (n + RK_TILE - 1) / RK_TILE;
     const int ntiles = (n + RS_TILE - 1) / RS_TILE;
     const FOp *d_fins = reinterpret_cast<const FOp *>(dev + sp.o_fins);
     const int *d_finsoff = reinterpret_cast<const int *>(dev + sp.o_finsoff);
@@ -2098,12 +2125,15 @@ float rc_order_stat_score_batch(void *ctx, const unsigned int *prog, const unsig
     cudaMemsetAsync(d_status, 0, io_end - o_status, c->s);
     size_t smem = 0, select_smem = 0;
     const size_t sample_smem = key_smem(sp, 2);
-    const auto keys = key_kernel(sp, rk_keys<RK_ABS, RK_NR>, rk_keys<RK_ABS, RK_NR_DEEP>, &smem);
-    const auto select_keys = key_kernel(sp, os_keys<RK_NR>, os_keys<RK_NR_DEEP>, &select_smem);
+    const int ktiles = (n + RK_TILE - 1) / RK_TILE;
+    const long long blocks = (long long)wseg * ktiles;
+    const auto keys = key_kernel(c, sp, rk_keys<RK_ABS, RK_NR>, rk_keys<RK_ABS, RK_NR_DEEP>, blocks,
+                                 true, &smem);
+    const auto select_keys =
+        key_kernel(c, sp, os_keys<RK_NR>, os_keys<RK_NR_DEEP>, blocks, false, &select_smem);
     if (!keys || !select_keys ||
         rc_raise_smem((const void *)rb_sample<RK_ABS>, sample_smem) != 0)
         return -1.0f;
-    const int ktiles = (n + RK_TILE - 1) / RK_TILE;
     const FOp *d_fins = reinterpret_cast<const FOp *>(dev + sp.o_fins);
     const int *d_finsoff = reinterpret_cast<const int *>(dev + sp.o_finsoff);
     const int4 *d_finfo = reinterpret_cast<const int4 *>(dev + sp.o_finfo);
