@@ -160,6 +160,8 @@ __device__ __forceinline__ bool ft_rescue(int flags, FitState &st, int rb)
     return true;
 }
 
+/* (pointers first, then an even number of ints: no padding, so that the bytes
+   of a FitArgs stand for it in the graph key) */
 struct FitArgs {
     const float *cols;
     const float *y;
@@ -168,11 +170,9 @@ struct FitArgs {
     const double *y64;
     const double *tsign64;
     const double *w;
-    int n, npad, v;
     const uint4 *rec;
     const int *node_off;
     const int *pcount;
-    int kmax;
     const double *c0;
     const int *gauge;      /* [2P] correlation gauge pair (scale, offset), -1 = none */
     const int *valid;
@@ -181,10 +181,6 @@ struct FitArgs {
     const int4 *finfo;     /* [P] forward count, reverse count, active threads | assembly
                               class << 16 | chain << 24,
                               spill slots | tape slots << 16 */
-    int fslots;            /* spill slots needed by the chain */
-    int ftape;             /* partial-tape slots needed by the batch */
-    int fmaxins;           /* longest forward + reverse list */
-    size_t asm_region;     /* assembly region of the chain */
     const int2 *fcinfo;    /* [P] cached forward count (after the reverse list),
                               first cache column */
     float *cache;          /* [columns][npad] values of constant-free subtrees */
@@ -192,11 +188,26 @@ struct FitArgs {
     const FOp *sub_fins;   /* forward lists of the cached subtrees */
     const int *sub_off;    /* [nsub + 1] */
     const int *sub_col;    /* [nsub] */
-    int nsub;
-    int sub_slots, sub_maxins;
     const FOp *xfins;      /* implicit metric: input-mode lists [forward | reverse] */
     const int *xfins_off;  /* [P + 1] */
     const int4 *xinfo;     /* forward count, reverse count, spill slots, tape slots */
+    FitState *state;
+    double *part;          /* [P][ntiles][FT_PART_STRIDE] */
+    double *run;           /* [P] objective of the trial sweep so far (ft_trial_lost) */
+    int *lists;            /* the chain's [2][FOP_COUNT][P] */
+    int *counts;           /* the chain's [2][FOP_COUNT] candidates queued per kind */
+    int *work;             /* the chain's [2][FOP_COUNT] persistent-grid work counters */
+    double *outc;
+    double *outsse;
+    int *outstatus;
+    int n, npad, v;
+    int kmax;
+    int fslots;            /* spill slots needed by the chain */
+    int ftape;             /* partial-tape slots needed by the batch */
+    int fmaxins;           /* longest forward + reverse list */
+    unsigned asm_region;   /* assembly region of the chain, bytes */
+    int nsub;
+    int sub_slots, sub_maxins;
     int xmaxins, xslots, xtape;
     int iters, metric, flags;
     int ntiles;
@@ -204,16 +215,8 @@ struct FitArgs {
     int ijac_tape;         /* internal-node tape slots of the Jacobian launch */
     int Wmax;
     int nprog;
-    FitState *state;
-    double *part;      /* [P][ntiles][FT_PART_STRIDE] */
-    double *run;       /* [P] objective of the trial sweep so far (ft_trial_lost) */
-    int *lists;        /* the chain's [2][FOP_COUNT][P] */
-    int *counts;       /* the chain's [2][FOP_COUNT] candidates queued per kind */
-    int *work;         /* the chain's [2][FOP_COUNT] persistent-grid work counters */
-    double *outc;
-    double *outsse;
-    int *outstatus;
 };
+static_assert(std::has_unique_object_representations_v<FitArgs>, "the graph key holds its bytes");
 
 /* ---- sweep kernels ------------------------------------------------------ */
 
@@ -1052,7 +1055,7 @@ __device__ void ft_sweep_item(const FitArgs &a, unsigned char *sm, int cand, int
     const int tid = threadIdx.x, T = blockDim.x;
     const int slots = a.fslots > 0 ? a.fslots : 1;
     double *red = reinterpret_cast<double *>(
-        region + (ft_op_assembles(OPK) ? a.asm_region : 16 * (size_t)slots * T));
+        region + (ft_op_assembles(OPK) ? (size_t)a.asm_region : 16 * (size_t)slots * T));
     const FitState *st = a.state + cand;
     const int ib = a.fins_off[cand];
     const int4 info = a.finfo[cand];
@@ -2571,7 +2574,7 @@ FitChain make_chain(RcCtx *c, const FitArgs &a, const FitPrep &b, const XPrep &x
     }
     ch.a.fslots = slots;
     ch.a.fmaxins = maxins;
-    ch.a.asm_region = region;
+    ch.a.asm_region = (unsigned)region;
     ch.a.mmax = mmax;
     ch.a.ijac_tape = ninternal;
     ch.a.Wmax = 4 * ((pmax + 1 + 3) / 4);
@@ -2650,7 +2653,7 @@ FitChain make_chain(RcCtx *c, const FitArgs &a, const FitPrep &b, const XPrep &x
         };
         T = FT_GROUP_T;
         while (small && T > FT_LOSS_T && loss_smem(T) > FT_SMEM_MAX) T /= 2;
-        ch.a.asm_region = regions(T);
+        ch.a.asm_region = (unsigned)regions(T);
         sa = ft_sweep4_smem(FOP_ASM32, maxins, slots, ch.a.asm_region, T);
         TL = extra ? FT_LOSS_T : FT_GROUP_T;
         while (TL > FT_LOSS_T && loss_smem(TL) > FT_SMEM_MAX) TL /= 2;
@@ -2955,22 +2958,19 @@ float fit_run(RcCtx *c, const unsigned int *prog, const unsigned int *off, const
             ok = cudaGetLastError() == cudaSuccess;
         }
     } else {
-        std::string key;
-        auto add = [&](unsigned long long v) { key += std::to_string(v) + "|"; };
-        add((unsigned long long)(uintptr_t)dev);
-        for (int v : {nprog, kmax, ntiles, iters, metric, flags, steps, b.ftape, b.ncache, a.nsub,
-                      b.sub_slots, b.sub_maxins, use64 ? 1 : 0})
-            add((unsigned long long)(unsigned)v);
-        add(io_end);
+        /* all that the nodes of the graph hold: the batch's and the chains'
+           arguments (every pointer into the workspace and to the context's
+           data among them) and the launches */
+        std::string key(reinterpret_cast<const char *>(&a), sizeof(a));
+        auto add = [&](const auto &v) { key.append(reinterpret_cast<const char *>(&v), sizeof(v)); };
         for (const FitChain &ch : chains) {
-            for (int v : {ch.ncand, ch.nk, ch.a.fslots, ch.a.fmaxins, ch.a.mmax, ch.a.Wmax,
-                          ch.a.ijac_tape, ch.a.xslots, ch.a.xtape, ch.a.xmaxins})
-                add((unsigned long long)(unsigned)v);
-            add(ch.a.asm_region);
+            add(ch.a);
+            add(ch.ncand);
             for (int w = 0; w < ch.nk; ++w) {
-                add((unsigned long long)(uintptr_t)ch.sw[w].fn);
+                add(ch.sw[w].fn);
                 add(ch.sw[w].smem);
-                add((unsigned long long)ch.sw[w].grid);
+                add(ch.sw[w].grid);
+                add(ch.sw[w].threads);
             }
         }
         const bool replay = c->fit_graph && c->fit_graph_key == key;
