@@ -682,11 +682,17 @@ __global__ void __launch_bounds__(RS_T) rk_runs(const u64 *ka, const u64 *kb,
 }
 
 /* One block per segment: the tile partials summed into two 128-bit values,
-   written as (hi, lo) u64 pairs at out[4 * seg ...] (two's complement). */
-__global__ void __launch_bounds__(RS_T) rk_final(const __int128 *part, int ntiles, u64 *out)
+   written as (hi, lo) u64 pairs at out[4 * seg ...] (two's complement); a
+   segment of a failed candidate has no ranks: zeros. */
+__global__ void __launch_bounds__(RS_T) rk_final(const __int128 *part, int ntiles,
+                                                 const int *status, u64 *out)
 {
     __shared__ __int128 red[RS_T];
     const int seg = blockIdx.x, tid = threadIdx.x;
+    if (status && status[seg]) {
+        if (tid < 4) out[(size_t)seg * 4 + tid] = 0ULL;
+        return;
+    }
     __int128 ab = 0, aa = 0;
     for (int t = tid; t < ntiles; t += RS_T) {
         ab += part[((size_t)seg * ntiles + t) * 2 + 0];
@@ -1748,7 +1754,7 @@ int rk_prepare(RcCtx *c)
     c->launches += 3 + rs_sort<true>(b, 1, n, d_abort, c->s, false);
     rk_runs<RK_FILL><<<ntiles, RS_T, 0, c->s>>>(b.ka, b.kb, b.va, b.vb, b.par, n, ntiles, nullptr,
                                                 c->d_rank_b, part);
-    rk_final<<<1, RS_T, 0, c->s>>>(part, ntiles, reinterpret_cast<u64 *>(c->dev + o_out));
+    rk_final<<<1, RS_T, 0, c->s>>>(part, ntiles, nullptr, reinterpret_cast<u64 *>(c->dev + o_out));
     cudaMemcpyAsync(c->host + o_out, c->dev + o_out, io_end - o_out, cudaMemcpyDeviceToHost, c->s);
     if (rc_finish(c) != 0) return -1;
     if (*reinterpret_cast<const int *>(c->host + o_abort) != 0) return -1;
@@ -1982,7 +1988,7 @@ float rc_rank_score_batch(void *ctx, const unsigned int *prog, const unsigned in
         c->launches += 3 + rs_sort<true>(b, ns, n, d_abort, c->s, true);
         rk_runs<RK_SUMS><<<(unsigned)ns * ntiles, RS_T, 0, c->s>>>(
             b.ka, b.kb, b.va, b.vb, b.par, n, ntiles, c->d_rank_b, nullptr, part);
-        rk_final<<<ns, RS_T, 0, c->s>>>(part, ntiles, d_out + 4 * (size_t)s0);
+        rk_final<<<ns, RS_T, 0, c->s>>>(part, ntiles, d_status + s0, d_out + 4 * (size_t)s0);
     };
     /* the bucketed sums of segments [s0, s0 + ns); a flagged segment is left
        to the radix sort */
