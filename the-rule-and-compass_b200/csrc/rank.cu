@@ -754,14 +754,15 @@ __device__ __forceinline__ unsigned rb_hash(unsigned a, unsigned b)
 
 /* Keys of S sample rows per segment: S / 2 row pairs, pair p at rows 2q and
    2q + 1 with q drawn by a fixed hash from the p-th of S / 2 equal strata of
-   the n / 2 pairs; the f64 sweep and the keys of rk_keys. */
+   the n / 2 pairs; the f64 sweep and the keys of rk_keys. A segment's samples
+   start `room` keys after those of the one before it. */
 template <int MODE>
 __global__ void __launch_bounds__(RK_T) rb_sample(const FOp *fins, const int *fins_off,
                                                   const int4 *finfo, const int *valid,
                                                   const double *c0, int kmax, const double *cols,
                                                   const double *y, int npad, int n, int ntrials,
-                                                  int seg0,
-                                                  int sblocks, int S, int maxins, u64 *samp)
+                                                  int seg0, int sblocks, int S, int room, int maxins,
+                                                  u64 *samp)
 {
     using V4 = FiV<double, 2>::V4;
     extern __shared__ __align__(16) unsigned char sm[];
@@ -795,7 +796,7 @@ __global__ void __launch_bounds__(RK_T) rb_sample(const FOp *fins, const int *fi
             const double r = pr[i] - y[2 * q + i];
             if (isfinite(r)) k = rk_abs_key(r);
         }
-        samp[(size_t)ls * RB_MAXS + 2 * p + i] = k;
+        samp[(size_t)ls * room + 2 * p + i] = k;
     }
 }
 
@@ -1358,7 +1359,7 @@ __global__ void __launch_bounds__(OS_SEL_T) os_bracket(const u64 *samp, int all,
         if (tid < 2) bracket[2 * ls + tid] = tid == 0 ? 0ULL : ~0ULL;
         return;
     }
-    for (int i = tid; i < OS_S; i += OS_SEL_T) s[i] = samp[(size_t)ls * RB_MAXS + i];
+    for (int i = tid; i < OS_S; i += OS_SEL_T) s[i] = samp[(size_t)ls * OS_S + i];
     __syncthreads();
     rb_sort<OS_S / RB_ST>(s);
     if (tid < 2) bracket[2 * ls + tid] = s[OS_S / 2 + (tid == 0 ? -OS_D : OS_D)];
@@ -2003,7 +2004,7 @@ float rc_rank_score_batch(void *ctx, const unsigned int *prog, const unsigned in
             const int sblocks = (S / 2 + RK_T - 1) / RK_T;
             rb_sample<RK_RANK><<<(unsigned)ns * sblocks, RK_T, sample_smem, c->s>>>(
                 d_fins, d_finsoff, d_finfo, d_valid, d_c0, kmax, c->d_cols64, c->d_y64, c->npad, n, ntrials,
-                s0, sblocks, S, sp.b.fmaxins, r.samp);
+                s0, sblocks, S, RB_MAXS, sp.b.fmaxins, r.samp);
             rb_splitters<<<ns, RB_ST, sizeof(u64) * P2, c->s>>>(r.samp, S, P2, m, r.spl, r.nspl);
             c->launches += 2;
         } else {
@@ -2115,7 +2116,8 @@ float rc_order_stat_score_batch(void *ctx, const unsigned int *prog, const unsig
     /* a median by selection (a wave's key lists in RK_WAVE_BYTES, a segment
        it cannot settle sorted alone), the interquartile mean by sorting */
     const size_t work = cur;
-    const size_t sel_per = sizeof(u64) * ((size_t)n + RB_MAXS + 2) + 2 * sizeof(unsigned);
+    const size_t nsamp = n <= OS_LIST_ALL ? 0 : OS_S;
+    const size_t sel_per = sizeof(u64) * ((size_t)n + nsamp + 2) + 2 * sizeof(unsigned);
     const int wseg = what == 0
                          ? (int)std::min<size_t>(std::max<size_t>(RK_WAVE_BYTES / sel_per, 1), nsegs)
                          : wave_segments(nsegs, n, false);
@@ -2159,7 +2161,7 @@ float rc_order_stat_score_batch(void *ctx, const unsigned int *prog, const unsig
     auto select_wave = [&](int s0, int ns) {
         size_t wc = work;
         u64 *list = reinterpret_cast<u64 *>(dev + rc_take(&wc, sizeof(u64) * (size_t)ns * n));
-        u64 *samp = reinterpret_cast<u64 *>(dev + rc_take(&wc, sizeof(u64) * (size_t)ns * RB_MAXS));
+        u64 *samp = reinterpret_cast<u64 *>(dev + rc_take(&wc, sizeof(u64) * (size_t)ns * nsamp));
         u64 *bracket = reinterpret_cast<u64 *>(dev + rc_take(&wc, sizeof(u64) * 2 * (size_t)ns));
         unsigned *cnt = reinterpret_cast<unsigned *>(dev + rc_take(&wc, sizeof(unsigned) * 2 * (size_t)ns));
         cudaMemsetAsync(cnt, 0, sizeof(unsigned) * 2 * (size_t)ns, c->s);
@@ -2168,7 +2170,7 @@ float rc_order_stat_score_batch(void *ctx, const unsigned int *prog, const unsig
             const int sblocks = (OS_S / 2 + RK_T - 1) / RK_T;
             rb_sample<RK_ABS><<<(unsigned)ns * sblocks, RK_T, sample_smem, c->s>>>(
                 d_fins, d_finsoff, d_finfo, d_valid, d_c0, kmax, c->d_cols64, c->d_y64, c->npad, n,
-                ntrials, s0, sblocks, OS_S, sp.b.fmaxins, samp);
+                ntrials, s0, sblocks, OS_S, OS_S, sp.b.fmaxins, samp);
             c->launches += 1;
         }
         os_bracket<<<ns, OS_SEL_T, 0, c->s>>>(samp, all, bracket);
