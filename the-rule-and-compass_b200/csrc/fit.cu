@@ -612,7 +612,9 @@ __host__ __device__ inline size_t ft_sweep4_smem(int opk, int maxins, int slots,
 /* One row's place in an assembly, from its prediction (eval.cu:1692-1804
    for f32, :1492-1630 for f64): whether it counts, whether it is usable, the
    adjoint seed (its square-root IRLS/GN weight), the weighted residual and
-   its objective term. */
+   its objective term, a product rounded by itself: a grouped tile keeps it in
+   shared memory before it is added, a tile of one group adds it in place, and
+   the two have to agree. */
 struct FtRow {
     bool use, ok;
     float s_zero;
@@ -665,10 +667,10 @@ __device__ __forceinline__ FtRow ft_row_f32(const FitArgs &a, int rr, int r1, fl
         const double qq = ft_logistic_q(u);
         sw = wr * qq * (1.0 - qq);
         resp = -tt / qq;
-        o.loss = wr * ft_softplus_neg(u);
+        o.loss = __dmul_rn(wr, ft_softplus_neg(u));
     } else {
         sw = ft_row_weight(wr, (double)r, a.metric);
-        o.loss = wr * (double)ft_row_loss_f(r, a.metric);
+        o.loss = __dmul_rn(wr, (double)ft_row_loss_f(r, a.metric));
     }
     const float s = sqrtf((float)sw);
     o.ok = good;
@@ -710,7 +712,7 @@ __device__ __forceinline__ FtRow ft_row_f64(const FitArgs &a, int rr, int r1, do
     }
     const double s = sqrt(sw);
     o.ok = good;
-    o.loss = wr * rho;
+    o.loss = __dmul_rn(wr, rho);
     if (good) {
         o.seed = s > 0.0 ? s : 1.0;
         o.s_zero = s > 0.0 ? 0.0f : 1.0f;
