@@ -448,7 +448,7 @@ def score_plain_and_absolute(ev, prog, off, pcount, vals, N, flushbuf, seed, sam
                          "config": "the same batch and rows, absolute error"}}
 
 
-def fit_lane_ops(plans, sweeps, N, metric):
+def fit_lane_ops(plans, sweeps, lost, N, metric):
     """Algorithmic work of one fit in FP32-lane-op equivalents, from the
     sweeps each candidate actually ran (the device's per-candidate counts):
     per row, an f32 assembly is the forward (L) and reverse (2.5 L) sweeps
@@ -456,13 +456,17 @@ def fit_lane_ops(plans, sweeps, N, metric):
     FP64 issues at half the FP32 rate), an f32 objective sweep L + 2, and the
     f64 sweeps the same work at twice the cost; the implicit Jacobian is four
     passes (7 L) plus G, its cost sweep the forward and input adjoint (3.5 L)
-    plus the norm and the division. L = the candidate's records."""
+    plus the norm and the division. L = the candidate's records. The 2,048-row
+    tiles that an objective sweep left out (`lost`, the device's counts) are
+    no work done."""
     tot = 0.0
-    for pl, sw in zip(plans, sweeps):
+    ntiles = (N + 2047) // 2048
+    for pl, sw, lo in zip(plans, sweeps, lost):
         L = len(pl.words) / 4.0
         p = pl.nconst
         G = p * (p + 1) / 2.0 + p + 1 + (2 if metric in (2, 3) else 0) * (p + 2)
         a32, l32, a64, l64 = (float(q) for q in sw)
+        l32, l64 = l32 - lo[0] / ntiles, l64 - lo[1] / ntiles
         if metric == 6:
             per = 2.0 * a64 * (7.0 * L + G) + 2.0 * l64 * (3.5 * L + 6.0)
         else:
@@ -523,13 +527,14 @@ def time_fit(pkg, ev, plans, metric, N, steps, warmup, flushbuf, plain_n, seed, 
             wall.append(time.perf_counter() - t0)
             dev_ms.append(ms)
     launches = ev.launch_count() - n0
-    sweeps = ev.fit_sweeps(P)
+    sweeps, lost = ev.fit_sweeps(P), ev.fit_lost_tiles(P)
     out = dict(P=P, N=N, dev_ms=dev_ms, wall=wall, clocks=clk.summary(), launches=launches,
                unit_count=float(P), status=np.bincount(st, minlength=9).tolist(),
                h2d=int(prog.nbytes + off.nbytes + pcount.nbytes + c0.nbytes + gauge.nbytes),
                d2h=int(P * (kmax * 8 + 8 + 4)), loss=loss, status_list=st,
                sweeps_mean=sweeps.mean(0).tolist(), fit_budgets_kb=budgets,
-               lane_ops=fit_lane_ops(plans, sweeps, N, metric))
+               sweeps_lost_mean=(lost.mean(0) / ((N + 2047) // 2048)).tolist(),
+               lane_ops=fit_lane_ops(plans, sweeps, lost, N, metric))
     if plain_n:
         rng = np.random.Generator(np.random.PCG64(seed + 77))
         idx = np.sort(rng.choice(P, size=min(plain_n, P), replace=False))
@@ -556,7 +561,9 @@ def fit_summary(r, peaks, what):
          "e2e": r["unit_count"] * len(r["wall"]) / sum(r["wall"]),
          "ms_per_step": float(np.mean(r["dev_ms"])), "steps": len(r["dev_ms"]),
          "config": what, "gpu_launches": r["launches"], "status_histogram": r["status"],
-         "sweeps_per_candidate": r["sweeps_mean"], "fit_budgets_kb": r.get("fit_budgets_kb"),
+         "sweeps_per_candidate": r["sweeps_mean"],
+         "objective_sweeps_left_out_per_candidate": r["sweeps_lost_mean"],
+         "fit_budgets_kb": r.get("fit_budgets_kb"),
          "clocks": r["clocks"]}
     for k in ("status_histogram_reference_mode", "status57_classified", "cpu_baseline"):
         if k in r:
@@ -1008,7 +1015,8 @@ def fit_roofline(r, peaks):
     peak = 148 * 128 * peaks.get("sm_max_mhz", 1965.0) * 1e6 / 1e9
     return {"bound": "fp32_issue", "achieved": achieved, "peak": peak, "unit": "Glane-op/s",
             "frac": achieved / peak, "traffic": FIT_ASM_TRAFFIC,
-            "note": "the sweeps each candidate ran (device counts) x N x their per-row "
+            "note": "the sweeps each candidate ran (device counts, less the tiles that lost "
+                    "trials left out) x N x their per-row "
                     "FP32-lane-op equivalents (f32 assembly 3.5 L + 2 G, f32 objective L + 2, "
                     "f64 sweeps twice the f32 cost; G = p(p+1)/2 + p + 1 FMAs of the Gram "
                     "fold), L = records, / CUDA-event time of the whole fused fit (the graph "

@@ -237,10 +237,17 @@ int rc_fit_budgets(void *ctx, int *out_kb);
    call on the context), out[4 * cand + k]: k = 0 f32 assembly sweeps, 1 f32
    objective sweeps, 2 f64 assembly sweeps (implicit: Jacobian sweeps), 3 f64
    objective sweeps (implicit: cost sweeps); the correlation arm's assembly
-   and trial sweeps count as 0 and 1. A trial's objective sweep counts although
-   it ends early once its sum exceeds the objective to beat. Returns 0, or -1 when the last call was
-   not a fit of nprog candidates. No counterpart in the reference ABI. */
+   and trial sweeps count as 0 and 1. A trial's objective sweep counts whole
+   although it ends early once its sum exceeds the objective to beat
+   (rc_last_fit_lost_tiles). Returns 0, or -1 when the last call was not a fit
+   of nprog candidates. No counterpart in the reference ABI. */
 int rc_last_fit_sweeps(void *ctx, int nprog, int *out);
+/* The 2,048-row tiles that those sweeps left out because their trial was lost
+   already, out[2 * cand + k]: k = 0 f32, 1 f64 (implicit: cost) objective
+   sweeps. Which tiles are left out depends on their order in time, so the
+   counts differ between runs (the results do not). Returns as
+   rc_last_fit_sweeps does. No counterpart in the reference ABI. */
+int rc_last_fit_lost_tiles(void *ctx, int nprog, int *out);
 /* Per-row gradients of fit-record programs from the fused adjoint sweep, over
    rows [row0, row0 + nrows): want = 1 writes d f / d c_j (f32,
    out[(cand * nrows + r) * kmax + j]); want = 2 writes d f / d x_k

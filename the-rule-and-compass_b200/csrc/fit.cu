@@ -52,8 +52,9 @@
 #define FT_TILE_ROWS 2048
 #define FT_NBLK_MAX 21                     /* 4x4 blocks of a 24-wide augmented Gram */
 #define FT_PART_LOSS (FT_NBLK_MAX * 16)
-#define FT_PART_BAD (FT_PART_LOSS + 1)
+#define FT_PART_BAD (FT_PART_LOSS + 1) /* > 0: a failed row; FT_BAD_LOST: not swept */
 #define FT_PART_SKIP (FT_PART_LOSS + 2)
+#define FT_BAD_LOST (-1.0)
 #define FT_PART_STRIDE (FT_PART_LOSS + 4)
 #define FT_NTRI (FT_MAX_CONST * (FT_MAX_CONST + 1) / 2)
 
@@ -116,7 +117,10 @@ struct FitState {
     int nsw[4];            /* sweeps run: f32 assembly, f32 objective, f64 assembly, f64
                               objective (correlation and implicit kinds count in their
                               class: CASM / CSCORE as f32, IJAC / ICOST as f64) */
+    int lost[2];           /* tiles that lost trials' f32 and f64 objective sweeps left
+                              out (ft_trial_lost) */
 };
+static_assert(sizeof(FitState) % 8 == 0, "copied in 8-byte words");
 
 /* Fit flags of rc_fit_batch_fused. */
 #define FT_FLAG_NO_POLISH 1 /* skip the f64 re-baseline and polish */
@@ -485,7 +489,8 @@ __global__ void __launch_bounds__(FT_IMAXT, 1) ft_cost_sweep(FitArgs a, int q)
         if (s_lost) {
             if (tid == 0) {
                 double *pt = a.part + ((size_t)cand * a.ntiles + tile) * FT_PART_STRIDE;
-                pt[FT_PART_LOSS] = pt[FT_PART_BAD] = pt[FT_PART_SKIP] = 0.0;
+                pt[FT_PART_LOSS] = 0.0;
+                pt[FT_PART_BAD] = FT_BAD_LOST;
             }
             continue;
         }
@@ -1148,7 +1153,8 @@ __global__ void __launch_bounds__(ft_op_assembles(K0) ? 640 : 1024, 1) ft_sweep4
             if (s_lost) {
                 if (tid == 0) {
                     double *pt = a.part + ((size_t)cand * a.ntiles + tile) * FT_PART_STRIDE;
-                    pt[FT_PART_LOSS] = pt[FT_PART_BAD] = 0.0;
+                    pt[FT_PART_LOSS] = 0.0;
+                    pt[FT_PART_BAD] = FT_BAD_LOST;
                 }
                 continue;
             }
@@ -1356,6 +1362,7 @@ __device__ void ft_advance(const FitArgs &a, FitState &st, int cand, int p, doub
                 st.req = FT_REQ_NONE;
                 st.f64 = 0;
                 st.nsw[0] = st.nsw[1] = st.nsw[2] = st.nsw[3] = 0;
+                st.lost[0] = st.lost[1] = 0;
                 st.status = 0;
                 st.best = 0.0;
                 st.rank = st.skip = st.improved = st.start = 0;
@@ -1820,7 +1827,7 @@ __global__ void __launch_bounds__(FT_CTRL_T) ft_control(FitArgs a, int q, int in
     __shared__ int s_task, s_cand, s_op;
     __shared__ double s_loss;
     __shared__ double red[FT_CTRL_T];
-    __shared__ int s_bad, s_skip;
+    __shared__ int s_bad, s_skip, s_lost;
     const int tid = threadIdx.x;
     const int nq = q ^ 1;
     int total = 0;
@@ -1832,6 +1839,7 @@ __global__ void __launch_bounds__(FT_CTRL_T) ft_control(FitArgs a, int q, int in
         if (tid == 0) {
             const int t = atomicAdd(work, 1);
             s_task = t;
+            s_lost = 0;
             if (t < total) {
                 int cand = t, op = FOP_NONE;
                 if (!init) {
@@ -1897,20 +1905,23 @@ __global__ void __launch_bounds__(FT_CTRL_T) ft_control(FitArgs a, int q, int in
         {
             double loss = 0.0;
             double m[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-            int bad = 0, skip = 0;
+            int bad = 0, skip = 0, lost = 0;
             if (!init) {
                 const bool asm_ = ft_op_assembles(op), csc = op == FOP_CSCORE;
                 for (int t = tid; t < a.ntiles; t += FT_CTRL_T) {
                     const double *pp = pt + (size_t)t * FT_PART_STRIDE;
                     loss += pp[FT_PART_LOSS];
-                    bad |= pp[FT_PART_BAD] != 0.0;
+                    bad |= pp[FT_PART_BAD] > 0.0;
+                    lost += pp[FT_PART_BAD] == FT_BAD_LOST;
                     if (asm_) skip |= pp[FT_PART_SKIP] != 0.0;
                     if (csc)
                         for (int k = 0; k < 6; ++k) m[k] += pp[k];
                 }
             }
+            if (lost) atomicAdd(&s_lost, lost);
             bad = __syncthreads_or(bad);
             skip = __syncthreads_or(skip);
+            if (tid == 0) sst.lost[op == FOP_LOSS32 ? 0 : 1] += s_lost;
             const int nsum = op == FOP_CSCORE ? 7 : 1;
             for (int k = 0; k < nsum; ++k) {
                 red[tid] = k == 0 ? loss : m[k - 1];
@@ -3041,6 +3052,19 @@ float fit_run(RcCtx *c, const unsigned int *prog, const unsigned int *off, const
     return ms;
 }
 
+/* `k` ints at `off` of every candidate's state of the last fit. */
+int read_fit_counts(RcCtx *c, int nprog, size_t off, int k, int *out)
+{
+    if (!c || !out || !c->fit_state || nprog != c->fit_state_n) return -1;
+    if (cudaMemcpy2DAsync(out, k * sizeof(int), c->fit_state + off, c->fit_state_stride,
+                          k * sizeof(int), (size_t)nprog, cudaMemcpyDeviceToHost,
+                          c->s) != cudaSuccess) {
+        cudaGetLastError();
+        return -1;
+    }
+    return rc_finish(c);
+}
+
 }  // namespace
 
 extern "C" {
@@ -3233,16 +3257,15 @@ int rc_fit_budgets(void *ctx, int *out_kb)
    no fit of nprog candidates is the last call's. */
 int rc_last_fit_sweeps(void *ctx, int nprog, int *out)
 {
-    RcCtx *c = (RcCtx *)ctx;
-    if (!c || !out || !c->fit_state || nprog != c->fit_state_n) return -1;
-    const size_t off = offsetof(FitState, nsw);
-    if (cudaMemcpy2DAsync(out, 4 * sizeof(int), c->fit_state + off, c->fit_state_stride,
-                          4 * sizeof(int), (size_t)nprog, cudaMemcpyDeviceToHost,
-                          c->s) != cudaSuccess) {
-        cudaGetLastError();
-        return -1;
-    }
-    return rc_finish(c);
+    return read_fit_counts((RcCtx *)ctx, nprog, offsetof(FitState, nsw), 4, out);
+}
+
+/* Tiles of FT_TILE_ROWS rows that each candidate's objective sweeps left out
+   in the context's last fit, out[2 * cand + k]: k = 0 f32, 1 f64 (implicit:
+   cost) sweeps. Returns as rc_last_fit_sweeps does. */
+int rc_last_fit_lost_tiles(void *ctx, int nprog, int *out)
+{
+    return read_fit_counts((RcCtx *)ctx, nprog, offsetof(FitState, lost), 2, out);
 }
 
 int rc_fit_kernel_info(int kmax, int *threads, int *smem_bytes, int *max_constants)

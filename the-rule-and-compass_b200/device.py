@@ -77,6 +77,7 @@ SIGNATURES = {
     "rc_rank_tuning": (ci, [cvp, ci, ci]),
     "rc_rank_last_fallbacks": (ci, [cvp]),
     "rc_last_fit_sweeps": (ci, [cvp, ci, ctypes.POINTER(ctypes.c_int32)]),
+    "rc_last_fit_lost_tiles": (ci, [cvp, ci, ctypes.POINTER(ctypes.c_int32)]),
     "rc_multi_create": (cvp, [f32p, ci, ci, f32p, ci, i32p]),
     "rc_multi_destroy": (None, [cvp]),
     "rc_multi_set_fit_data": (ci, [cvp, f64p, f64p, f64p]),
@@ -444,6 +445,14 @@ class GpuEvaluator:
         out = np.zeros((nprog, 4), np.int32)
         if lib().rc_last_fit_sweeps(self.ctx, nprog, _p(out, ctypes.c_int32)) != 0:
             raise DeviceError("rc_last_fit_sweeps failed")
+        return out
+
+    def fit_lost_tiles(self, nprog):
+        """2,048-row tiles per candidate that the last fit's objective sweeps
+        left out because their trial was lost: int32 [P][2] (f32, f64)."""
+        out = np.zeros((nprog, 2), np.int32)
+        if lib().rc_last_fit_lost_tiles(self.ctx, nprog, _p(out, ctypes.c_int32)) != 0:
+            raise DeviceError("rc_last_fit_lost_tiles failed")
         return out
 
     def score_profile(self):
