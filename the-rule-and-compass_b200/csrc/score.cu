@@ -357,6 +357,16 @@ int rc_score_tile_rows(int n)
     while (rows < RC_TILE_ROWS && (long long)rows * 32 < n) rows *= 2;
     return rows;
 }
+/* Tiles are short for the sake of small batches; a batch with items to spare
+   takes several a work item, up to RC_TILE_ROWS rows, so that its programs
+   are staged, and its blocks wait for an item, once for all of them (an item
+   of one short tile spends as long on that as on its rows). Items an SM from
+   which a span is doubled: 4,096 programs x 65,536 rows, squared error, 2.06 ms
+   of device time with one tile an item, 1.08-1.16 with 8 to 16 items an SM,
+   1.46 with 32; 4,096 x 8,192 under the maximum 0.71 with one tile, 0.50 with
+   8 or 12 items, 0.71 with 16; but few items leave the last ones alone: 100
+   pool programs x 262,144 rows 0.36 ms with 12 or 16, 0.42 with 8 or 10. */
+const int SPAN_ITEMS = 12;
 const int LANE_T = 128;
 
 /* The scoring kernel of a launch: the 256-thread shape has the common modes
@@ -628,7 +638,13 @@ float rc_score_run(RcCtx *c, const uint32_t *words, const uint32_t *off, int wid
             a.group = group;
             a.subtiles = tile_rows / (T * 4);
             const int ngroups = (nb + group - 1) / group;
-            a.nitems = ngroups * ntiles;
+            /* (a candidate's bits do not depend on its item's span either) */
+            a.span = 1;
+            while (2 * a.span * tile_rows <= RC_TILE_ROWS &&
+                   (long long)ngroups * ((ntiles + 2 * a.span - 1) / (2 * a.span)) >=
+                       (long long)c->sm_count * SPAN_ITEMS)
+                a.span *= 2;
+            a.nitems = ngroups * ((ntiles + a.span - 1) / a.span);
             a.maxins = bk[b].maxins;
             a.nslots = std::max(bk[b].nslots, 1);
             a.counter = d_cnt + b + 2 * pass;
@@ -1209,6 +1225,7 @@ extern "C" int rc_score_batch_noalloc(const float *cols, const float *y, int n, 
     a.group = group;
     a.subtiles = TILE_ROWS / SUB;
     a.ntiles = ntiles;
+    a.span = 1;
     a.nitems = ((nprog + a.group - 1) / a.group) * ntiles;
     a.maxins = RC_MAX_INS;
     a.nslots = RC_SHALLOW_SLOTS;

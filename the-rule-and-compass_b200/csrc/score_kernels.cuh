@@ -499,7 +499,8 @@ struct ScoreArgs {
     int group;            /* candidates per work item */
     int subtiles;         /* sub-tiles (T*4 rows each) per tile */
     int ntiles;
-    int nitems;
+    int span;             /* tiles of an item */
+    int nitems;           /* groups of candidates x spans of tiles */
     int maxins;
     int nslots;
     int *counter;
@@ -621,7 +622,8 @@ template <int T>
 struct ScoreSmem {
     static __host__ __device__ size_t xs_bytes(int v, int staged) { return staged ? (size_t)v * T * 16 : 0; }
     static __host__ __device__ size_t stk_bytes(int nslots) { return (size_t)nslots * T * 24; }
-    static __host__ __device__ size_t warp_bytes(int group) { return (size_t)group * (T / 32) * 4 * 8; }
+    /* (two: one tile's sums are folded while the next one's are made) */
+    static __host__ __device__ size_t warp_bytes(int group) { return 2 * (size_t)group * (T / 32) * 4 * 8; }
     static __host__ __device__ size_t prog_bytes(int group, int maxins) { return (size_t)group * maxins * sizeof(RcIns); }
     static __host__ __device__ size_t total(int v, int staged, int nslots, int group, int maxins)
     {
@@ -645,9 +647,11 @@ __global__ void __launch_bounds__(T) rc_score_kernel(ScoreArgs a)
     float4 *stk = reinterpret_cast<float4 *>(smem_raw + ScoreSmem<T>::xs_bytes(a.v, a.staged));
     uint2 *estk = reinterpret_cast<uint2 *>(stk + a.nslots * T);
     double *swarp = reinterpret_cast<double *>(estk + a.nslots * T);
-    RcIns *sprog = reinterpret_cast<RcIns *>(swarp + a.group * NW * 4);
+    RcIns *sprog = reinterpret_cast<RcIns *>(swarp + 2 * a.group * NW * 4);
+    /* (what an item is, in shared memory: registers are short) */
     __shared__ int s_item;
-    __shared__ unsigned s_bad;
+    __shared__ volatile int s_cbase, s_gcount, s_tile1;
+    __shared__ unsigned s_bad; /* candidates known to be hard failures */
     __shared__ unsigned long long s_rows, s_ops;
     const int SUB = T * 4;
     const int mode = MODE >= 0 ? MODE : a.mode;
@@ -658,106 +662,117 @@ __global__ void __launch_bounds__(T) rc_score_kernel(ScoreArgs a)
         __syncthreads();
         const int item = s_item;
         if (item >= a.nitems) break;
-        const int g = item / a.ntiles;
-        const int tile = item - g * a.ntiles;
+        const int nspans = (a.ntiles + a.span - 1) / a.span;
+        const int g = item / nspans;
+        const int tile0 = (item - g * nspans) * a.span;
         const int cbase = g * a.group;
         const int gcount = min(a.group, a.ncand - cbase);
-
-        unsigned skipmask = 0;
+        unsigned known = 0;
         for (int c = 0; c < gcount; ++c) {
             const int cand = a.order[cbase + c];
             const int b = a.ins_off[cand];
             const int e = a.ins_len ? b + a.ins_len[cand] : a.ins_off[cand + 1];
             for (int q = tid; q < e - b; q += T) sprog[c * a.maxins + q] = a.ins[b + q];
-            if (skip_bad && *((volatile int *)(a.bad + cand))) skipmask |= 1u << c;
+            if (skip_bad && *((volatile int *)(a.bad + cand))) known |= 1u << c;
         }
-        /* one answer per warp: the votes below need all of its lanes */
-        skipmask = __reduce_or_sync(0xffffffffu, skipmask);
-        for (int q = tid; q < gcount * NW * 4; q += T) swarp[q] = 0.0;
         if (tid == 0) {
-            s_bad = 0;
+            s_cbase = cbase;
+            s_gcount = gcount;
+            s_tile1 = min(a.ntiles, tile0 + a.span);
+            s_bad = known;
             s_rows = 0;
             s_ops = 0;
         }
         __syncthreads();
 
-        /* each warp runs one candidate over all of the tile's rows before its
-           single reduction; the features come straight from L2 */
-        for (int c = 0; c < gcount; ++c) {
-            /* a candidate already known to be a hard failure skips its rows */
-            if (skip_bad && (skipmask & (1u << c))) continue;
-            const int cand = a.order[cbase + c];
-            double a0 = 0.0, a1 = 0.0, e0 = 0.0, e1 = 0.0;
-            int bad = 0;
-            int wrows = 0; /* rows of this warp the candidate was evaluated on */
-            for (int s = 0; s < a.subtiles; ++s) {
-                const int row0 = (tile * a.subtiles + s) * SUB;
-                if (row0 >= a.n) break;
-                const int myrow = row0 + 4 * tid;
-                wrows += max(0, min(128, a.n - (row0 + 128 * warp)));
-                float4 p, pe;
-                rc_run<T, TRACK>(sprog + c * a.maxins, nullptr, false, a.cols, a.npad, myrow, stk,
-                                 estk, tid, p, pe, a.fcols);
-                const float4 yv4 = __ldg(reinterpret_cast<const float4 *>(a.y + myrow));
-                const float pr[4] = {p.x, p.y, p.z, p.w};
-                const float pq[4] = {pe.x, pe.y, pe.z, pe.w};
-                const float yy[4] = {yv4.x, yv4.y, yv4.z, yv4.w};
+        for (int tile = tile0; tile < s_tile1; ++tile) {
+            /* each warp runs one candidate over all of the tile's rows before its
+               single reduction; the features come straight from L2 */
+            for (int c = 0; c < s_gcount; ++c) {
+                /* a candidate already known to be a hard failure skips its rows
+                   (one answer per warp: the votes below need all of its lanes,
+                   and other warps may be ahead) */
+                if (skip_bad &&
+                    (__shfl_sync(0xffffffffu, *(volatile unsigned *)&s_bad, 0) >> c & 1u)) {
+                    if (lane < 4) swarp[(((tile & 1) * a.group + c) * NW + warp) * 4 + lane] = 0.0;
+                    continue;
+                }
+                const int cand = a.order[s_cbase + c];
+                double a0 = 0.0, a1 = 0.0, e0 = 0.0, e1 = 0.0;
+                int bad = 0;
+                int wrows = 0; /* rows of this warp the candidate was evaluated on */
+                for (int s = 0; s < a.subtiles; ++s) {
+                    const int row0 = (tile * a.subtiles + s) * SUB;
+                    if (row0 >= a.n) break;
+                    const int myrow = row0 + 4 * tid;
+                    wrows += max(0, min(128, a.n - (row0 + 128 * warp)));
+                    float4 p, pe;
+                    rc_run<T, TRACK>(sprog + c * a.maxins, nullptr, false, a.cols, a.npad, myrow, stk,
+                                     estk, tid, p, pe, a.fcols);
+                    const float4 yv4 = __ldg(reinterpret_cast<const float4 *>(a.y + myrow));
+                    const float pr[4] = {p.x, p.y, p.z, p.w};
+                    const float pq[4] = {pe.x, pe.y, pe.z, pe.w};
+                    const float yy[4] = {yv4.x, yv4.y, yv4.z, yv4.w};
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const int row = myrow + i;
-                    if (row < a.n)
-                        rc_accumulate(a, mode, pr[i], pq[i], yy[i], row, cand, a0, a1, e0, e1,
-                                      bad);
+                    for (int i = 0; i < 4; ++i) {
+                        const int row = myrow + i;
+                        if (row < a.n)
+                            rc_accumulate(a, mode, pr[i], pq[i], yy[i], row, cand, a0, a1, e0, e1,
+                                          bad);
+                    }
+                    /* a hard failure ends this warp's rows of the candidate; the
+                       lowest failing 4-row group is kept for the f64 re-check */
+                    if (skip_bad && __any_sync(0xffffffffu, bad)) {
+                        const int grp = __reduce_min_sync(0xffffffffu,
+                                                          bad ? (unsigned)myrow : 0x7fffffffu);
+                        if (a.badrow && lane == 0) atomicMax(a.badrow + cand, RC_BADROW_BASE - grp);
+                        break;
+                    }
                 }
-                /* a hard failure ends this warp's rows of the candidate; the
-                   lowest failing 4-row group is kept for the f64 re-check */
-                if (skip_bad && __any_sync(0xffffffffu, bad)) {
-                    const int grp = __reduce_min_sync(0xffffffffu,
-                                                      bad ? (unsigned)myrow : 0x7fffffffu);
-                    if (a.badrow && lane == 0) atomicMax(a.badrow + cand, RC_BADROW_BASE - grp);
-                    break;
+                if (a.rows && lane == 0 && wrows > 0) {
+                    atomicAdd(&s_rows, (unsigned long long)wrows);
+                    atomicAdd(&s_ops, (unsigned long long)wrows * (unsigned long long)a.opw[cand]);
+                }
+                if (mode == SM_PREDICT) continue;
+                if (mode == SM_MAXIMUM) {
+                    a0 = rc_warp_max(a0);
+                    e0 = rc_warp_max(e0);
+                } else {
+                    a0 = rc_warp_sum(a0);
+                    if (TRACK) e0 = rc_warp_sum(e0);
+                    if (mode == SM_CORR_PASS2 || (mode >= SM_LOG_LOSS && mode <= SM_HINGE_SQUARED)) {
+                        a1 = rc_warp_sum(a1);
+                        if (TRACK) e1 = rc_warp_sum(e1);
+                    }
+                }
+                const unsigned anybad = __any_sync(0xffffffffu, bad);
+                if (lane == 0) {
+                    double *sw = swarp + (((tile & 1) * a.group + c) * NW + warp) * 4;
+                    sw[0] = a0;
+                    sw[1] = a1;
+                    sw[2] = e0;
+                    sw[3] = e1;
+                    if (anybad) atomicOr(&s_bad, 1u << c);
                 }
             }
-            if (a.rows && lane == 0 && wrows > 0) {
-                atomicAdd(&s_rows, (unsigned long long)wrows);
-                atomicAdd(&s_ops, (unsigned long long)wrows * (unsigned long long)a.opw[cand]);
-            }
-            if (mode == SM_PREDICT) continue;
-            if (mode == SM_MAXIMUM) {
-                a0 = rc_warp_max(a0);
-                e0 = rc_warp_max(e0);
-            } else {
-                a0 = rc_warp_sum(a0);
-                if (TRACK) e0 = rc_warp_sum(e0);
-                if (mode == SM_CORR_PASS2 || (mode >= SM_LOG_LOSS && mode <= SM_HINGE_SQUARED)) {
-                    a1 = rc_warp_sum(a1);
-                    if (TRACK) e1 = rc_warp_sum(e1);
-                }
-            }
-            const unsigned anybad = __any_sync(0xffffffffu, bad);
-            if (lane == 0) {
-                double *sw = swarp + (c * NW + warp) * 4;
-                sw[0] = a0;
-                sw[1] = a1;
-                sw[2] = e0;
-                sw[3] = e1;
-                if (anybad) atomicOr(&s_bad, 1u << c);
-            }
-        }
-        __syncthreads();
+            __syncthreads();
 
-        /* Warps in ascending order: one partial per (candidate, tile). */
-        if (tid < gcount * 4 && mode != SM_PREDICT) {
-            const int c = tid >> 2, q = tid & 3;
-            const int cand = a.order[cbase + c];
-            double s = 0.0;
-            for (int w = 0; w < NW; ++w) {
-                const double v = swarp[(c * NW + w) * 4 + q];
-                s = (mode == SM_MAXIMUM) ? fmax(s, v) : s + v;
+            /* Warps in ascending order: one partial per (candidate, tile). The
+               other warps go on to the next tile, whose sums take the other half. */
+            if (tid < s_gcount * 4 && mode != SM_PREDICT) {
+                const int c = tid >> 2, q = tid & 3;
+                const int cand = a.order[s_cbase + c];
+                double s = 0.0;
+                for (int w = 0; w < NW; ++w) {
+                    const double v = swarp[(((tile & 1) * a.group + c) * NW + w) * 4 + q];
+                    s = (mode == SM_MAXIMUM) ? fmax(s, v) : s + v;
+                }
+                a.part[((size_t)q * a.nprog + cand) * a.ptiles + tile] = s;
             }
-            a.part[((size_t)q * a.nprog + cand) * a.ptiles + tile] = s;
-            if (q == 0 && (s_bad & (1u << c)) && !(skipmask & (1u << c))) atomicOr(&a.bad[cand], 1);
         }
+        if (skip_bad && tid < s_gcount && (s_bad & (1u << tid)) &&
+            !*((volatile int *)(a.bad + a.order[s_cbase + tid])))
+            atomicOr(a.bad + a.order[s_cbase + tid], 1);
         if (a.rows && tid == 0 && s_rows) {
             atomicAdd(a.rows, s_rows);
             atomicAdd(a.rows + 2, s_ops);
