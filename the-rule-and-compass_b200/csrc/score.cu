@@ -146,9 +146,16 @@ int rc_decode_postfix(const uint32_t *words, size_t nwords, int v, RcIns *out, i
 
 namespace {
 
-/* Rows x programs from which a batch's constant subtrees and columns are
-   worth their two launches (about 30 us with the host's share; a batch of
-   that many row evaluations runs for 150 us and more). */
+/* Rows, and rows x programs, from which a batch's constant subtrees and
+   columns are worth their two launches and the host's share, which is 0.16 us
+   a program: what the rows of a program save is that much at about 400,000
+   rows (call times, squared error, shared / not: 4,096 x 65,536 2.44 /
+   1.90 ms, 4,096 x 262,144 4.21 / 3.90, 1,024 x 262,144 1.36 / 1.40,
+   1,024 x 1,048,576 3.50 / 3.75; 64 x 1,048,576 0.37 / 0.39, 16 x 1,048,576
+   0.55 / 0.55). A correlation evaluates its rows twice in f32 and, where the
+   f64 lane takes a candidate, twice there: 4,096 x 65,536 4.11 / 3.80 ms,
+   1,024 x 131,072 1.68 / 1.87, 4,096 x 131,072 6.15 / 6.09. */
+const int FOLD_ROWS = 1 << 19, FOLD_ROWS_CORR = 1 << 17;
 const long long FOLD_MIN = 1LL << 24;
 /* Columns only while the inputs and they stay in L2 (126 MB). */
 const size_t FCOL_BYTES = (size_t)96 << 20;
@@ -454,7 +461,8 @@ float rc_score_run(RcCtx *c, const uint32_t *words, const uint32_t *off, int wid
     ins_off[nprog] = (int)pos;
     /* constant subtrees and shared columns, for a batch large enough */
     FoldedBatch fb;
-    if ((long long)nprog * c->n >= FOLD_MIN)
+    const bool corr = (mode == SM_CORRELATION || mode == SM_CORRELATION_SIGNED);
+    if (c->n >= (corr ? FOLD_ROWS_CORR : FOLD_ROWS) && (long long)nprog * c->n >= FOLD_MIN)
         fold_programs(c->score_lists, ins, ins_off, nprog, c->v, sizeof(float) * (size_t)c->npad, fb);
     const bool folded = !fb.folds.empty() || !fb.spec.empty();
     if (folded) {
@@ -495,7 +503,6 @@ float rc_score_run(RcCtx *c, const uint32_t *words, const uint32_t *off, int wid
     order.reserve(nprog);
     for (int b = 0; b < 2; ++b) order.insert(order.end(), bk[b].cands.begin(), bk[b].cands.end());
 
-    const bool corr = (mode == SM_CORRELATION || mode == SM_CORRELATION_SIGNED);
     const bool track = mode < SM_EVAL_SQUARED;
 
     /* 3. layout: inputs [ins | ins_off | order | opw], outputs
