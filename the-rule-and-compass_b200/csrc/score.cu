@@ -372,8 +372,12 @@ int rc_score_tile_rows(int n)
    of device time with one tile an item, 1.08-1.16 with 8 to 16 items an SM,
    1.46 with 32; 4,096 x 8,192 under the maximum 0.71 with one tile, 0.50 with
    8 or 12 items, 0.71 with 16; but few items leave the last ones alone: 100
-   pool programs x 262,144 rows 0.36 ms with 12 or 16, 0.42 with 8 or 10. */
-const int SPAN_ITEMS = 12;
+   pool programs x 262,144 rows 0.36 ms with 12 or 16, 0.42 with 8 or 10. The
+   longer the span, the less its items save and the more their last wave costs:
+   past 8,192 rows more of them are asked for (256 x 262,144 0.50 ms with tiles
+   of their own, 0.58 with 13.8 items an SM of two; 4,096 x 262,144 3.65 and,
+   with 28 items of four, 2.85). */
+inline long long span_items(int rows) { return rows <= 8192 ? 12 : 16; }
 const int LANE_T = 128;
 
 /* The scoring kernel of a launch: the 256-thread shape has the common modes
@@ -647,10 +651,11 @@ float rc_score_run(RcCtx *c, const uint32_t *words, const uint32_t *off, int wid
             const int ngroups = (nb + group - 1) / group;
             /* (a candidate's bits do not depend on its item's span either) */
             a.span = 1;
-            while (2 * a.span * tile_rows <= RC_TILE_ROWS &&
-                   (long long)ngroups * ((ntiles + 2 * a.span - 1) / (2 * a.span)) >=
-                       (long long)c->sm_count * SPAN_ITEMS)
-                a.span *= 2;
+            for (int s = 2; s * tile_rows <= RC_TILE_ROWS &&
+                            (long long)ngroups * ((ntiles + s - 1) / s) >=
+                                c->sm_count * span_items(s * tile_rows);
+                 s *= 2)
+                a.span = s;
             a.nitems = ngroups * ((ntiles + a.span - 1) / a.span);
             a.maxins = bk[b].maxins;
             a.nslots = std::max(bk[b].nslots, 1);
