@@ -686,14 +686,15 @@ __global__ void __launch_bounds__(T) rc_score_kernel(ScoreArgs a)
         __syncthreads();
 
         for (int tile = tile0; tile < s_tile1; ++tile) {
+            /* candidates already known to be hard failures skip their rows (one
+               answer per warp: the votes below need all of its lanes, and other
+               warps may be ahead) */
+            const unsigned skip =
+                skip_bad ? __shfl_sync(0xffffffffu, *(volatile unsigned *)&s_bad, 0) : 0u;
             /* each warp runs one candidate over all of the tile's rows before its
                single reduction; the features come straight from L2 */
             for (int c = 0; c < s_gcount; ++c) {
-                /* a candidate already known to be a hard failure skips its rows
-                   (one answer per warp: the votes below need all of its lanes,
-                   and other warps may be ahead) */
-                if (skip_bad &&
-                    (__shfl_sync(0xffffffffu, *(volatile unsigned *)&s_bad, 0) >> c & 1u)) {
+                if (skip >> c & 1u) {
                     if (lane < 4) swarp[(((tile & 1) * a.group + c) * NW + warp) * 4 + lane] = 0.0;
                     continue;
                 }
