@@ -1,5 +1,5 @@
 """Folded constant subtrees and shared columns of the scorer at the row counts
-that they start from (524,288, a correlation 131,072): a batch just past them,
+that they start from (393,216, a correlation 131,072): a batch just past them,
 and one just below, gives every program the bits and status it gets alone
 (where nothing is folded or shared), in scores and in predictions."""
 import importlib
@@ -26,8 +26,8 @@ def _programs(pkg, E, rng, count):
     return out + [W.random_scoring_tree(rng, 3) for _ in range(count - len(out))]
 
 
-@pytest.mark.parametrize("kind,n,count", [(0, 524288, 34), (1, 524325, 34), (4, 524325, 34),
-                                          (10, 524288, 34), (0, 524287, 34), (5, 131072, 132),
+@pytest.mark.parametrize("kind,n,count", [(0, 393216, 44), (1, 393253, 44), (4, 393253, 44),
+                                          (10, 393216, 44), (0, 393215, 44), (5, 131072, 132),
                                           (6, 131077, 132), (5, 131071, 132)])
 def test_a_batch_past_the_line_gives_the_bits_of_each_program_alone(pkg, E, kind, n, count):
     rng = np.random.Generator(np.random.PCG64(n + kind))
@@ -47,13 +47,13 @@ def test_a_batch_past_the_line_gives_the_bits_of_each_program_alone(pkg, E, kind
 
 
 def test_predictions_past_the_line(pkg, E):
-    n = 524293
+    n = 393221
     rng = np.random.Generator(np.random.PCG64(n))
     x = rng.normal(0.0, 1.0, (3, n)).astype(np.float32)
     ev = pkg.GpuEvaluator(x.reshape(-1), n, 3, x[0])
-    prog, off = pkg.Population(_programs(pkg, E, rng, 34)).programs()
+    prog, off = pkg.Population(_programs(pkg, E, rng, 44)).programs()
     big = ev.predictions(prog, off)
-    for k in range(34):
+    for k in range(44):
         p1 = prog[off[k]:off[k + 1]]
         one = ev.predictions(p1, np.array([0, len(p1)], np.uint32))[0]
         ok = ~np.isnan(one)
