@@ -30,6 +30,12 @@
 
 #define RV_K 3   /* attempts per slot computed on the device */
 #define RV_T 128
+/* Slots from which the parents' metadata is read back by itself, before the
+   children are built: a copy and a wait of about 12 us, which the host's work
+   beside the children repays on large pools (a call of 50 slots 234 us without
+   it and 247 with, 1,600 405 and 417, 4,800 609 and 607, 16,000 1,420 and
+   1,337). */
+#define RV_EARLY 4096
 
 namespace {
 
@@ -252,9 +258,13 @@ extern "C" float rc_pool_vary(void *ctx, int which, int islands, int pop, int wi
                                                              d_pcost, d_pcost16, d_phash, d_bad);
 
     /* read back while the children are built: the parents' hashes and the
-       elites are ready when the items arrive */
-    cudaMemcpyAsync(host + o_plen, dev + o_plen, o_items - o_plen, cudaMemcpyDeviceToHost, c->s);
-    cudaEventRecord(c->sp[0], c->s);
+       elites are ready when the items arrive (a small pool's come with them:
+       RV_EARLY) */
+    const bool early = nslots >= RV_EARLY;
+    if (early) {
+        cudaMemcpyAsync(host + o_plen, dev + o_plen, o_items - o_plen, cudaMemcpyDeviceToHost, c->s);
+        cudaEventRecord(c->sp[0], c->s);
+    }
 
     /* 2. the first RV_K attempts of every child slot */
     RvParents dpar;
@@ -267,9 +277,12 @@ extern "C" float rc_pool_vary(void *ctx, int which, int islands, int pop, int wi
     uint32_t *d_progs = reinterpret_cast<uint32_t *>(dev + o_progs);
     rv_children<<<(nitems + RV_T - 1) / RV_T, RV_T, 0, c->s>>>(
         cfg, dpar, reinterpret_cast<const uint8_t *>(dev + o_restart), d_bad, d_items, d_progs);
-    cudaMemcpyAsync(host + o_items, dev + o_items, meta_end - o_items, cudaMemcpyDeviceToHost, c->s);
+    const size_t late = early ? o_items : o_plen;
+    cudaMemcpyAsync(host + late, dev + late, meta_end - late, cudaMemcpyDeviceToHost, c->s);
     c->launches += 2;
-    if (cudaGetLastError() != cudaSuccess || cudaEventSynchronize(c->sp[0]) != cudaSuccess) {
+    if (!early) {
+        if (rc_finish(c) != 0) return -1.0f;
+    } else if (cudaGetLastError() != cudaSuccess || cudaEventSynchronize(c->sp[0]) != cudaSuccess) {
         cudaStreamSynchronize(c->s);
         cudaGetLastError();
         return -1.0f;
@@ -319,7 +332,7 @@ extern "C" float rc_pool_vary(void *ctx, int which, int islands, int pop, int wi
         }
         elites[i] = elite;
     }
-    if (rc_finish(c) != 0) return -1.0f; /* the items are here */
+    if (early && rc_finish(c) != 0) return -1.0f; /* the items are here */
     for (int i = 0; i < islands; ++i) {
         const bool rs = restart && restart[i];
         const int elite = elites[i];
