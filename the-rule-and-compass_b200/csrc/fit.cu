@@ -2745,7 +2745,13 @@ unsigned long long enqueue_fit(RcCtx *c, cudaStream_t s_, const FitArgs &a, int 
 }
 
 /* At most this many (candidate, tile) items per SM: every kind of a step in
-   one launch, on one chain. */
+   one launch, on one chain: half the launches of a step, which short steps
+   wait for, against the overlap of chains and shapes of their own. With the
+   line at 2 instead: squared error, 300 x 2,000 rows 4.9 -> 5.5 ms, 500 x 2,000
+   5.3 -> 5.7, 110 x 8,000 as it is, 280 x 8,000 6.3 -> 6.1, 9 x 131,072
+   3.6 -> 3.1; correlation, 50 x 30,011 2.2 -> 2.4, 17 x 131,072 2.8 -> 2.3;
+   implicit, 110 x 8,000 6.7 -> 4.8: tables of many tiles and the implicit fits
+   would rather have it lower, many candidates over few tiles where it is. */
 #define FT_SMALL_ITEMS_PER_SM 8
 
 float fit_run(RcCtx *c, const unsigned int *prog, const unsigned int *off, const int *pcount,

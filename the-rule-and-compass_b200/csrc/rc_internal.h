@@ -35,7 +35,7 @@ enum RcInsKind {
     K_IF = 6,         /* TOS = slot[arg] > 0 ? slot[arg + 1] : TOS */
     K_HALT = 7,       /* result = TOS (depth 1) or slot[0] (depth > 1) */
     K_NAN = 8,        /* the whole program is a hard failure (NaN every row) */
-    /* made from the kinds above for one batch (rc_fold_programs): */
+    /* made from the kinds above for one batch (fold_programs, score.cu): */
     K_PUSH_COL = 9,   /* spill TOS; TOS = op(input), read from the batch's column imm */
     K_PUSH_FOLD = 10  /* spill TOS; TOS = a folded constant subtree: f32 bits of its value here
                          and of its error bound in the next word's imm (f64 lane: the low
