@@ -1342,10 +1342,10 @@ __global__ void __launch_bounds__(OS_T) os_pick(const u64 *ka, const u64 *kb,
  * bracket is everything: a sample's two launches against a longer list for one
  * block, by the candidates that share the launches (8 x 24,000 rows 0.24 ms
  * listed and 0.26 sampled, 100 x 24,000 0.58 and 0.54, 8 x 48,000 0.28 and
- * 0.26, 100 x 48,000 0.70 and 0.66). A middle outside the bracket (rows that the sample
- * did not stand for) sends the segment to the sort, so the value is exact
- * either way. The pass writes 0.75 B a key where keys and their sort moved
- * 8 B and eight times 16. */
+ * 0.26, 100 x 48,000 0.70 and 0.66). A middle outside the bracket (rows that
+ * the sample did not stand for) sends the segment to the sort, so the value is
+ * exact either way. The pass writes 0.75 B a key where keys and their sort
+ * moved 8 B and eight times 16. */
 #define OS_S 4096
 #define OS_D 192
 #define OS_LIST_ALL 32768
