@@ -759,9 +759,10 @@ __global__ void __launch_bounds__(T) rc_score_kernel(ScoreArgs a)
             __syncthreads();
 
             /* Warps in ascending order: one partial per (candidate, tile). The
-               other warps go on to the next tile, whose sums take the other half. */
-            if (tid < s_gcount * 4 && mode != SM_PREDICT) {
-                const int c = tid >> 2, q = tid & 3;
+               other warps go on to the next tile, whose sums take the other half.
+               (A group of 32 has more sums than the 64-thread shape threads.) */
+            for (int i = tid; i < s_gcount * 4 && mode != SM_PREDICT; i += T) {
+                const int c = i >> 2, q = i & 3;
                 const int cand = a.order[s_cbase + c];
                 double s = 0.0;
                 for (int w = 0; w < NW; ++w) {
@@ -769,6 +770,7 @@ __global__ void __launch_bounds__(T) rc_score_kernel(ScoreArgs a)
                     s = (mode == SM_MAXIMUM) ? fmax(s, v) : s + v;
                 }
                 a.part[((size_t)q * a.nprog + cand) * a.ptiles + tile] = s;
+                if (T >= 4 * 32) break;
             }
         }
         if (skip_bad && tid < s_gcount && (s_bad & (1u << tid)) &&
