@@ -378,7 +378,9 @@ int rc_score_tile_rows(int n)
    longer the span, the less its items save and the more their last wave costs:
    past 8,192 rows more of them are asked for (256 x 262,144 0.50 ms with tiles
    of their own, 0.58 with 13.8 items an SM of two; 4,096 x 262,144 3.65 and,
-   with 28 items of four, 2.85). */
+   with 28 items of four, 2.85). The 64-thread shape takes tiles one by one: its
+   blocks are small and many, and share out the items evenly (1,024 programs of
+   18 slots x 65,536 rows 2.47 ms, with spans 3.47). */
 inline long long span_items(int rows) { return rows <= 8192 ? 12 : 16; }
 const int LANE_T = 128;
 
@@ -662,7 +664,7 @@ float rc_score_run(RcCtx *c, const uint32_t *words, const uint32_t *off, int wid
             const int ngroups = (nb + group - 1) / group;
             /* (a candidate's bits do not depend on its item's span either) */
             a.span = 1;
-            for (int s = 2; s * tile_rows <= RC_TILE_ROWS &&
+            for (int s = 2; T == 256 && s * tile_rows <= RC_TILE_ROWS &&
                             (long long)ngroups * ((ntiles + s - 1) / s) >=
                                 c->sm_count * span_items(s * tile_rows);
                  s *= 2)
@@ -673,8 +675,8 @@ float rc_score_run(RcCtx *c, const uint32_t *words, const uint32_t *off, int wid
             a.counter = d_cnt + b + 2 * pass;
             a.mode = kmode;
             const size_t smem = T == 256
-                ? ScoreSmem<256>::total(c->v, staged, a.nslots, group, a.maxins)
-                : ScoreSmem<64>::total(c->v, staged, a.nslots, group, a.maxins);
+                ? ScoreSmem<256>::total(c->v, staged, a.nslots, group, a.span, a.maxins)
+                : ScoreSmem<64>::total(c->v, staged, a.nslots, group, a.span, a.maxins);
             const void *fn = score_kernel_fn(T, track, kmode);
             if (set_smem(fn, smem) != 0) {
                 st->failed = 1;
@@ -1188,7 +1190,7 @@ extern "C" int rc_score_batch_noalloc(const float *cols, const float *y, int n, 
     const int G = 8;
     const int group = G < nprog ? G : nprog;
     /* features are read from global memory (L2), nothing is staged */
-    const size_t smem = ScoreSmem<256>::total(v, 0, RC_SHALLOW_SLOTS, group, RC_MAX_INS);
+    const size_t smem = ScoreSmem<256>::total(v, 0, RC_SHALLOW_SLOTS, group, 1, RC_MAX_INS);
     const size_t lsmem = lane_smem(RC_SHALLOW_SLOTS);
     NoallocDevice *d = &g_noalloc[dev];
     {
@@ -1202,7 +1204,7 @@ extern "C" int rc_score_batch_noalloc(const float *cols, const float *y, int n, 
                 cudaGetLastError();
                 return -1;
             }
-            const size_t maxsmem = ScoreSmem<256>::total(0, 0, RC_SHALLOW_SLOTS, G, RC_MAX_INS);
+            const size_t maxsmem = ScoreSmem<256>::total(0, 0, RC_SHALLOW_SLOTS, G, 1, RC_MAX_INS);
             if (set_smem((const void *)rc_score_kernel<256, true, -1>, maxsmem) != 0 ||
                 set_smem((const void *)rc_score64_kernel<LANE_T, -1>, lsmem) != 0)
                 return -1;

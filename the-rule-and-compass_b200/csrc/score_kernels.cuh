@@ -622,12 +622,12 @@ template <int T>
 struct ScoreSmem {
     static __host__ __device__ size_t xs_bytes(int v, int staged) { return staged ? (size_t)v * T * 16 : 0; }
     static __host__ __device__ size_t stk_bytes(int nslots) { return (size_t)nslots * T * 24; }
-    /* (two: one tile's sums are folded while the next one's are made) */
-    static __host__ __device__ size_t warp_bytes(int group) { return 2 * (size_t)group * (T / 32) * 4 * 8; }
+    /* (twice for a span: one tile's sums are folded while the next one's are made) */
+    static __host__ __device__ size_t warp_bytes(int group, int span) { return (size_t)(span > 1 ? 2 : 1) * group * (T / 32) * 4 * 8; }
     static __host__ __device__ size_t prog_bytes(int group, int maxins) { return (size_t)group * maxins * sizeof(RcIns); }
-    static __host__ __device__ size_t total(int v, int staged, int nslots, int group, int maxins)
+    static __host__ __device__ size_t total(int v, int staged, int nslots, int group, int span, int maxins)
     {
-        return xs_bytes(v, staged) + stk_bytes(nslots) + warp_bytes(group) + prog_bytes(group, maxins);
+        return xs_bytes(v, staged) + stk_bytes(nslots) + warp_bytes(group, span) + prog_bytes(group, maxins);
     }
 };
 
@@ -647,10 +647,11 @@ __global__ void __launch_bounds__(T) rc_score_kernel(ScoreArgs a)
     float4 *stk = reinterpret_cast<float4 *>(smem_raw + ScoreSmem<T>::xs_bytes(a.v, a.staged));
     uint2 *estk = reinterpret_cast<uint2 *>(stk + a.nslots * T);
     double *swarp = reinterpret_cast<double *>(estk + a.nslots * T);
-    RcIns *sprog = reinterpret_cast<RcIns *>(swarp + 2 * a.group * NW * 4);
+    const int half = a.span > 1 ? a.group : 0; /* the other tile's sums */
+    RcIns *sprog = reinterpret_cast<RcIns *>(swarp + (a.group + half) * NW * 4);
     /* (what an item is, in shared memory: registers are short) */
     __shared__ int s_item;
-    __shared__ volatile int s_cbase, s_gcount, s_tile1;
+    __shared__ int s_cbase, s_gcount, s_tile1;
     __shared__ unsigned s_bad; /* candidates known to be hard failures */
     __shared__ unsigned long long s_rows, s_ops;
     const int SUB = T * 4;
@@ -695,7 +696,7 @@ __global__ void __launch_bounds__(T) rc_score_kernel(ScoreArgs a)
                single reduction; the features come straight from L2 */
             for (int c = 0; c < s_gcount; ++c) {
                 if (skip >> c & 1u) {
-                    if (lane < 4) swarp[(((tile & 1) * a.group + c) * NW + warp) * 4 + lane] = 0.0;
+                    if (lane < 4) swarp[(((tile & 1) * half + c) * NW + warp) * 4 + lane] = 0.0;
                     continue;
                 }
                 const int cand = a.order[s_cbase + c];
@@ -748,7 +749,7 @@ __global__ void __launch_bounds__(T) rc_score_kernel(ScoreArgs a)
                 }
                 const unsigned anybad = __any_sync(0xffffffffu, bad);
                 if (lane == 0) {
-                    double *sw = swarp + (((tile & 1) * a.group + c) * NW + warp) * 4;
+                    double *sw = swarp + (((tile & 1) * half + c) * NW + warp) * 4;
                     sw[0] = a0;
                     sw[1] = a1;
                     sw[2] = e0;
@@ -766,7 +767,7 @@ __global__ void __launch_bounds__(T) rc_score_kernel(ScoreArgs a)
                 const int cand = a.order[s_cbase + c];
                 double s = 0.0;
                 for (int w = 0; w < NW; ++w) {
-                    const double v = swarp[(((tile & 1) * a.group + c) * NW + w) * 4 + q];
+                    const double v = swarp[(((tile & 1) * half + c) * NW + w) * 4 + q];
                     s = (mode == SM_MAXIMUM) ? fmax(s, v) : s + v;
                 }
                 a.part[((size_t)q * a.nprog + cand) * a.ptiles + tile] = s;
